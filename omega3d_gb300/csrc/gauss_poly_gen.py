@@ -7,13 +7,19 @@ and rho = sqrt(q),
     bbb = D(q) / sigma^5,   D(q) = 2 G'(q),
 
 and G(q) = q^(-3/2) (the singular kernel) to float precision beyond q = 48.  On [0, 48] the
-FP32 kernels evaluate G and D from the polynomials written here instead of erf/exp: one
-polynomial of degree DEG in t = q * s + o (t in [-1, 1]) per interval [e_j, e_(j+1)] of
-EDGES, fitted by least squares in the Chebyshev basis on a dense grid (near-minimax) and
-converted to monomials for Horner's rule.  G and D are computed here in double: the Taylor
-series for q < 1 (30 terms) and the closed form above.  The reported error includes the
-rounding of q to float (up to 2.5 x 6e-8 relative for D ~ q^(-5/2)), which every float
-evaluation of the core has.
+FP32 kernels evaluate G from the polynomials written here instead of erf/exp, and the
+gradient's factor -bbb/3 from the same polynomial's derivative: one polynomial of degree DEG
+per interval [2 j, 2 j + 2) in
+
+    tau = fma(u, -1.5, 1.5),   u = q - 2 j   (exact),
+
+so that dG/dtau = G'(q) / -1.5 = -D(q) / 3 is the number the kernels need, and one table
+of DEG + 1 floats per interval serves both.  24 intervals: a warp's lanes read coefficient k
+of their own intervals from 24 consecutive floats, which lie in different shared-memory
+banks whatever mix of intervals the lanes hold.  The fit is a least-squares fit of the
+relative errors of G and of D together.  G and D are computed here in double: the Taylor
+series for q < 1 (30 terms) and the closed form above.  The reported errors are those of
+the float32 evaluation (Horner's rule for G and its derivative) at float q.
 
 Run from this directory:  python gauss_poly_gen.py   (rewrites o3g_gauss_poly.h and
 o3g_gauss_poly_ds.h and prints the worst relative error of each evaluation).
@@ -24,13 +30,11 @@ import numpy as np
 from numpy.polynomial import chebyshev as C
 from scipy.special import erf
 
-# interval j = [j, j + 1) for j = 0..47, so that the kernels find j as the integer part of
-# q (one conversion, no square root); degree 5 reaches the float rounding of q already
+# the accurate mode's intervals: [j, j + 1) for j = 0..47
 EDGES = [float(j) for j in range(49)]
-DEG = 5
-# one interval's row: s, o, then (G_k, D_k) from k = DEG down to 0 (the order Horner's rule
-# consumes them)
-STRIDE = 2 + 2 * (DEG + 1)
+# the FP32 table: interval j covers [2 j, 2 j + 2)
+N32 = 24
+DEG = 7
 CONST = np.sqrt(2.0 / np.pi)
 
 
@@ -68,67 +72,73 @@ def gauss_D(q):
     return out
 
 
-def _horner_f32(p, t):
-    t = t.astype(np.float32)
-    acc = np.full_like(t, np.float32(p[-1]))
-    for a in p[-2::-1]:
-        acc = (acc.astype(np.float64) * t + np.float64(np.float32(a))).astype(np.float32)
-    return acc
+def gauss_D3(q):
+    return -gauss_D(q) / 3.0
+
+
+def _fma32(a, b, c):
+    return (np.asarray(a, np.float64) * np.asarray(b, np.float64) + np.asarray(c, np.float64)).astype(np.float32)
+
+
+def eval32(row, lo, q):
+    """G and -D/3 as the kernels evaluate them: float32, fused multiply-adds; row is c[DEG]..c[0]."""
+    q = np.asarray(q, np.float32)
+    u = (q.astype(np.float64) - lo).astype(np.float32)
+    t = _fma32(u, np.float32(-1.5), np.float32(1.5))
+    c = [np.float32(v) for v in row]
+    d = np.full_like(t, c[0])
+    g = _fma32(np.full_like(t, c[0]), t, c[1])
+    for k in range(2, len(c)):
+        d = _fma32(d, t, g)
+        g = _fma32(g, t, c[k])
+    return g, d
 
 
 def fit():
-    table, worst = [], 0.0
-    for lo, hi in zip(EDGES[:-1], EDGES[1:]):
-        s, o = 2.0 / (hi - lo), -(hi + lo) / (hi - lo)
-        q = np.linspace(lo, hi, 40001)
-        t = q * s + o
-        row = [s, o]
-        polys = []
-        for F in (gauss_G, gauss_D):
-            y = F(q)
-            p = C.cheb2poly(C.chebfit(t, y, DEG))
-            # checked slightly beyond the interval: the index rounds q to an edge's side
-            qq = np.linspace(lo - 1e-4 * (hi - lo), hi + 1e-4 * (hi - lo), 4001)
-            qq = qq[qq >= 0]
-            yy = F(qq)
-            # t = fmaf(q, s, o) on the float inputs: one rounding
-            tt = (qq.astype(np.float32).astype(np.float64) * np.float64(np.float32(s)) +
-                  np.float64(np.float32(o))).astype(np.float32)
-            worst = max(worst, float(np.max(np.abs(_horner_f32(p, tt) - yy) / np.abs(yy))))
-            polys.append(p)
-        for k in range(DEG, -1, -1):
-            row += [polys[0][k], polys[1][k]]
-        row += [0.0] * (STRIDE - len(row))
+    table, worst = [], [0.0, 0.0]
+    x = np.cos(np.pi * (np.arange(400) + 0.5) / 400)       # Chebyshev nodes
+    for j in range(N32):
+        lo = 2.0 * j
+        q = lo + 1.0 + x
+        t = -1.5 * x
+        V = np.vander(t, DEG + 1, increasing=True)
+        dV = np.zeros_like(V)
+        dV[:, 1:] = V[:, :-1] * np.arange(1, DEG + 1)
+        # the unknowns in the Chebyshev basis of x, for conditioning
+        M = np.linalg.lstsq(V, C.chebvander(x, DEG), rcond=None)[0]
+        G, D3 = gauss_G(q), gauss_D3(q)
+        A = np.vstack([V / G[:, None], dV / D3[:, None]])
+        c = M @ np.linalg.lstsq(A @ M, np.ones(2 * x.size), rcond=None)[0]
+        row = [np.float32(v) for v in c[::-1]]
+        qq = np.linspace(lo, lo + 2.0, 40001).astype(np.float32)
+        g, d = eval32(row, lo, qq)
+        q64 = qq.astype(np.float64)
+        worst[0] = max(worst[0], float(np.max(np.abs(g / gauss_G(q64) - 1.0))))
+        worst[1] = max(worst[1], float(np.max(np.abs(d / gauss_D3(q64) - 1.0))))
         table.append(row)
     return table, worst
 
 
 def write(table, worst, path):
-    # pair-interleaved and coefficient-major: the float pairs (s, o), (G_k, D_k) for
-    # k = DEG..0 are entries e2 = 0..DEG+1, entry e2 of interval j at float2 index
-    # e2 * N + j.  The lanes of a warp reading entry e2 of their own intervals touch one
-    # 112-byte span, and one 8-byte load gives both Horner chains their coefficient.
-    names = ["(s, o)"] + ["(G%d, D%d)" % (k, k) for k in range(DEG, -1, -1)]
     lines = []
-    for e2 in range(STRIDE // 2):
-        vals = ", ".join("%.9ef, %.9ef" % (np.float32(row[2 * e2]), np.float32(row[2 * e2 + 1])) for row in table)
-        lines.append("    // %s\n    %s," % (names[e2], vals))
+    for e in range(DEG + 1):
+        vals = ", ".join("%.9ef" % np.float32(row[e]) for row in table)
+        lines.append("    // c%d\n    %s," % (DEG - e, vals))
     body = "\n".join(lines)
     txt = f"""// o3g_gauss_poly.h -- GENERATED by gauss_poly_gen.py (do not edit): piecewise polynomials of
-// the FP32 Gaussian core on q in [0, 48]: G(q) (r3 = G / sigma^3) and D(q) = 2 G'(q)
-// (bbb = D / sigma^5), degree {DEG} in t = fma(q, s, o) per interval; float32 evaluation with
-// fused multiply-adds from a float q stays within {worst:.2e} relative of the double-precision
-// functions at the exact q (this includes the rounding of q itself).
+// the FP32 Gaussian core on q in [0, 48]: G(q) (r3 = G / sigma^3), degree {DEG} in
+// tau = fma(q - 2 j, -1.5, 1.5) on interval j = [2 j, 2 j + 2); dG/dtau = -G'(q) 2/3 is the
+// gradient's -bbb/3 = (dG/dtau) / sigma^5.  Evaluated in float32 with fused multiply-adds
+// at a float q, G stays within {worst[0]:.2e} and dG/dtau within {worst[1]:.2e} relative of the
+// double-precision functions.
 #pragma once
 
 namespace o3g {{
 
 constexpr int kGaussPolyDeg = {DEG};
-constexpr int kGaussPolyStride = {STRIDE};   // floats per interval: (s, o), (G[k], D[k]) for k = {DEG}..0
-constexpr int kGaussPolyN = {len(table)};        // intervals; interval j covers [j, j + 1)
-constexpr int kGaussPolyLast = {len(table) - 1};
-// float pair e2 of interval j at kGaussPoly[2 (e2 * kGaussPolyN + j)], [.. + 1]
-__device__ const __align__(16) float kGaussPoly[{STRIDE} * {len(table)}] = {{
+constexpr int kGaussPolyN = {len(table)};        // intervals; interval j covers [2 j, 2 j + 2)
+// coefficient c_k of interval j at kGaussPoly[({DEG} - k) * kGaussPolyN + j]
+__device__ const __align__(16) float kGaussPoly[{DEG + 1} * {len(table)}] = {{
 {body}
 }};
 
@@ -163,7 +173,7 @@ def fit_ds():
         t = q * s + o
         row = [s32, o32]
         polys = []
-        for F in (gauss_G, gauss_D):
+        for F in (gauss_G, gauss_D3):
             y = F(q)
             polys.append(C.cheb2poly(C.chebfit(t, y, DEG_DS)))
             # the kernel's evaluation: float tail, then (hi, lo) steps (double stands in for
@@ -202,8 +212,8 @@ def write_ds(table, worst, path):
         lines.append("    // %s\n    %s," % (names[k], vals))
     body = "\n".join(lines)
     txt = f"""// o3g_gauss_poly_ds.h -- GENERATED by gauss_poly_gen.py (do not edit): piecewise polynomials
-// of the Gaussian core for the accurate (double-single) precision mode, on the intervals of
-// o3g_gauss_poly.h: G(q) and D(q) = 2 G'(q), degree {DEG_DS} in t = q s + o (s, o the float
+// of the Gaussian core for the accurate (double-single) precision mode: G(q) and
+// D(q) = -(2/3) G'(q), degree {DEG_DS} in t = q s + o (s, o the float
 // values below).  Coefficients of degree >= {NDS} are floats (Horner in float); degrees
 // {NDS - 1}..0 are (hi, lo) float pairs (Horner in double-single).  Evaluated that way from an
 // exact q the result stays within {worst:.2e} relative of the double-precision functions.
@@ -211,10 +221,11 @@ def write_ds(table, worst, path):
 
 namespace o3g {{
 
+constexpr int kGaussDsN = {len(table)};        // intervals; interval j covers [j, j + 1)
 constexpr int kGaussDsDeg = {DEG_DS};
 constexpr int kGaussDsPairs = {NDS};
 constexpr int kGaussDsStride = {STRIDE_DS};   // s, o, (G[k], D[k]) for k = {DEG_DS}..{NDS}, then (G[k] hi, lo, D[k] hi, lo) for k = {NDS - 1}..0
-// entry e of interval j at kGaussPolyDs[e * kGaussPolyN + j]
+// entry e of interval j at kGaussPolyDs[e * kGaussDsN + j]
 __device__ const __align__(16) float kGaussPolyDs[{STRIDE_DS} * {len(table)}] = {{
 {body}
 }};
@@ -230,7 +241,7 @@ if __name__ == "__main__":
     tab, w = fit()
     out = os.path.join(here, "o3g_gauss_poly.h")
     write(tab, w, out)
-    print("wrote %s; worst float32 relative error %.3e" % (out, w))
+    print("wrote %s; worst float32 relative errors %.3e (G) %.3e (derivative)" % (out, w[0], w[1]))
     tab, w = fit_ds()
     out = os.path.join(here, "o3g_gauss_poly_ds.h")
     write_ds(tab, w, out)

@@ -51,7 +51,7 @@ struct BatchArgs {
 };
 
 template <int C, int MODE, bool GRADS, int TPT, class T>
-__global__ void __launch_bounds__(kBlock) k_batch(const BatchArgs<T> a) {
+__global__ void __launch_bounds__(kBlock, PairMinBlocks<C, MODE, GRADS, TPT>::value) k_batch(const BatchArgs<T> a) {
   constexpr bool ACC = (MODE == MODE_COMP);
   constexpr bool CLASSIFY = (C == CORE_GAUSS || C == CORE_EXP);
   constexpr int NA = GRADS ? 15 : 3;
@@ -63,9 +63,9 @@ __global__ void __launch_bounds__(kBlock) k_batch(const BatchArgs<T> a) {
   __shared__ float4 QB[2][5][kBlock / 2];   // staged tiles as source pairs, double-buffered
   __shared__ int s_item, s_last;
   // the Gaussian core's polynomial table, read from shared memory by the near-field pairs
-  __shared__ __align__(16) float gsh[C == CORE_GAUSS && std::is_same<T, float>::value ? kGaussPolyStride * kGaussPolyN : 1];
+  __shared__ __align__(16) float gsh[C == CORE_GAUSS ? kGaussTab : 1];
   const float* gtab = nullptr;
-  if constexpr (C == CORE_GAUSS && std::is_same<T, float>::value) {
+  if constexpr (C == CORE_GAUSS) {
     stage_gauss_table(gsh);   // visible after the first __syncthreads of the item loop
     gtab = gsh;
   }
@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(kBlock) k_batch(const BatchArgs<T> a) {
       for (int c = 0; c < NA; ++c) acc[k][c] = acc2[k][c].x + acc2[k][c].y;
     if (!ACC && GRADS) {
 #pragma unroll
-      for (int k = 0; k < TPT; ++k) fold_grads(acc[k]);
+      for (int k = 0; k < TPT; ++k) fold_grads<C>(acc[k]);
     }
 
     const BatchSysDev* S = a.sys + tb.x;

@@ -133,6 +133,13 @@ template <class T> struct GaussP;
 template <> struct GaussP<float>  { static constexpr float  qfar = 48.0f; static constexpr int nterms = 9; };
 template <> struct GaussP<double> { static constexpr double qfar = 90.0;  static constexpr int nterms = 17; };
 
+// the hardware's reciprocal square root with nothing around it (rsqrtf() scales subnormal
+// arguments, four more instructions): a subnormal x counts as 0 and gives infinity
+__device__ __forceinline__ float rsq_hw(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
 // reciprocal square root: plain = hardware approximation (MUFU.RSQ, <= 2 ulp);
 // accurate = one Newton-Raphson step on top (y' = y + y/2 (1 - x y^2)), ~1 ulp.
 template <bool ACC>
@@ -239,138 +246,68 @@ __device__ __forceinline__ double dev_expm1(double x) { return expm1(x); }
 __device__ __forceinline__ float dev_sqrt(float x) { return sqrtf(x); }
 __device__ __forceinline__ double dev_sqrt(double x) { return sqrt(x); }
 
-// G(q) and D(q) = 2 G'(q) of the Gaussian core for q in [0, qfar] in FP32, from the
-// piecewise polynomials of o3g_gauss_poly.h (Horner's rule in t = q s_j + o_j): branch-free,
-// no erf/exp/division.
-//
-// Interval of q: j covers [j, j + 1) up to [47, 48], so j is the integer part of q (q >= 0)
-// capped at the last; the fits are checked 1e-4 of their width beyond both ends.
-__device__ __forceinline__ int gauss_interval(float q) { return min((int)q, kGaussPolyLast); }
-
-// G(q) and D(q) by Horner's rule in t.  The table holds float pairs (s, o), (G_k, D_k),
-// coefficient-major (pair e2 of interval j at e2 * N + j), so the lanes of a warp, whatever
-// their intervals (neighbouring targets and sources give neighbouring q), read each pair
-// from a few cache lines or banks, and the two chains advance together in packed FMAs (FFMA2: each
-// lane rounds like FFMA, so G and D are bit-identical to two scalar chains).  `tab`: a
-// block's shared-memory copy of kGaussPoly (stage_gauss_table, 8-byte aligned), or nullptr
-// for the global table through the read-only cache.
-__device__ __forceinline__ float2 gtab_ld2(const float* tab, int i2) {
-  return tab ? reinterpret_cast<const float2*>(tab)[i2] : __ldg(reinterpret_cast<const float2*>(kGaussPoly) + i2);
-}
-__device__ __forceinline__ float gtab_ld(const float* tab, int i) { return tab ? tab[i] : __ldg(kGaussPoly + i); }
-__device__ __forceinline__ void gauss_poly(float q, float& G, float& D, const float* tab = nullptr) {
-  constexpr int N = kGaussPolyN;
-  const int j = gauss_interval(q);   // pair e2 of this interval: e2 * N + j
-  const float2 so = gtab_ld2(tab, j);
-  const float t = fmaf(q, so.x, so.y);
-  const float2 tt = make_float2(t, t);
-  float2 gd = gtab_ld2(tab, N + j);
-#pragma unroll
-  for (int k = 1; k <= kGaussPolyDeg; ++k) gd = __ffma2_rn(gd, tt, gtab_ld2(tab, (1 + k) * N + j));
-  G = gd.x;
-  D = gd.y;
-}
-__device__ __forceinline__ float gauss_poly_g(float q, const float* tab = nullptr) {
-  constexpr int N = kGaussPolyN;
-  const int j = gauss_interval(q);
-  const float2 so = gtab_ld2(tab, j);
-  const float t = fmaf(q, so.x, so.y);
-  float g = gtab_ld(tab, 2 * (N + j));
-#pragma unroll
-  for (int k = 1; k <= kGaussPolyDeg; ++k) g = fmaf(g, t, gtab_ld(tab, 2 * ((1 + k) * N + j)));
-  return g;
-}
-// copies the polynomial table into a block's shared array (all threads call; synchronise
-// before the first use)
+// copies the FP32 Gaussian polynomial table (o3g_gauss_poly.h) into a block's shared array
+// (all threads call; synchronise before the first use)
+constexpr int kGaussTab = (kGaussPolyDeg + 1) * kGaussPolyN;
 __device__ __forceinline__ void stage_gauss_table(float* s) {
-  for (int i = threadIdx.x; i < kGaussPolyStride * kGaussPolyN; i += blockDim.x) s[i] = kGaussPoly[i];
+  for (int i = threadIdx.x; i < kGaussTab; i += blockDim.x) s[i] = kGaussPoly[i];
 }
 
-// Gaussian core with gradient factor (the project's own definition, see o3dgpu.h):
-// r3 = G(q) / sigma^3, bbb = 2 G'(q) / sigma^5 with q = d^2 / sigma^2; the singular kernel
-// beyond q = qfar.  FP32 evaluates G from the polynomials above; FP64 (the comparator) from
-// the Taylor series for q < 1 and the closed form with erf/exp beyond.
-template <bool ACC, class T>
-__device__ __forceinline__ void gauss_g(T distsq, T sig2, T& r3, T& bbb, const float* tab = nullptr) {
-  const T c = T(0.79788456080286535588);  // sqrt(2/pi)
-  if (distsq > GaussP<T>::qfar * sig2) {   // q > qfar without the division
-    const T rs = rsq<ACC>(distsq);
-    const T rs2 = rs * rs;
+// The gradient factor: the kernels form b3 = -bbb / 3 (Kernels.h's bbb) and multiply the
+// gradient sums by kGradScale once at the end, which saves a multiplication per pair and the
+// factor's rounding: for the singular kernel b3 is r3 / d^2 itself.  The WL core's bbb has no
+// common factor 3; it is summed as it is.
+template <int C> struct GradScale { static constexpr float value = C == CORE_WL ? 1.0f : -3.0f; };
+
+// Gaussian core in FP64 (the project's own definition, see o3dgpu.h): r3 = G(q) / sigma^3,
+// bbb = 2 G'(q) / sigma^5 with q = d^2 / sigma^2; the singular kernel beyond q = qfar; the
+// Taylor series for q < 1 and the closed form with erf/exp beyond.  (FP32 evaluates packed
+// pairs from polynomials: core2 in o3g_pair_impl.cuh.)
+template <bool GRADS>
+__device__ __forceinline__ void gauss_f64(double distsq, double sig2, double& r3, double& b3) {
+  const double c = 0.79788456080286535588;  // sqrt(2/pi)
+  if (distsq > GaussP<double>::qfar * sig2) {   // q > qfar without the division
+    const double rs = rsqrt(distsq);
+    const double rs2 = rs * rs;
     r3 = rs2 * rs;
-    bbb = T(-3.0) * r3 * rs2;
+    if (GRADS) b3 = r3 * rs2;
     return;
   }
-  if constexpr (std::is_same<T, float>::value) {
-    const float rsg = rsq<ACC>(sig2);
-    const float rsg2 = rsg * rsg;
-    float G, D;
-    gauss_poly(distsq * rsg2, G, D, tab);
-    const float isig3 = rsg2 * rsg;
-    r3 = G * isig3;
-    bbb = D * isig3 * rsg2;
-    return;
-  }
-  const T q = distsq / sig2;
-  if (q < T(1.0)) {
-    T g = T(0), gp = T(0);
+  const double q = distsq / sig2;
+  const double rsg = rsqrt(sig2);
+  const double isig3 = rsg * rsg * rsg;
+  if (q < 1.0) {
+    double g = 0.0, gp = 0.0;
 #pragma unroll
-    for (int n = GaussP<T>::nterms; n >= 1; --n) g = g * q + T(gauss_coef(n));
-#pragma unroll
-    for (int n = GaussP<T>::nterms; n >= 2; --n) gp = gp * q + T((n - 1) * gauss_coef(n));
-    const T rsg = rsq<ACC>(sig2);
-    const T isig3 = rsg * rsg * rsg;
+    for (int n = GaussP<double>::nterms; n >= 1; --n) g = g * q + gauss_coef(n);
     r3 = c * g * isig3;
-    bbb = T(2.0) * c * gp * isig3 * (rsg * rsg);
-  } else {
-    const T rs = rsq<ACC>(distsq);
-    const T rs2 = rs * rs;
-    const T rho = dev_sqrt(q);
-    const T e = dev_exp(T(-0.5) * q);
-    const T g = dev_erf(rho * T(0.70710678118654752440)) - c * rho * e;
-    const T rsg = rsq<ACC>(sig2);
-    r3 = g * rs2 * rs;
-    bbb = (c * e * (rsg * rsg * rsg) - T(3.0) * r3) * rs2;
-  }
-}
-template <bool ACC, class T>
-__device__ __forceinline__ T gauss_v(T distsq, T sig2, const float* tab = nullptr) {
-  const T c = T(0.79788456080286535588);
-  if (distsq > GaussP<T>::qfar * sig2) {
-    const T rs = rsq<ACC>(distsq);
-    return rs * rs * rs;
-  }
-  if constexpr (std::is_same<T, float>::value) {
-    const float rsg = rsq<ACC>(sig2);
-    const float rsg2 = rsg * rsg;
-    return gauss_poly_g(distsq * rsg2, tab) * (rsg2 * rsg);
-  }
-  const T q = distsq / sig2;
-  if (q < T(1.0)) {
-    T g = T(0);
+    if (GRADS) {
 #pragma unroll
-    for (int n = GaussP<T>::nterms; n >= 1; --n) g = g * q + T(gauss_coef(n));
-    const T rsg = rsq<ACC>(sig2);
-    return c * g * rsg * rsg * rsg;
+      for (int n = GaussP<double>::nterms; n >= 2; --n) gp = gp * q + (n - 1) * gauss_coef(n);
+      b3 = (-2.0 / 3.0) * c * gp * isig3 * (rsg * rsg);
+    }
   } else {
-    const T rs = rsq<ACC>(distsq);
-    const T rho = dev_sqrt(q);
-    const T e = dev_exp(T(-0.5) * q);
-    const T g = dev_erf(rho * T(0.70710678118654752440)) - c * rho * e;
-    return g * rs * rs * rs;
+    const double rs = rsqrt(distsq);
+    const double rs2 = rs * rs;
+    const double rho = sqrt(q);
+    const double e = exp(-0.5 * q);
+    const double g = erf(rho * 0.70710678118654752440) - c * rho * e;
+    r3 = g * rs2 * rs;
+    if (GRADS) b3 = (r3 - (c / 3.0) * e * isig3) * rs2;
   }
 }
 
-// r3 and bbb of one pair; dx,dy,dz = target - source; cst as above.
+// r3 and b3 (bbb for WL) of one pair; dx,dy,dz = target - source; cst as above.
 template <int C, bool ACC, class T>
-__device__ __forceinline__ void core_g(T dx, T dy, T dz, T cst, T& r3, T& bbb, const float* gtab = nullptr) {
-  if (C == CORE_RM) {
+__device__ __forceinline__ void core_g(T dx, T dy, T dz, T cst, T& r3, T& b3) {
+  if constexpr (C == CORE_RM) {
     // CoreFunc.h:66-71: r2 = d^2 + sr^2 + tr^2, r3 = r2^-1.5, bbb = -3 r3 / r2
     const T r2 = fma(dx, dx, fma(dy, dy, fma(dz, dz, cst)));
     const T rs = rsq<ACC>(r2);
     const T rs2 = rs * rs;
     r3 = rs2 * rs;
-    bbb = T(-3.0) * r3 * rs2;
-  } else if (C == CORE_WL) {
+    b3 = r3 * rs2;
+  } else if constexpr (C == CORE_WL) {
     // CoreFunc.h:266-274: d2 = d^2 + r^2; r3 = (d^2 + 2.5 r^2) d2^-2.5; bbb = 2 d2^-2.5 - 5 r3 / d2
     const T distsq = fma(dx, dx, fma(dy, dy, dz * dz));
     const T d2 = distsq + cst;
@@ -379,8 +316,8 @@ __device__ __forceinline__ void core_g(T dx, T dy, T dz, T cst, T& r3, T& bbb, c
     const T rs2 = rs * rs;
     const T dn5 = rs2 * rs2 * rs;
     r3 = d2top * dn5;
-    bbb = fma(T(-5.0) * r3, rs2, T(2.0) * dn5);
-  } else if (C == CORE_EXP) {
+    b3 = fma(T(-5.0) * r3, rs2, T(2.0) * dn5);
+  } else if constexpr (C == CORE_EXP) {
     // CoreFunc.h:226-236 with the branches of exp_cond / exp_bbb (:119-174).  The core
     // jumps by reld3/2 (5e-4) where it switches form at reld3 = 0.001, so distsq is formed
     // in the reference's operation order, each operation rounded (Kernels.h:167-170), and
@@ -397,51 +334,51 @@ __device__ __forceinline__ void core_g(T dx, T dy, T dz, T cst, T& r3, T& bbb, c
     // exp_bbb (CoreFunc.h:121-132, :164-177), also in its double build
     if (reld3 > T(16.0f)) {
       r3 = ood3;
-      bbb = T(-3.0) * r3 / distsq;
+      b3 = r3 / distsq;
     } else if (reld3 < T(0.001f)) {
       r3 = corefac;
-      bbb = T(-1.5) * dist * r3 * r3;
+      b3 = T(0.5) * dist * r3 * r3;
     } else if (REF) {
       // plain FP32: the reference's own float arithmetic, 1 - exp(-x) and corefac exp(-x)
       // (exp_cond / exp_bbb, CoreFunc.h:127-128, :175-177), exp nearly correctly rounded
       const float e = exp_tang((float)-reld3);
       const float r3f = __fmul_rn((float)ood3, __fsub_rn(1.0f, e));
       r3 = (T)r3f;
-      bbb = (T)(__fdiv_rn(__fmul_rn(3.0f, __fsub_rn(__fmul_rn((float)corefac, e), r3f)), (float)distsq));
+      b3 = (T)(__fdiv_rn(__fsub_rn(r3f, __fmul_rn((float)corefac, e)), (float)distsq));
     } else {
       // compensated and FP64: 1 - exp(-x) through expm1, which keeps the digits that
       // float 1 - exp(-x) loses (about eps/x) near the core
       const T em1 = dev_expm1(-reld3);
       r3 = ood3 * (-em1);
-      bbb = T(3.0) * (corefac * (em1 + T(1.0)) - r3) / distsq;
+      b3 = (r3 - corefac * (em1 + T(1.0))) / distsq;
     }
-  } else if (C == CORE_V2) {
+  } else if constexpr (C == CORE_V2) {
     // CoreFunc.h:318-330: denom = d^4 + sr^4 + tr^4; r3 = denom^-0.75; bbb = -3 r3 denom^-0.5
     const T distsq = fma(dx, dx, fma(dy, dy, dz * dz));
     const T denom = fma(distsq, distsq, cst);
     const T rs = rsq<ACC>(denom);
     r3 = rs * dev_sqrt(rs);
-    bbb = T(-3.0) * r3 * rs;
+    b3 = r3 * rs;
   } else {
-    const T distsq = fma(dx, dx, fma(dy, dy, dz * dz));
-    gauss_g<ACC, T>(distsq, cst, r3, bbb, gtab);
+    static_assert(C != CORE_GAUSS || std::is_same<T, double>::value, "the FP32 Gaussian core is evaluated packed");
+    gauss_f64<true>(fma(dx, dx, fma(dy, dy, dz * dz)), cst, r3, b3);
   }
 }
 
 // r3 only (velocity-only kernels): CoreFunc.h:48-52, :246-252, :202-209, :297-304
 template <int C, bool ACC, class T>
-__device__ __forceinline__ T core_v(T dx, T dy, T dz, T cst, const float* gtab = nullptr) {
-  if (C == CORE_RM) {
+__device__ __forceinline__ T core_v(T dx, T dy, T dz, T cst) {
+  if constexpr (C == CORE_RM) {
     const T r2 = fma(dx, dx, fma(dy, dy, fma(dz, dz, cst)));
     const T rs = rsq<ACC>(r2);
     return rs * rs * rs;
-  } else if (C == CORE_WL) {
+  } else if constexpr (C == CORE_WL) {
     const T distsq = fma(dx, dx, fma(dy, dy, dz * dz));
     const T d2 = distsq + cst;
     const T rs = rsq<ACC>(d2);
     const T rs2 = rs * rs;
     return fma(T(2.5), cst, distsq) * (rs2 * rs2 * rs);
-  } else if (C == CORE_EXP) {
+  } else if constexpr (C == CORE_EXP) {
     constexpr bool REF = !ACC && std::is_same<T, float>::value;   // as in core_g
     const T distsq = dist2_ref(dx, dy, dz);
     const T dist = dev_sqrt(distsq);
@@ -452,13 +389,15 @@ __device__ __forceinline__ T core_v(T dx, T dy, T dz, T cst, const float* gtab =
     if (reld3 < T(0.001f)) return corefac;
     if (REF) return (T)__fmul_rn((float)ood3, __fsub_rn(1.0f, exp_tang((float)-reld3)));
     return ood3 * (-dev_expm1(-reld3));
-  } else if (C == CORE_V2) {
+  } else if constexpr (C == CORE_V2) {
     const T distsq = fma(dx, dx, fma(dy, dy, dz * dz));
     const T rs = rsq<ACC>(fma(distsq, distsq, cst));
     return rs * dev_sqrt(rs);
   } else {
-    const T distsq = fma(dx, dx, fma(dy, dy, dz * dz));
-    return gauss_v<ACC, T>(distsq, cst, gtab);
+    static_assert(C != CORE_GAUSS || std::is_same<T, double>::value, "the FP32 Gaussian core is evaluated packed");
+    double r3, b3;
+    gauss_f64<false>(fma(dx, dx, fma(dy, dy, dz * dz)), cst, r3, b3);
+    return r3;
   }
 }
 

@@ -117,13 +117,13 @@ __device__ __forceinline__ void ds_accum(float& acc, float& acc_lo, dsf x, dsf c
   acc_lo = __fadd_rn(acc_lo, __fadd_rn(sm.l, tl));
 }
 
-// G(q) (and D(q) = 2 G'(q) when GRAD) of the Gaussian core for q in [0, 48], q double-single:
+// G(q) (and D(q) = -(2/3) G'(q) when GRAD) of the Gaussian core for q in [0, 48], q double-single:
 // Horner's rule in float for the degrees >= kGaussDsPairs, then in double-single
 template <bool GRAD>
 __device__ __forceinline__ void gauss_poly_ds(dsf q, dsf& G, dsf& D) {
-  constexpr int N = kGaussPolyN;
+  constexpr int N = kGaussDsN;
   const float* tb = kGaussPolyDs;
-  const int j = gauss_interval(q.h);
+  const int j = min((int)q.h, kGaussDsN - 1);   // interval j covers [j, j + 1)
   const dsf t = ds_add_f(ds_mul_f(q, __ldg(tb + j)), __ldg(tb + N + j));
   constexpr int NF = kGaussDsDeg + 1 - kGaussDsPairs;      // float coefficients per function
   float g = __ldg(tb + 2 * N + j), d = GRAD ? __ldg(tb + 3 * N + j) : 0.f;
@@ -143,29 +143,29 @@ __device__ __forceinline__ void gauss_poly_ds(dsf q, dsf& G, dsf& D) {
   D = dd;
 }
 
-// Core factor in double-single for CORE_SING, CORE_RM and CORE_GAUSS: r3 (and bbb, rounded
-// to float, when GRAD), from d^2 and the radii sr, tr (tr = 0 for singular targets)
+// Core factor in double-single for CORE_SING, CORE_RM and CORE_GAUSS: r3 (and b3 = -bbb/3,
+// rounded to float, when GRAD), from d^2 and the radii sr, tr (tr = 0 for singular targets)
 template <int C, bool GRAD>
-__device__ __forceinline__ void core_ds(dsf d2, float sr, float tr, dsf& r3, float& bbb) {
+__device__ __forceinline__ void core_ds(dsf d2, float sr, float tr, dsf& r3, float& b3) {
   if (C == CORE_SING) {
     const dsf rs = ds_rsqrt(d2);
     const dsf rs2 = ds_mul(rs, rs);
     r3 = ds_mul(rs2, rs);
-    if (GRAD) bbb = __fmul_rn(__fmul_rn(-3.0f, r3.h), rs2.h);
+    if (GRAD) b3 = __fmul_rn(r3.h, rs2.h);
     return;
   }
   const dsf sig2 = ds_add(ds_prod(sr, sr), ds_prod(tr, tr));
   if (C == CORE_RM) {
-    // CoreFunc.h:66-71: r2 = d^2 + sr^2 + tr^2, r3 = r2^-1.5, bbb = -3 r3 / r2
+    // CoreFunc.h:66-71: r2 = d^2 + sr^2 + tr^2, r3 = r2^-1.5, bbb = -3 r3 / r2 (b3 = r3 / r2)
     const dsf rs = ds_rsqrt(ds_add(d2, sig2));
     const dsf rs2 = ds_mul(rs, rs);
     r3 = ds_mul(rs2, rs);
-    if (GRAD) bbb = __fmul_rn(__fmul_rn(-3.0f, r3.h), rs2.h);
+    if (GRAD) b3 = __fmul_rn(r3.h, rs2.h);
     return;
   }
   // Gaussian: the singular kernel beyond q = 48 (the correction is below 3e-10 there)
   if (d2.h > 48.0f * sig2.h) {
-    core_ds<CORE_SING, GRAD>(d2, 0.f, 0.f, r3, bbb);
+    core_ds<CORE_SING, GRAD>(d2, 0.f, 0.f, r3, b3);
     return;
   }
   const dsf rsg = ds_rsqrt(sig2);
@@ -174,7 +174,7 @@ __device__ __forceinline__ void core_ds(dsf d2, float sr, float tr, dsf& r3, flo
   gauss_poly_ds<GRAD>(ds_mul(d2, rsg2), G, D);
   const dsf isig3 = ds_mul(rsg2, rsg);
   r3 = ds_mul(G, isig3);
-  if (GRAD) bbb = __fmul_rn(__fmul_rn(ds_round(D), ds_round(isig3)), ds_round(rsg2));
+  if (GRAD) b3 = __fmul_rn(__fmul_rn(ds_round(D), ds_round(isig3)), ds_round(rsg2));
 }
 
 }  // namespace o3g

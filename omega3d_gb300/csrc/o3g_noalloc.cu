@@ -103,7 +103,7 @@ static int32_t noalloc_run(int ns, const float* sx, const float* sy, const float
   DeviceFacts df;
   O3G_TRY(device_facts(&df));
   int nb = 0;
-  O3G_TRY(occupancy_blocks((const void*)&k_pair<C, MODE, GRADS, HAVE_TR, TPT, float, float>, kBlock, &nb));
+  O3G_TRY(occupancy_blocks((const void*)&k_pair_f<C, MODE, GRADS, HAVE_TR, TPT>, kBlock, &nb));
   PairPlan pl;
   plan_pair(ns, nt, TPT, nb * df.num_sms, &pl);
   const int nsp = same ? (pl.ns_pad > pl.nt_pad ? pl.ns_pad : pl.nt_pad) : pl.ns_pad;
@@ -153,7 +153,7 @@ static int32_t noalloc_run(int ns, const float* sx, const float* sy, const float
   a.spos = spos; a.sstr = sstr; a.ntiles = pl.ntiles; a.tiles_per_split = pl.tiles_per_split;
   a.tpos = tpos; a.nt = nt; a.nt_pad = pl.nt_pad; a.partial = partial; a.out = out;
   a.tperm = nullptr; a.tile_lo = tile_lo; a.tile_hi = tile_hi;
-  k_pair<C, MODE, GRADS, HAVE_TR, TPT, float, float><<<dim3(pl.tblocks, pl.nsplit), kBlock, 0, st>>>(a);
+  k_pair_f<C, MODE, GRADS, HAVE_TR, TPT><<<dim3(pl.tblocks, pl.nsplit), kBlock, 0, st>>>(a);
   note_launch();
   if (pl.nsplit > 1) {
     k_reduce<NC, ACC, float, float><<<dim3((nt + 255) / 256, NC), 256, 0, st>>>(partial, pl.nsplit, nt, pl.nt_pad,

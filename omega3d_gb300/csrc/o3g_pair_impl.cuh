@@ -58,25 +58,24 @@ template <class T, class O> struct PairArgs {
   const float4* tile_hi;     // per half tile: (max x, max y, max z, -)
 };
 
-// one pair, velocity + gradient.  a[0..2] velocity, a[3..11] gradient sums of
-// bbb * d (x) (s x d) in the reference order, a[12..14] = sum r3 * s (folded into the
-// antisymmetric gradient terms by fold_grads, Kernels.h:184-192).
-template <int C, bool ACC, bool HAVE_TR, class T>
-__device__ __forceinline__ void pair_g(const V4<T>& t, const V4<T>& s, const V4<T>& w, T* a,
-                                       const float* gtab = nullptr) {
+// one FP64 pair, velocity + gradient.  a[0..2] velocity, a[3..11] gradient sums of
+// b3 * d (x) (s x d) in the reference order (b3 = bbb / GradScale), a[12..14] = sum r3 * s
+// (both joined by fold_grads, Kernels.h:184-192).
+template <int C, bool HAVE_TR, class T>
+__device__ __forceinline__ void pair_g(const V4<T>& t, const V4<T>& s, const V4<T>& w, T* a) {
   const T dx = t.x - s.x;
   const T dy = t.y - s.y;
   const T dz = t.z - s.z;
-  T r3, bbb;
-  if (C == CORE_SING) {
+  T r3, b3;
+  if constexpr (C == CORE_SING) {
     const T r2 = fma(dx, dx, fma(dy, dy, dz * dz));
-    const T rs = rsq<ACC>(r2);
+    const T rs = rsqrt(r2);
     const T rs2 = rs * rs;
     r3 = rs2 * rs;
-    bbb = T(-3.0) * r3 * rs2;
+    b3 = r3 * rs2;
   } else {
     const T cst = HAVE_TR ? (s.w + t.w) : s.w;
-    core_g<C, ACC, T>(dx, dy, dz, cst, r3, bbb, gtab);
+    core_g<C, true, T>(dx, dy, dz, cst, r3, b3);
   }
   T cx = dz * w.y - dy * w.z;
   T cy = dx * w.z - dz * w.x;
@@ -84,9 +83,9 @@ __device__ __forceinline__ void pair_g(const V4<T>& t, const V4<T>& s, const V4<
   a[0] = fma(r3, cx, a[0]);
   a[1] = fma(r3, cy, a[1]);
   a[2] = fma(r3, cz, a[2]);
-  cx *= bbb;
-  cy *= bbb;
-  cz *= bbb;
+  cx *= b3;
+  cy *= b3;
+  cz *= b3;
   a[3] = fma(dx, cx, a[3]);
   a[4] = fma(dx, cy, a[4]);
   a[5] = fma(dx, cz, a[5]);
@@ -102,19 +101,18 @@ __device__ __forceinline__ void pair_g(const V4<T>& t, const V4<T>& s, const V4<
 }
 
 // velocity only
-template <int C, bool ACC, bool HAVE_TR, class T>
-__device__ __forceinline__ void pair_v(const V4<T>& t, const V4<T>& s, const V4<T>& w, T* a,
-                                       const float* gtab = nullptr) {
+template <int C, bool HAVE_TR, class T>
+__device__ __forceinline__ void pair_v(const V4<T>& t, const V4<T>& s, const V4<T>& w, T* a) {
   const T dx = t.x - s.x;
   const T dy = t.y - s.y;
   const T dz = t.z - s.z;
   T r3;
-  if (C == CORE_SING) {
-    const T rs = rsq<ACC>(fma(dx, dx, fma(dy, dy, dz * dz)));
+  if constexpr (C == CORE_SING) {
+    const T rs = rsqrt(fma(dx, dx, fma(dy, dy, dz * dz)));
     r3 = rs * rs * rs;
   } else {
     const T cst = HAVE_TR ? (s.w + t.w) : s.w;
-    r3 = core_v<C, ACC, T>(dx, dy, dz, cst, gtab);
+    r3 = core_v<C, true, T>(dx, dy, dz, cst);
   }
   a[0] = fma(r3, dz * w.y - dy * w.z, a[0]);
   a[1] = fma(r3, dx * w.z - dz * w.x, a[1]);
@@ -132,17 +130,17 @@ __device__ __forceinline__ void pair_g_ds(const V4<float>& t, const V4<float>& s
   const dsf dz = ds_two_sum(t.z, -s.z);
   const dsf d2 = ds_add(ds_add(ds_sq(dx), ds_sq(dy)), ds_sq(dz));
   dsf r3;
-  float bbb;
-  core_ds<C, true>(d2, w.w, HAVE_TR ? t.w : 0.f, r3, bbb);
+  float b3;
+  core_ds<C, true>(d2, w.w, HAVE_TR ? t.w : 0.f, r3, b3);
   const dsf cx = ds_cross(dz, w.y, dy, w.z);
   const dsf cy = ds_cross(dx, w.z, dz, w.x);
   const dsf cz = ds_cross(dy, w.x, dx, w.y);
   ds_accum(a[0], a[15], r3, cx);
   ds_accum(a[1], a[16], r3, cy);
   ds_accum(a[2], a[17], r3, cz);
-  const float bx = __fmul_rn(__fadd_rn(cx.h, cx.l), bbb);
-  const float by = __fmul_rn(__fadd_rn(cy.h, cy.l), bbb);
-  const float bz = __fmul_rn(__fadd_rn(cz.h, cz.l), bbb);
+  const float bx = __fmul_rn(__fadd_rn(cx.h, cx.l), b3);
+  const float by = __fmul_rn(__fadd_rn(cy.h, cy.l), b3);
+  const float bz = __fmul_rn(__fadd_rn(cz.h, cz.l), b3);
   const float ex = dx.h, ey = dy.h, ez = dz.h;
   a[3] = fmaf(ex, bx, a[3]);
   a[4] = fmaf(ex, by, a[4]);
@@ -165,32 +163,37 @@ __device__ __forceinline__ void pair_v_ds(const V4<float>& t, const V4<float>& s
   const dsf dz = ds_two_sum(t.z, -s.z);
   const dsf d2 = ds_add(ds_add(ds_sq(dx), ds_sq(dy)), ds_sq(dz));
   dsf r3;
-  float bbb;
-  core_ds<C, false>(d2, w.w, HAVE_TR ? t.w : 0.f, r3, bbb);
+  float b3;
+  core_ds<C, false>(d2, w.w, HAVE_TR ? t.w : 0.f, r3, b3);
   ds_accum(a[0], a[3], r3, ds_cross(dz, w.y, dy, w.z));
   ds_accum(a[1], a[4], r3, ds_cross(dx, w.z, dz, w.x));
   ds_accum(a[2], a[5], r3, ds_cross(dy, w.x, dx, w.y));
 }
 
-// a[12..14] -> antisymmetric gradient terms: tvx += sz r3, twx -= sy r3, tuy -= sz r3,
-// twy += sx r3, tuz += sy r3, tvz -= sx r3 (Kernels.h:185-191)
-template <class T>
+// The gradient sums from their parts: a[3..11] by the factor that b3 leaves out, and
+// a[12..14] into the antisymmetric terms: tvx += sz r3, twx -= sy r3, tuy -= sz r3,
+// twy += sx r3, tuz += sy r3, tvz -= sx r3 (Kernels.h:185-191).  NO_ZZ: a[11] was not summed;
+// d . (s x d) = 0, so the sums of b3 d (x) (s x d) have no trace.
+template <int C, bool NO_ZZ = false, class T>
 __device__ __forceinline__ void fold_grads(T* a) {
-  a[4] += a[14];
-  a[5] -= a[13];
-  a[6] -= a[14];
-  a[8] += a[12];
-  a[9] += a[13];
-  a[10] -= a[12];
+  constexpr T k = T(GradScale<C>::value);
+  if (NO_ZZ) a[11] = -(a[3] + a[7]);
+  a[3] *= k;
+  a[4] = fma(k, a[4], a[14]);
+  a[5] = fma(k, a[5], -a[13]);
+  a[6] = fma(k, a[6], -a[14]);
+  a[7] *= k;
+  a[8] = fma(k, a[8], a[12]);
+  a[9] = fma(k, a[9], a[13]);
+  a[10] = fma(k, a[10], -a[12]);
+  a[11] *= k;
 }
 
-// Sweep the staged tile (kBlock sources in shared memory) for TPT targets.  In the
-// compensated mode the plain partial of every FOLD sources is folded into (hi, lo) with
-// Fast2Sum.
+// Sweep the staged tile (kBlock sources in shared memory) for TPT targets, FP64 or accurate.
+// In the accurate mode the partial of every FOLD sources is folded into (hi, lo).
 template <int C, int MODE, bool GRADS, bool HAVE_TR, int TPT, class T, int NA, int NC, int NH, int NS = kBlock>
 __device__ __forceinline__ void sweep_tile(const V4<T>* sp, const V4<T>* sw, const V4<T>* tp, T (*acc)[NA],
-                                           float (*hi)[NH], float (*lo)[NH], const float* gtab = nullptr) {
-  constexpr bool ACC = (MODE == MODE_COMP);
+                                           float (*hi)[NH], float (*lo)[NH]) {
   constexpr bool SUMC = SumComp<MODE>::value;
   constexpr int FOLD = SUMC ? 16 : NS;
 #pragma unroll 1
@@ -205,38 +208,26 @@ __device__ __forceinline__ void sweep_tile(const V4<T>* sp, const V4<T>* sw, con
           if (GRADS) pair_g_ds<C, HAVE_TR>(tp[k], s, w, acc[k]);
           else       pair_v_ds<C, HAVE_TR>(tp[k], s, w, acc[k]);
         } else {
-          if (GRADS) pair_g<C, ACC, HAVE_TR, T>(tp[k], s, w, acc[k], gtab);
-          else       pair_v<C, ACC, HAVE_TR, T>(tp[k], s, w, acc[k], gtab);
+          if (GRADS) pair_g<C, HAVE_TR, T>(tp[k], s, w, acc[k]);
+          else       pair_v<C, HAVE_TR, T>(tp[k], s, w, acc[k]);
         }
       }
     }
     if (SUMC) {
 #pragma unroll
       for (int k = 0; k < TPT; ++k) {
-        if (GRADS) fold_grads(acc[k]);
+        if (GRADS) fold_grads<C>(acc[k]);
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
-          float s, e;
-          if constexpr (MODE == MODE_DS) {
-            // two-sum: exact in any order (a running sum that passes near zero while the
-            // partials are large would otherwise lose the partial's rounding)
-            const dsf t2 = ds_two_sum(hi[k][c], (float)acc[k][c]);
-            s = t2.h;
-            e = t2.l;
-          } else {
-            // Fast2Sum: exact error term when |hi| >= |partial|, the usual case once a few
-            // folds have accumulated; otherwise that fold loses at most its own rounding
-            s = hi[k][c] + (float)acc[k][c];
-            e = (float)acc[k][c] - (s - hi[k][c]);
-          }
-          hi[k][c] = s;
-          lo[k][c] += e;
+          // two-sum: exact in any order (a running sum that passes near zero while the
+          // partials are large would otherwise lose the partial's rounding)
+          const dsf t2 = ds_two_sum(hi[k][c], (float)acc[k][c]);
+          hi[k][c] = t2.h;
+          lo[k][c] += t2.l;
         }
-        if constexpr (MODE == MODE_DS) {
-          // the velocity sums' low parts (the last three accumulators)
+        // the velocity sums' low parts (the last three accumulators)
 #pragma unroll
-          for (int c = 0; c < 3; ++c) lo[k][c] += (float)acc[k][NA - 3 + c];
-        }
+        for (int c = 0; c < 3; ++c) lo[k][c] += (float)acc[k][NA - 3 + c];
 #pragma unroll
         for (int c = 0; c < NA; ++c) acc[k][c] = T(0);
       }
@@ -245,9 +236,16 @@ __device__ __forceinline__ void sweep_tile(const V4<T>* sp, const V4<T>* sw, con
 }
 
 // ---- packed FP32: two sources per instruction (FFMA2 / FADD2 / FMUL2 on float2) -----------
-// The FP32 kernels are bound by instruction issue, not by the FMA pipe: a packed
-// instruction does two sources' operation in one issue slot.  Each lane of a packed
-// operation rounds exactly like the scalar instruction.  A staged tile is re-laid out in
+// What bounds these kernels is the FMA pipe: RM plain with gradients takes 34 packed
+// operations and two MUFU per pair of sources, 34 cycles per pair and warp scheduler at two
+// cycles each, and runs at 41 (65,536 particles, one GB300; was 47 with 37 operations).
+// The rest is the register file: a micro-benchmark of FFMA2 alone takes 2.1 cycles when one
+// operand is the previous instruction's, 2.95 with three new ones (FMUL2, FADD2 2.1; a
+// scalar FFMA 1.08), so the accumulations below are written in runs that share an operand.
+// Scalar accumulations on the paired registers were slower (44 to 48 cycles), as was a
+// fully scalar sweep (45 at best).  A packed instruction does two sources' operation in one
+// issue slot, and each lane of it
+// rounds exactly like the scalar instruction.  A staged tile is re-laid out in
 // shared memory as pairs of sources (2p, 2p+1), component-major so every load yields
 // float2 operands directly:
 //   Q[0][p] = (-x0, -x1, -y0, -y1)    Q[1][p] = (-z0, -z1, c0, c1)     (c: core parameter)
@@ -272,70 +270,155 @@ __device__ __forceinline__ void stage_pair(const V4<float>& s, const V4<float>& 
 __device__ __forceinline__ float2 f2lo(const float4& q) { return make_float2(q.x, q.y); }
 __device__ __forceinline__ float2 f2hi(const float4& q) { return make_float2(q.z, q.w); }
 
+__device__ __forceinline__ float2 f2(float v) { return make_float2(v, v); }
+
+// x^(-1/2) (rs), x^(-1) (s2) and x^(-3/2) (r3) of two lanes.  ACC: one Newton step whose
+// residual e = 1 - x s2 is formed from the rounded square s2 = rs^2 by one fma, so the
+// corrections r3 (1 + 3e/2) and s2 (1 + e) also undo s2's own rounding: r3 keeps about half
+// the error of the cube of a corrected rs, for the same seven operations.
+template <bool ACC>
+__device__ __forceinline__ void rsq2(const float2& x, float2& s2, float2& r3) {
+  const float2 rs = make_float2(rsq_hw(x.x), rsq_hw(x.y));
+  s2 = __fmul2_rn(rs, rs);
+  r3 = __fmul2_rn(s2, rs);
+  if (ACC) {
+    const float2 e = __ffma2_rn(make_float2(-x.x, -x.y), s2, f2(1.f));
+    r3 = __ffma2_rn(r3, __fmul2_rn(e, f2(1.5f)), r3);
+    s2 = __ffma2_rn(s2, e, s2);
+  }
+}
+
+// The Gaussian core of two lanes (o3g_gauss_poly.h): q = d^2 / sigma^2, the polynomial of its
+// interval for r3 = G / sigma^3 and that polynomial's derivative for b3 = (dG/dtau) / sigma^5,
+// the singular kernel beyond q = 48.  The interval j = floor(q / 2) comes from a round-down
+// fma (2^23 + q / 2 has ulp 1); fminf caps it at the last one (q = 48 exactly, infinities)
+// and turns a NaN into it, so the table index stays in range whatever the data.  `gtab` is
+// the block's shared-memory copy: coefficient k of all 24 intervals lies in 24 different
+// banks, so a warp's read takes one pass whatever intervals its lanes hold.
+template <bool ACC, bool GRADS>
+__device__ __forceinline__ void gauss2(const float2& r2, const float2& sig2, const float* gtab, float2& r3,
+                                       float2& b3) {
+  const float2 lim = __fmul2_rn(sig2, f2(GaussP<float>::qfar));
+  const bool fx = r2.x > lim.x, fy = r2.y > lim.y;
+  float2 g = f2(0.f), d = f2(0.f);
+  if (!(fx && fy)) {
+    float2 i2, i3;
+    rsq2<ACC>(sig2, i2, i3);
+    const float2 q = __fmul2_rn(r2, i2);
+    float2 fj = __ffma2_rd(q, f2(0.5f), f2(8388608.f));
+    fj = make_float2(fminf(fj.x, 8388608.f + (kGaussPolyN - 1)), fminf(fj.y, 8388608.f + (kGaussPolyN - 1)));
+    const float* tx = gtab + (__float_as_int(fj.x) - 0x4B000000);
+    const float* ty = gtab + (__float_as_int(fj.y) - 0x4B000000);
+    const float2 u = __ffma2_rn(__fadd2_rn(fj, f2(-8388608.f)), f2(-2.f), q);
+    const float2 t = __ffma2_rn(u, f2(-1.5f), f2(1.5f));
+    d = make_float2(tx[0], ty[0]);
+    g = __ffma2_rn(d, t, make_float2(tx[kGaussPolyN], ty[kGaussPolyN]));
+#pragma unroll
+    for (int k = 2; k <= kGaussPolyDeg; ++k) {
+      if (GRADS) d = __ffma2_rn(d, t, g);
+      g = __ffma2_rn(g, t, make_float2(tx[k * kGaussPolyN], ty[k * kGaussPolyN]));
+    }
+    g = __fmul2_rn(g, i3);
+    if (GRADS) d = __fmul2_rn(d, __fmul2_rn(i3, i2));
+  }
+  if (fx || fy) {
+    float2 s2, s3;
+    rsq2<ACC>(r2, s2, s3);
+    g = make_float2(fx ? s3.x : g.x, fy ? s3.y : g.y);
+    if (GRADS) {
+      const float2 s5 = __fmul2_rn(s3, s2);
+      d = make_float2(fx ? s5.x : d.x, fy ? s5.y : d.y);
+    }
+  }
+  r3 = g;
+  b3 = d;
+}
+
+// r3 (and b3) of the two lanes' pairs; EXP, which follows the reference's own float
+// arithmetic, runs the scalar core per lane
+template <int C, bool ACC, bool GRADS>
+__device__ __forceinline__ void core2(const float2& dx, const float2& dy, const float2& dz, const float2& cst,
+                                      const float* gtab, float2& r3, float2& b3) {
+  if constexpr (C == CORE_EXP) {
+    if (GRADS) {
+      core_g<C, ACC, float>(dx.x, dy.x, dz.x, cst.x, r3.x, b3.x);
+      core_g<C, ACC, float>(dx.y, dy.y, dz.y, cst.y, r3.y, b3.y);
+    } else {
+      r3.x = core_v<C, ACC, float>(dx.x, dy.x, dz.x, cst.x);
+      r3.y = core_v<C, ACC, float>(dx.y, dy.y, dz.y, cst.y);
+    }
+  } else if constexpr (C == CORE_RM) {
+    // CoreFunc.h:66-71
+    float2 s2;
+    rsq2<ACC>(__ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, cst))), s2, r3);
+    if (GRADS) b3 = __fmul2_rn(r3, s2);
+  } else {
+    const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
+    if constexpr (C == CORE_SING) {
+      float2 s2;
+      rsq2<ACC>(r2, s2, r3);
+      if (GRADS) b3 = __fmul2_rn(r3, s2);
+    } else if constexpr (C == CORE_WL) {
+      // CoreFunc.h:266-274
+      float2 s2, s3;
+      rsq2<ACC>(__fadd2_rn(r2, cst), s2, s3);
+      const float2 dn5 = __fmul2_rn(s3, s2);
+      r3 = __fmul2_rn(__ffma2_rn(f2(2.5f), cst, r2), dn5);
+      if (GRADS) b3 = __ffma2_rn(__fmul2_rn(r3, f2(-5.f)), s2, __fmul2_rn(dn5, f2(2.f)));
+    } else if constexpr (C == CORE_V2) {
+      // CoreFunc.h:318-330: rs = (d^4 + c)^(-1/2), r3 = rs sqrt(rs).  d^4 may be subnormal where
+      // r3 is still finite, so rs comes from rsqrtf(); sqrt(rs) = rs rs^(-1/2) with one
+      // Newton step
+      const float2 den = __ffma2_rn(r2, r2, cst);
+      const float2 rs = make_float2(rsq<ACC>(den.x), rsq<ACC>(den.y));
+      const float2 y = make_float2(rsq_hw(rs.x), rsq_hw(rs.y));
+      const float2 z = __fmul2_rn(rs, y);
+      const float2 e = __ffma2_rn(make_float2(-z.x, -z.y), y, f2(1.f));
+      r3 = __fmul2_rn(rs, __ffma2_rn(__fmul2_rn(z, f2(0.5f)), e, z));
+      if (GRADS) b3 = __fmul2_rn(r3, rs);
+    } else {
+      static_assert(C == CORE_GAUSS, "");
+      gauss2<ACC, GRADS>(r2, cst, gtab, r3, b3);
+    }
+  }
+}
+
 // one target (tt = (x,x), (y,y), (z,z), (c,c)) against the source pair of q0..q4; a[] as in
-// pair_g / pair_v, one float2 lane per source.  RM and the singular far-field kernel are
-// packed throughout; the other cores evaluate r3 (and bbb) per lane with the scalar core.
-template <int C, bool ACC, bool HAVE_TR, bool GRADS>
+// pair_g / pair_v, one float2 lane per source.  NO_ZZ: a[11] is left out (fold_grads).
+template <int C, bool ACC, bool HAVE_TR, bool GRADS, bool NO_ZZ>
 __device__ __forceinline__ void pair2(const float2* tt, const float4& q0, const float4& q1, const float4& q2,
                                       const float4& q3, const float4& q4, float2* a, const float* gtab) {
   const float2 dx = __fadd2_rn(tt[0], f2lo(q0));
   const float2 dy = __fadd2_rn(tt[1], f2hi(q0));
   const float2 dz = __fadd2_rn(tt[2], f2lo(q1));
-  float2 r3, bbb = make_float2(0.f, 0.f);
-  if constexpr (C == CORE_SING || C == CORE_RM) {
-    float2 r2;
-    if constexpr (C == CORE_RM) {
-      const float2 cst = HAVE_TR ? __fadd2_rn(f2hi(q1), tt[3]) : f2hi(q1);
-      r2 = __ffma2_rn(dz, dz, cst);
-    } else {
-      r2 = __fmul2_rn(dz, dz);
-    }
-    r2 = __ffma2_rn(dy, dy, r2);
-    r2 = __ffma2_rn(dx, dx, r2);
-    float2 rs = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
-    if (ACC) {
-      // y' = y + y/2 (1 - x y^2), as rsq<true>: fma(-y/2, x y^2 - 1, y)
-      const float2 h = __fmul2_rn(r2, rs);
-      const float2 e = __ffma2_rn(h, rs, make_float2(-1.f, -1.f));
-      rs = __ffma2_rn(__fmul2_rn(rs, make_float2(-0.5f, -0.5f)), e, rs);
-    }
-    const float2 rs2 = __fmul2_rn(rs, rs);
-    r3 = __fmul2_rn(rs2, rs);
-    if (GRADS) bbb = __fmul2_rn(__fmul2_rn(r3, make_float2(-3.f, -3.f)), rs2);
-  } else {
-    const float2 cst = HAVE_TR ? __fadd2_rn(f2hi(q1), tt[3]) : f2hi(q1);
-    if (GRADS) {
-      core_g<C, ACC, float>(dx.x, dy.x, dz.x, cst.x, r3.x, bbb.x, gtab);
-      core_g<C, ACC, float>(dx.y, dy.y, dz.y, cst.y, r3.y, bbb.y, gtab);
-    } else {
-      r3.x = core_v<C, ACC, float>(dx.x, dy.x, dz.x, cst.x, gtab);
-      r3.y = core_v<C, ACC, float>(dx.y, dy.y, dz.y, cst.y, gtab);
-    }
-  }
+  const float2 cst = HAVE_TR && C != CORE_SING ? __fadd2_rn(f2hi(q1), tt[3]) : f2hi(q1);
+  float2 r3, b3;
+  core2<C, ACC, GRADS>(dx, dy, dz, cst, gtab, r3, b3);
   const float2 wx = f2lo(q2), wy = f2hi(q2), wz = f2lo(q3);
   const float2 nwx = f2hi(q3), nwy = f2lo(q4), nwz = f2hi(q4);
-  float2 cx = __ffma2_rn(dz, wy, __fmul2_rn(dy, nwz));   // dz wy - dy wz
-  float2 cy = __ffma2_rn(dx, wz, __fmul2_rn(dz, nwx));   // dx wz - dz wx
-  float2 cz = __ffma2_rn(dy, wx, __fmul2_rn(dx, nwy));   // dy wx - dx wy
+  float2 cx = __fmul2_rn(dy, nwz), cy = __fmul2_rn(dx, wz), cz = __fmul2_rn(dx, nwy);
+  cx = __ffma2_rn(dz, wy, cx);    // dz wy - dy wz
+  cy = __ffma2_rn(dz, nwx, cy);   // dx wz - dz wx
+  cz = __ffma2_rn(dy, wx, cz);    // dy wx - dx wy
   a[0] = __ffma2_rn(r3, cx, a[0]);
   a[1] = __ffma2_rn(r3, cy, a[1]);
   a[2] = __ffma2_rn(r3, cz, a[2]);
   if (GRADS) {
-    cx = __fmul2_rn(cx, bbb);
-    cy = __fmul2_rn(cy, bbb);
-    cz = __fmul2_rn(cz, bbb);
-    a[3] = __ffma2_rn(dx, cx, a[3]);
-    a[4] = __ffma2_rn(dx, cy, a[4]);
-    a[5] = __ffma2_rn(dx, cz, a[5]);
-    a[6] = __ffma2_rn(dy, cx, a[6]);
-    a[7] = __ffma2_rn(dy, cy, a[7]);
-    a[8] = __ffma2_rn(dy, cz, a[8]);
-    a[9] = __ffma2_rn(dz, cx, a[9]);
-    a[10] = __ffma2_rn(dz, cy, a[10]);
-    a[11] = __ffma2_rn(dz, cz, a[11]);
     a[12] = __ffma2_rn(r3, wx, a[12]);
     a[13] = __ffma2_rn(r3, wy, a[13]);
     a[14] = __ffma2_rn(r3, wz, a[14]);
+    cx = __fmul2_rn(cx, b3);
+    cy = __fmul2_rn(cy, b3);
+    cz = __fmul2_rn(cz, b3);
+    a[3] = __ffma2_rn(dx, cx, a[3]);
+    a[4] = __ffma2_rn(dx, cy, a[4]);
+    a[5] = __ffma2_rn(dx, cz, a[5]);
+    a[8] = __ffma2_rn(dy, cz, a[8]);
+    a[7] = __ffma2_rn(dy, cy, a[7]);
+    a[6] = __ffma2_rn(dy, cx, a[6]);
+    a[9] = __ffma2_rn(dz, cx, a[9]);
+    a[10] = __ffma2_rn(dz, cy, a[10]);
+    if (!NO_ZZ) a[11] = __ffma2_rn(dz, cz, a[11]);
   }
 }
 
@@ -347,14 +430,18 @@ __device__ __forceinline__ void sweep_pairs(const float4 (*Q)[kBlock / 2], int p
                                             float2 (*acc)[NA], float (*hi)[NH], float (*lo)[NH], const float* gtab) {
   constexpr bool ACC = (MODE == MODE_COMP);
   constexpr int FOLD = ACC ? 8 : NP;
+  // the compensated loop holds 90 to 96 registers (5 blocks per SM) when it is not unrolled;
+  // the plain one gains 1 % from two pairs per turn
+  constexpr int UN = ACC ? 1 : 2;
 #pragma unroll 1
   for (int j0 = 0; j0 < NP; j0 += FOLD) {
-#pragma unroll 2
+#pragma unroll UN
     for (int j = j0; j < j0 + FOLD; ++j) {
       const int p = p0 + j;
       const float4 q0 = Q[0][p], q1 = Q[1][p], q2 = Q[2][p], q3 = Q[3][p], q4 = Q[4][p];
 #pragma unroll
-      for (int k = 0; k < TPT; ++k) pair2<C, ACC, HAVE_TR, GRADS>(tt[k], q0, q1, q2, q3, q4, acc[k], gtab);
+      for (int k = 0; k < TPT; ++k)
+        pair2<C, ACC, HAVE_TR, GRADS, ACC>(tt[k], q0, q1, q2, q3, q4, acc[k], gtab);
     }
     if (ACC) {
 #pragma unroll
@@ -362,7 +449,7 @@ __device__ __forceinline__ void sweep_pairs(const float4 (*Q)[kBlock / 2], int p
         float a1[NA];
 #pragma unroll
         for (int c = 0; c < NA; ++c) a1[c] = acc[k][c].x + acc[k][c].y;
-        if (GRADS) fold_grads(a1);
+        if (GRADS) fold_grads<C, ACC>(a1);
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
           const float s = hi[k][c] + a1[c];
@@ -438,6 +525,7 @@ __device__ __forceinline__ bool half_is_far(const float4& slo, const float4& shi
 
 template <int C, int MODE, bool GRADS, bool HAVE_TR, int TPT, class T, class O>
 __global__ void __launch_bounds__(kBlock) k_pair(const PairArgs<T, O> a) {
+  static_assert(MODE == MODE_FP64 || MODE == MODE_DS, "PLAIN and COMPENSATED run in k_pair_f");
   constexpr bool ACC = SumComp<MODE>::value;
   constexpr bool CLASSIFY = (C == CORE_GAUSS || C == CORE_EXP);
   // accumulators during the sweep (the accurate mode adds the velocity sums' low parts)
@@ -503,7 +591,7 @@ __global__ void __launch_bounds__(kBlock) k_pair(const PairArgs<T, O> a) {
 #pragma unroll
   for (int k = 0; k < TPT; ++k) {
     const int idx = tbase + 32 * k;
-    if (!ACC && GRADS) fold_grads(acc[k]);
+    if (!ACC && GRADS) fold_grads<C>(acc[k]);
     if (a.partial) {
       if (ACC) {
         T* base = a.partial + (size_t)split * (2 * NC) * a.nt_pad;
@@ -529,13 +617,26 @@ __global__ void __launch_bounds__(kBlock) k_pair(const PairArgs<T, O> a) {
   }
 }
 
+// Blocks per SM asked of the compiler (0: its own choice).  The compensated Gaussian kernel
+// with gradients would take 124 registers (4 blocks); held to 5 blocks it spills 40 bytes outside the
+// pair loops and the 262,144-particle cloud goes from 102.8 to 98.0 ms (115.8 ms before
+// gauss2's table, rsq2 and the factored gradient).  RM compensated takes 90 (5 blocks) by
+// itself; 6 blocks (80 registers) were slower (5.58 against 5.49 ms at 65,536 particles).
+// The plain kernels with two targets per thread are held to the 128 registers of 4 blocks
+// (the batched ones would take 130 to 159).
+template <int C, int MODE, bool GRADS, int TPT> struct PairMinBlocks {
+  static constexpr int value = (C == CORE_GAUSS && MODE == MODE_COMP && GRADS && TPT == 1) ? 5
+                               : (MODE == MODE_PLAIN && GRADS && TPT == 2)                 ? 4
+                                                                                           : 0;
+};
+
 // k_pair for FP32 (PLAIN and COMPENSATED): the same blocks, tiles, far-field classification,
 // splits and epilogue, with the sweep in packed FP32 over pairs of sources.  The staged
 // tiles are double-buffered: the next tile is loaded into the other buffer before the
 // current one is swept, so one barrier per tile orders both (two, without the second
 // buffer, and the loads' latency in the open).
 template <int C, int MODE, bool GRADS, bool HAVE_TR, int TPT>
-__global__ void __launch_bounds__(kBlock) k_pair_f(const PairArgs<float, float> a) {
+__global__ void __launch_bounds__(kBlock, PairMinBlocks<C, MODE, GRADS, TPT>::value) k_pair_f(const PairArgs<float, float> a) {
   constexpr bool ACC = (MODE == MODE_COMP);
   constexpr bool CLASSIFY = (C == CORE_GAUSS || C == CORE_EXP);
   constexpr int NA = GRADS ? 15 : 3;
@@ -543,7 +644,7 @@ __global__ void __launch_bounds__(kBlock) k_pair_f(const PairArgs<float, float> 
   constexpr int NH = ACC ? NC : 1;
   __shared__ float4 QB[2][5][kBlock / 2];
   // the Gaussian core's polynomial table, read from shared memory by the near-field pairs
-  __shared__ __align__(16) float gsh[C == CORE_GAUSS ? kGaussPolyStride * kGaussPolyN : 1];
+  __shared__ __align__(16) float gsh[C == CORE_GAUSS ? kGaussTab : 1];
   const float* gtab = nullptr;
   if constexpr (C == CORE_GAUSS) {
     stage_gauss_table(gsh);   // visible after the first tile's __syncthreads
@@ -619,7 +720,7 @@ __global__ void __launch_bounds__(kBlock) k_pair_f(const PairArgs<float, float> 
     float a1[NA];
 #pragma unroll
     for (int c = 0; c < NA; ++c) a1[c] = acc[k][c].x + acc[k][c].y;
-    if (!ACC && GRADS) fold_grads(a1);
+    if (!ACC && GRADS) fold_grads<C>(a1);
     if (a.partial) {
       if (ACC) {
         float* base = a.partial + (size_t)split * (2 * NC) * a.nt_pad;
