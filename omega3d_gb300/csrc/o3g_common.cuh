@@ -66,8 +66,9 @@ struct DeviceFacts {
 };
 int32_t device_facts(DeviceFacts* f);
 
-// resident blocks per SM of `kernel` at `block` threads (cached)
-int32_t occupancy_blocks(const void* kernel, int block, int* nb);
+// resident blocks per SM of `kernel` at `block` threads and `dyn_smem` bytes of dynamic shared
+// memory (cached)
+int32_t occupancy_blocks(const void* kernel, int block, int* nb, size_t dyn_smem = 0);
 
 // optional timing of the main kernel of a call
 struct KernelTimer {

@@ -155,11 +155,7 @@ static int32_t noalloc_run(int ns, const float* sx, const float* sy, const float
   a.tperm = nullptr; a.tile_lo = tile_lo; a.tile_hi = tile_hi;
   k_pair_f<C, MODE, GRADS, HAVE_TR, TPT><<<dim3(pl.tblocks, pl.nsplit), kBlock, 0, st>>>(a);
   note_launch();
-  if (pl.nsplit > 1) {
-    k_reduce<NC, ACC, float, float><<<dim3((nt + 255) / 256, NC), 256, 0, st>>>(partial, pl.nsplit, nt, pl.nt_pad,
-                                                                                out, nullptr);
-    note_launch();
-  }
+  if (pl.nsplit > 1) launch_reduce<NC, ACC, float, float>(partial, pl.nsplit, nt, pl.nt_pad, out, nullptr, st);
   O3G_CUDA_TRY(cudaGetLastError());
   return O3G_OK;
 }

@@ -746,27 +746,65 @@ __global__ void __launch_bounds__(kBlock, PairMinBlocks<C, MODE, GRADS, TPT>::va
   }
 }
 
-// Sum the per-split partials in split order and add into the outputs.
+// Sums the per-split partials and adds them into the outputs.  blockDim.y threads share a
+// target's splits (each a contiguous run, then the runs in order: a fixed order, whatever the
+// scheduling), so that few targets with many splits still fill the GPU.  Compensated: (hi, lo)
+// pairs are added in double-single (two-sum), as exact as the double sums it replaces and on
+// FP32 instructions: GB300's FP64 adds made this kernel 389 us at 65,536 targets x 57 splits.
 template <int NC, bool ACC, class T, class O>
 __global__ void k_reduce(const T* __restrict__ partial, int nsplit, int nt, int nt_pad, OutPtrs<O> out,
                          const uint32_t* __restrict__ tperm) {
+  __shared__ T sh[2][256];
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  const int c = blockIdx.y;
-  if (idx >= nt) return;
-  O* p = out.p[c] + (tperm ? (int)tperm[idx] : idx);
-  if (ACC) {
-    double s = 0.0;
-    for (int k = 0; k < nsplit; ++k) {
-      const T* base = partial + (size_t)k * (2 * NC) * nt_pad;
-      s += (double)base[(size_t)c * nt_pad + idx];
-      s += (double)base[(size_t)(NC + c) * nt_pad + idx];
+  const int c = blockIdx.y, g = threadIdx.y, ng = blockDim.y;
+  const int per = (nsplit + ng - 1) / ng;
+  const int k0 = min(nsplit, g * per), k1 = min(nsplit, k0 + per);
+  T s = T(0), l = T(0);
+  if (idx < nt) {
+    const T* p = partial + ((size_t)k0 * (ACC ? 2 * NC : NC) + c) * nt_pad + idx;
+    const size_t step = (size_t)(ACC ? 2 * NC : NC) * nt_pad;
+#pragma unroll 4
+    for (int k = k0; k < k1; ++k, p += step) {
+      if constexpr (ACC) {
+        const dsf t = ds_two_sum(s, p[0]);
+        s = t.h;
+        l += t.l + p[(size_t)NC * nt_pad];
+      } else {
+        s += p[0];
+      }
     }
-    *p = (O)((double)*p + s);
-  } else {
-    T s = T(0);
-    for (int k = 0; k < nsplit; ++k) s += partial[((size_t)k * NC + c) * nt_pad + idx];
-    *p = (O)((T)*p + s);
   }
+  const int me = g * blockDim.x + threadIdx.x;
+  sh[0][me] = s;
+  sh[1][me] = l;
+  __syncthreads();
+  if (g != 0 || idx >= nt) return;
+  for (int k = 1; k < ng; ++k) {
+    const T v = sh[0][k * blockDim.x + threadIdx.x];
+    if constexpr (ACC) {
+      const dsf t = ds_two_sum(s, v);
+      s = t.h;
+      l += t.l + sh[1][k * blockDim.x + threadIdx.x];
+    } else {
+      s += v;
+    }
+  }
+  O* p = out.p[c] + (tperm ? (int)tperm[idx] : idx);
+  if (ACC) *p = (O)((double)*p + ((double)s + (double)l));
+  else     *p = (O)((T)*p + s);
+}
+template <int NC, bool ACC, class T, class O>
+void launch_reduce(const T* partial, int nsplit, int nt, int nt_pad, const OutPtrs<O>& out, const uint32_t* tperm,
+                   cudaStream_t st) {
+  // threads per target: one when the targets fill the GPU (4 at 16,384 targets x 64 splits read
+  // 256-byte rows and took 19.6 us against 13.4), up to 8 for a few thousand, which one thread
+  // each leaves waiting on its loads (1,280 panels x 171 splits: 59 us before)
+  int ng = 1;
+  while (ng < 8 && (long)nt * NC * ng < 100000 && nsplit >= 8 * ng) ng *= 2;
+  const int bx = 256 / ng;
+  k_reduce<NC, ACC, T, O><<<dim3((nt + bx - 1) / bx, NC), dim3(bx, ng), 0, st>>>(partial, nsplit, nt, nt_pad, out,
+                                                                               tperm);
+  note_launch();
 }
 
 // SoA -> packed float4/double4 sources, optionally gathered through perm
@@ -972,11 +1010,7 @@ int32_t run_points_points(int ns, const I* sx, const I* sy, const I* sz, const I
     k_pair<C, MODE, GRADS, HAVE_TR, TPT, T, O><<<grid, kBlock, 0, st>>>(a);
   note_launch();
   tm.end(st);
-  if (pl.nsplit > 1) {
-    dim3 rg((nt + 255) / 256, NC);
-    k_reduce<NC, ACC, T, O><<<rg, 256, 0, st>>>(partial, pl.nsplit, nt, pl.nt_pad, out, tperm);
-    note_launch();
-  }
+  if (pl.nsplit > 1) launch_reduce<NC, ACC, T, O>(partial, pl.nsplit, nt, pl.nt_pad, out, tperm, st);
   O3G_CUDA_TRY(cudaGetLastError());
   return O3G_OK;
 }

@@ -6,6 +6,7 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
+#include <tuple>
 #include <mutex>
 #include <utility>
 
@@ -90,17 +91,17 @@ int32_t workspace_get(cudaStream_t stream, size_t bytes, Workspace** out) {
   return O3G_OK;
 }
 
-int32_t occupancy_blocks(const void* kernel, int block, int* nb) {
+int32_t occupancy_blocks(const void* kernel, int block, int* nb, size_t dyn_smem) {
   static std::mutex mu;
-  static std::map<std::pair<const void*, int>, int> cache;
+  static std::map<std::tuple<const void*, int, int, size_t>, int> cache;
   int dev = -1;
   O3G_CUDA_TRY(cudaGetDevice(&dev));
   std::lock_guard<std::mutex> lk(mu);
-  auto key = std::make_pair(kernel, dev * 4096 + block);
+  const auto key = std::make_tuple(kernel, dev, block, dyn_smem);
   auto it = cache.find(key);
   if (it == cache.end()) {
     int n = 0;
-    O3G_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, block, 0));
+    O3G_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, block, dyn_smem));
     if (n < 1) n = 1;
     it = cache.emplace(key, n).first;
   }
