@@ -412,6 +412,527 @@ __global__ void __launch_bounds__(kPanelThreads) k_panel_lu(PanelArgs a) {
   if (nr > 0) stage_out(a.A + (size_t)a.k0 * a.ld + r0, a.ld, slab, R, nr, jb);
 }
 
+// ---- the panel factorisation in one thread-block cluster ---------------------------------
+// What bounds a panel is latency: one pivot exchange per column.  Through global memory
+// (k_panel_lu, 152 blocks) it costs 3.1 us a column; among the 16 blocks of one cluster the
+// candidates travel through distributed shared memory behind the hardware's cluster barrier.
+// The rows then have to fit 16 SMs: each thread keeps RPT = 2 rows of W = 64 columns in
+// registers, so up to 10,240 rows fit; a kNb-column panel is factored W columns at a time
+// (k_panel_next brings the second half up to date).  More rows than that go to k_panel_lu.
+//
+// Rows do not move while the sub-panel is factored: each thread tracks the position its row has
+// after the interchanges so far (LAPACK's order); the sub-panel's rows are stored there at
+// the end, and k_laswp moves the other columns'.  Pivot choice: largest |value|, lowest position on ties.
+// Inside, columns go in groups of kCpGroup.  Per column only the group's columns are touched:
+// the warps' candidates (redux), the block's candidate window sent to every block of the
+// cluster (st.async, which counts its bytes on the receiver's mbarrier), the same winner found
+// by every warp, the rank-1 update of the window.  Per group the pivot rows' other columns are
+// sent to every block, solved against the group's L (U12), and the rows take the rank-8 update
+// from registers and shared memory.
+// Measured (one GB300), factorisation at n = 10,240: 43.2 -> 31.5 ms.  Not kept: full
+// rows in every exchange with a rank-1 update of the whole width per column (2.3 us a column:
+// 500 instructions per warp and column, in series), the same fully unrolled (2.8 us: 300 KB of
+// code, fetched once), a cluster barrier instead of mbarriers (its release waits for the
+// finished columns' global stores).
+constexpr int kCpThreads = 320;
+constexpr int kCpWarps = kCpThreads / 32;
+constexpr int kCpMax = 16;                  // blocks per cluster
+constexpr int kCpGroup = 8;                 // columns between two updates of the rest
+constexpr int kCpW = 64, kCpRows = 2;       // columns of a sub-panel, rows per thread
+
+struct ClusterPanelArgs {
+  float* A;
+  long long ld;
+  int n, k0, c, w;        // matrix order, first column of the panel, of this sub-panel, its width
+  int* piv;
+  int* singular;
+  int* err;               // set when a wait runs out
+  const float* u;         // the rows of U above the sub-panel, (c - k0) x w column-major (k_panel_next)
+};
+template <int W, int RPT> struct ClusterShared {
+  static constexpr int R = W - kCpGroup;          // columns right of a group
+  float xch[2][kCpGroup][kCpMax][kCpGroup];       // the blocks' candidate windows, by group parity and column
+  float rows[2][kCpGroup][R];                     // the pivot rows' other columns, by group parity
+  float u12[2][kCpGroup][R];                      // the same after the solve
+  float own[kCpGroup][R];                         // those that this block sends
+  float cand[2][kCpGroup];                        // this block's candidate window, by column parity
+  uint2 head[2][kCpGroup][kCpMax];                // candidates' |value| bits + 1 (0: none) and positions
+  unsigned long long bar[3];                      // mbarriers: a column's candidates (by parity), a group's rows
+  unsigned wkey[2][kCpWarps], wpos[2][kCpWarps];
+  int ownk[kCpGroup];                             // the last group (+ 1) whose k-th pivot row is in this block
+  float done[W * RPT * kCpThreads];               // the finished columns
+};
+__device__ __forceinline__ unsigned cluster_rank() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ unsigned cluster_size() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ unsigned cluster_map(const void* p, unsigned rank) {
+  unsigned r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+  return r;
+}
+
+__device__ __forceinline__ void cluster_expect(unsigned bar, unsigned bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+// 8 bytes into another block's shared memory, counted there
+__device__ __forceinline__ void cluster_send(unsigned dst, unsigned v0, unsigned v1, unsigned bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];" ::"r"(dst),
+               "r"(v0), "r"(v1), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void cluster_send4(unsigned dst, const float4& v, unsigned bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(dst),
+               "r"(__float_as_uint(v.x)), "r"(__float_as_uint(v.y)), "r"(__float_as_uint(v.z)), "r"(__float_as_uint(v.w)),
+               "r"(bar)
+               : "memory");
+}
+// the largest key of the lanes and the lowest position among those that have it (0: none)
+__device__ __forceinline__ void best_of(unsigned& key, unsigned& pos) {
+  constexpr unsigned full = 0xffffffffu;
+  const unsigned m = __reduce_max_sync(full, key);
+  const unsigned eq = __ballot_sync(full, m != 0u && key == m);
+  // one lane, almost always
+  pos = __popc(eq) == 1 ? __shfl_sync(full, pos, __ffs(eq) - 1) : __reduce_min_sync(full, m != 0u && key == m ? pos : full);
+  key = m;
+}
+// waits (bounded) for the mbarrier's phase; every thread for itself.  All blocks of a cluster are
+// resident, so it can only run out if one of them faults.
+__device__ __forceinline__ bool cluster_wait(unsigned bar, unsigned parity, int* err) {
+  for (unsigned it = 0; it < (1u << 21); ++it) {   // each try suspends for 1 us at most
+    unsigned done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 1000;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (done) return true;
+  }
+  atomicExch(err, 1);
+  return false;
+}
+
+// rank-kCpGroup update of the columns [kCpGroup, V) of the rows' windows: row by row the
+// multipliers are x[q][0..kCpGroup), but a pivot row of this group takes only the earlier ones
+// and a finished row none.  (Rolled over k, the multipliers turning through x[.][0].)
+template <int V, int W, int RPT>
+__device__ __forceinline__ void panel_update(float (*x)[W], const int* pos, int cg, const float (*u12)[W - kCpGroup]) {
+  constexpr int B = kCpGroup;
+#pragma unroll 1
+  for (int k = 0; k < B; ++k) {
+    float l[RPT];
+#pragma unroll
+    for (int q = 0; q < RPT; ++q) l[q] = pos[q] > cg + k ? x[q][0] : 0.f;
+#pragma unroll
+    for (int v = 0; v < (V - B) / 4; ++v) {
+      const float4 u = reinterpret_cast<const float4*>(u12[k])[v];
+#pragma unroll
+      for (int q = 0; q < RPT; ++q) {
+        float* y = &x[q][B + 4 * v];
+        y[0] = fmaf(-l[q], u.x, y[0]);
+        y[1] = fmaf(-l[q], u.y, y[1]);
+        y[2] = fmaf(-l[q], u.z, y[2]);
+        y[3] = fmaf(-l[q], u.w, y[3]);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < RPT; ++q) {
+      const float t = x[q][0];
+#pragma unroll
+      for (int e = 0; e + 1 < B; ++e) x[q][e] = x[q][e + 1];
+      x[q][B - 1] = t;
+    }
+  }
+}
+
+// One group of columns; x[.][0..W) is the window that starts at the group's first column.  The
+// finished columns are kept in shared memory and the window slides on.
+template <int W, int RPT>
+__device__ __forceinline__ void panel_group(const ClusterPanelArgs& a, ClusterShared<W, RPT>& sh, float (*x)[W], int* pos,
+                                            int row0, int g0, unsigned rank, unsigned C, bool& dead) {
+  constexpr unsigned full = 0xffffffffu;
+  constexpr int B = kCpGroup, R = W - B;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int cg = a.c + g0, gp = (g0 / B) & 1;
+  const int nb = min(B, a.w - g0);
+  unsigned win = 0u;   // the winners' blocks, 4 bits each
+  // one copy of the column's code (unrolled eight times, fetching it took longer than running
+  // it): the current column is always x[.][0], and the group's window turns by one per column
+#pragma unroll 1
+  for (int jj = 0; jj < B; ++jj) {
+    if (jj < nb) {
+    const int cj = cg + jj, par = jj & 1;
+    // this thread's candidate, the warp's, the block's
+    unsigned key = 0u, mp = full;
+    int mq = 0;
+#pragma unroll
+    for (int q = 0; q < RPT; ++q) {
+      const float v = fabsf(x[q][0]);
+      const unsigned kq = pos[q] >= cj && v >= 0.f ? __float_as_uint(v) + 1u : 0u;   // NaN: no candidate
+      if (kq > key || (kq == key && kq != 0u && (unsigned)pos[q] < mp)) { key = kq; mp = (unsigned)pos[q]; mq = q; }
+    }
+    unsigned m = key, p = mp;
+    best_of(m, p);
+    // (wkey and wpos are double-buffered: a warp may be through this column's wait while
+    // another still reads them)
+    if (lane == 0) { sh.wkey[par][warp] = m; sh.wpos[par][warp] = p; }
+    const unsigned mw = m, pw_ = p;
+    __syncthreads();
+    m = lane < kCpWarps ? sh.wkey[par][lane] : 0u;
+    p = lane < kCpWarps ? sh.wpos[par][lane] : full;
+    best_of(m, p);
+    if (m != 0u ? (mw == m && pw_ == p) : warp == 0) {
+      // this warp holds the block's candidate: its window and head to every block
+      if (m != 0u && key == m && mp == p) {
+#pragma unroll
+        for (int v = 0; v < B / 4; ++v) {
+          float4 r = make_float4(x[0][4 * v], x[0][4 * v + 1], x[0][4 * v + 2], x[0][4 * v + 3]);
+#pragma unroll
+          for (int q = 1; q < RPT; ++q)
+            if (mq == q) r = make_float4(x[q][4 * v], x[q][4 * v + 1], x[q][4 * v + 2], x[q][4 * v + 3]);
+          reinterpret_cast<float4*>(sh.cand[par])[v] = r;
+        }
+      }
+      __syncwarp();
+      const int to = lane & 15, h = lane >> 4;
+      if (to < (int)C) {
+        const unsigned bar = cluster_map(&sh.bar[par], to);
+        cluster_send4(cluster_map(&sh.xch[gp][jj][rank][4 * h], to), reinterpret_cast<const float4*>(sh.cand[par])[h], bar);
+        if (h == 0) cluster_send(cluster_map(&sh.head[gp][jj][rank], to), m, p, bar);
+      }
+    }
+    const unsigned bar = (unsigned)__cvta_generic_to_shared(&sh.bar[par]);
+    if (tid == 0) cluster_expect(bar, C * (B * 4 + 8));
+    if (!dead) dead = !cluster_wait(bar, (unsigned)((g0 + jj) >> 1) & 1u, a.err);
+    // the cluster's pivot, found by every warp alike
+    const uint2 hd = lane < (int)C ? sh.head[gp][jj][lane] : make_uint2(0u, full);
+    m = hd.x;
+    p = hd.y;
+    best_of(m, p);
+    const unsigned hit = __ballot_sync(full, m != 0u && hd.x == m && hd.y == p);
+    const unsigned wb = hit ? (unsigned)__ffs(hit) - 1u : 0u;
+    win |= wb << (4 * jj);
+    const float* u = sh.xch[gp][jj][wb];
+    // no finite candidate (or a wait that ran out): keep the row
+    const int pw = m != 0u && !dead && (int)p >= cj && (int)p < a.n ? (int)p : cj;
+    const float pv = m > 1u ? u[0] : 0.f;
+    if (rank == 0 && tid == 0) {
+      a.piv[cj] = pw;
+      if (m <= 1u && *a.singular == 0) *a.singular = cj + 1;
+    }
+#pragma unroll
+    for (int q = 0; q < RPT; ++q) {
+      if (pos[q] == cj) pos[q] = pw;
+      else if (pos[q] == pw) pos[q] = cj;
+    }
+    if (pv != 0.f) {
+      float ue[B];
+#pragma unroll
+      for (int v = 0; v < B / 4; ++v) {
+        const float4 uv = reinterpret_cast<const float4*>(u)[v];
+        ue[4 * v] = uv.x; ue[4 * v + 1] = uv.y; ue[4 * v + 2] = uv.z; ue[4 * v + 3] = uv.w;
+      }
+      // the finished columns at the window's end take no update
+#pragma unroll
+      for (int k = 1; k < B; ++k)
+        if (k >= B - jj) ue[k] = 0.f;
+      // x / pv by the reciprocal and one correction (the quotient to within an ulp) where nothing
+      // overflows on the way; the division itself otherwise
+      const float ap = fabsf(pv);
+      const bool mid = ap > 1e-30f && ap < 1e30f;
+      const float rp = mid ? __frcp_rn(pv) : 0.f;
+#pragma unroll
+      for (int q = 0; q < RPT; ++q)
+        if (pos[q] > cj) {
+          float l;
+          if (mid) {
+            l = x[q][0] * rp;
+            l = fmaf(fmaf(-l, pv, x[q][0]), rp, l);
+          } else {
+            l = x[q][0] / pv;
+          }
+          x[q][0] = l;
+#pragma unroll
+          for (int k = 1; k < B; ++k) x[q][k] = fmaf(-l, ue[k], x[q][k]);
+        }
+    }
+    }
+#pragma unroll
+    for (int q = 0; q < RPT; ++q) {
+      const float t = x[q][0];
+#pragma unroll
+      for (int k = 0; k + 1 < B; ++k) x[q][k] = x[q][k + 1];
+      x[q][B - 1] = t;
+    }
+  }
+  if (g0 + B < a.w) {
+    // the group's pivot rows, right of it, to every block
+#pragma unroll
+    for (int q = 0; q < RPT; ++q) {
+      const int k = pos[q] - cg;
+      if (k >= 0 && k < B) {
+        sh.ownk[k] = g0 + 1;
+#pragma unroll
+        for (int v = 0; v < R / 4; ++v)
+          reinterpret_cast<float4*>(sh.own[k])[v] =
+              make_float4(x[q][B + 4 * v], x[q][B + 4 * v + 1], x[q][B + 4 * v + 2], x[q][B + 4 * v + 3]);
+      }
+    }
+    __syncthreads();
+    for (int e = warp; e < B * (int)C; e += kCpWarps) {   // a warp per row and destination
+      const int k = e % B, to = e / B;
+      if (sh.ownk[k] == g0 + 1 && lane < R / 4)
+        cluster_send4(cluster_map(&sh.rows[gp][k][4 * lane], to), reinterpret_cast<const float4*>(sh.own[k])[lane],
+                      cluster_map(&sh.bar[2], to));
+    }
+    const unsigned bar = (unsigned)__cvta_generic_to_shared(&sh.bar[2]);
+    if (tid == 0) cluster_expect(bar, B * R * 4);
+    if (!dead) dead = !cluster_wait(bar, (unsigned)gp, a.err);
+    // U12 = L11^-1 A12 of the group, a thread per column; L11 from the pivots' windows
+    if (tid < R) {
+      float uu[B];
+#pragma unroll
+      for (int k = 0; k < B; ++k) {
+        // the k-th pivot's window starts at its own column: its multipliers e < k are at B - k + e
+        const float* lk = sh.xch[gp][k][(win >> (4 * k)) & 15u];
+        float v = sh.rows[gp][k][tid];
+#pragma unroll
+        for (int e = 0; e < k; ++e) v = fmaf(-lk[B - k + e], uu[e], v);
+        uu[k] = v;
+        sh.u12[gp][k][tid] = v;
+      }
+    }
+    __syncthreads();
+    if (g0 < W / 2) panel_update<W, W, RPT>(x, pos, cg, sh.u12[gp]);
+    else            panel_update<W / 2, W, RPT>(x, pos, cg, sh.u12[gp]);
+  }
+#pragma unroll
+  for (int q = 0; q < RPT; ++q) {
+#pragma unroll
+    for (int jj = 0; jj < B; ++jj) sh.done[((g0 + jj) * RPT + q) * kCpThreads + tid] = x[q][jj];
+#pragma unroll
+    for (int k = 0; k < W; ++k) x[q][k] = k + B < W ? x[q][k + B] : 0.f;
+  }
+}
+
+template <int W, int RPT>
+__global__ void __launch_bounds__(kCpThreads, 1) k_panel_cluster(const ClusterPanelArgs a) {
+  extern __shared__ __align__(16) char cpsm[];
+  static_assert(kNb % W == 0 && W % 16 == 0, "whole sub-panels and groups");
+  using Sh = ClusterShared<W, RPT>;
+  static_assert(offsetof(Sh, rows) % 16 == 0 && offsetof(Sh, u12) % 16 == 0 &&
+                    offsetof(Sh, own) % 16 == 0 && offsetof(Sh, cand) % 16 == 0 && (W - kCpGroup) % 4 == 0 &&
+                    offsetof(Sh, xch) % 16 == 0 && offsetof(Sh, head) % 8 == 0 && offsetof(Sh, bar) % 8 == 0,
+                "vector accesses");
+  static_assert(kCpMax <= 16 && kCpGroup == 8 && (W - kCpGroup) / 4 <= 32, "lanes per destination");
+  static_assert(W - kCpGroup <= kCpThreads, "a thread per column of U12");
+  ClusterShared<W, RPT>& sh = *reinterpret_cast<ClusterShared<W, RPT>*>(cpsm);
+  const int tid = threadIdx.x;
+  const unsigned rank = cluster_rank(), C = cluster_size();
+  const int c = a.c, w = a.w, kp = a.c - a.k0;
+  const int row0 = c + (int)rank * (kCpThreads * RPT) + tid;   // this thread's rows: row0 + q kCpThreads
+  float x[RPT][W];
+  int pos[RPT];
+#pragma unroll
+  for (int q = 0; q < RPT; ++q) {
+    const int r = row0 + q * kCpThreads;
+    const bool in = r < a.n;
+    pos[q] = in ? r : -1;
+#pragma unroll
+    for (int k = 0; k < W; ++k) x[q][k] = in && k < w ? a.A[(size_t)(c + k) * a.ld + r] : 0.f;
+  }
+  if (tid < kCpGroup) sh.ownk[tid] = 0;
+  if (tid == 0) {
+#pragma unroll
+    for (int b = 0; b < 3; ++b)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((unsigned)__cvta_generic_to_shared(&sh.bar[b])) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  // the rows of U above this sub-panel (k_panel_next)
+  if (rank == 0)
+    for (int e = tid; e < kp * w; e += kCpThreads)
+      a.A[(size_t)(c + e / kp) * a.ld + a.k0 + e % kp] = a.u[e];
+  cluster_barrier();   // every block runs: its shared memory may be written
+  bool dead = false;
+#pragma unroll 1
+  for (int g0 = 0; g0 < w; g0 += kCpGroup) panel_group<W, RPT>(a, sh, x, pos, row0, g0, rank, C, dead);
+  // every row to the place the interchanges gave it
+#pragma unroll 4
+  for (int k = 0; k < w; ++k)
+#pragma unroll
+    for (int q = 0; q < RPT; ++q)
+      if (pos[q] >= 0) a.A[(size_t)(c + k) * a.ld + pos[q]] = sh.done[(k * RPT + q) * kCpThreads + tid];
+  cluster_barrier();   // no block leaves while another may still write to its shared memory
+}
+
+// Before a later sub-panel [c, c + w) of a panel: U = L11^-1 A12 for the rows [k0, c) and
+// A22 -= L21 U for the rows below, in FP32 on all SMs (kp = c - k0 and w at most 64).  Every block
+// solves U for itself (a warp per column, 8 side by side) and updates 64 rows; block 0 keeps U
+// in `u` (kp x w), from where the sub-panel's factorisation stores it: in A other blocks still
+// read A12.
+constexpr int kNextRows = 64, kNextMax = 64, kNextLd = kNextMax + 4;
+struct PanelNextShared {
+  alignas(16) float L11[kNextMax * kNextMax];     // column-major
+  alignas(16) float U[kNextMax][kNextLd];         // [k][column]
+  alignas(16) float L21[kNextMax][kNextLd];       // [k][row]
+};
+__global__ void __launch_bounds__(256) k_panel_next(float* A, long long ld, int n, int k0, int kp, int w, float* u) {
+  extern __shared__ __align__(16) char pnsm[];
+  PanelNextShared& sh = *reinterpret_cast<PanelNextShared*>(pnsm);
+  constexpr unsigned full = 0xffffffffu;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, c = k0 + kp;
+  const int r0 = c + blockIdx.x * kNextRows, nr = min(kNextRows, n - r0);
+  stage_in(sh.L11, kp, A + (size_t)k0 * ld + k0, ld, kp, kp);
+  constexpr int NQ = kNextMax / 8, NL = kNextMax / 32;
+  float y[NQ][NL];
+#pragma unroll
+  for (int t = 0; t < NQ; ++t)
+#pragma unroll
+    for (int b = 0; b < NL; ++b) {
+      const int col = warp + 8 * t, m = 32 * b + lane;
+      y[t][b] = col < w && m < kp ? A[(size_t)(c + col) * ld + k0 + m] : 0.f;
+    }
+  // L21: 64 rows x kp columns, 16 loads in flight per thread
+  {
+    float v[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const int e = tid + 256 * i, k = e / kNextRows, r = e % kNextRows;
+      v[i] = k < kp && r < nr ? A[(size_t)(k0 + k) * ld + r0 + r] : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const int e = tid + 256 * i;
+      sh.L21[e / kNextRows][e % kNextRows] = v[i];
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int b = 0; b < NL; ++b) {
+#pragma unroll 4
+    for (int il = 0; il < 32; ++il) {
+      const int i = 32 * b + il;
+      if (i >= kp) break;
+      float lc[NL];
+#pragma unroll
+      for (int e = b; e < NL; ++e) {
+        const int m = 32 * e + lane;
+        lc[e] = m > i && m < kp ? sh.L11[(size_t)i * kp + m] : 0.f;
+      }
+#pragma unroll
+      for (int t = 0; t < NQ; ++t) {
+        const float yi = __shfl_sync(full, y[t][b], il);
+#pragma unroll
+        for (int e = b; e < NL; ++e) y[t][e] = fmaf(-lc[e], yi, y[t][e]);
+      }
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < NQ; ++t)
+#pragma unroll
+    for (int b = 0; b < NL; ++b) {
+      const int col = warp + 8 * t, m = 32 * b + lane;
+      sh.U[m][col] = y[t][b];
+      if (blockIdx.x == 0 && col < w && m < kp) u[(size_t)col * kp + m] = y[t][b];
+    }
+  __syncthreads();
+  // thread (tr, tc) of 16 x 16: rows 4 tr .. + 3, columns 4 tc .. + 3
+  const int tr = tid & 15, tc = tid >> 4;
+  float acc[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int r = 4 * tr + i, col = 4 * tc + q;
+      acc[i][q] = r < nr && col < w ? A[(size_t)(c + col) * ld + r0 + r] : 0.f;
+    }
+#pragma unroll 4
+  for (int k = 0; k < kp; ++k) {
+    const float4 l = *reinterpret_cast<const float4*>(&sh.L21[k][4 * tr]);
+    const float4 v = *reinterpret_cast<const float4*>(&sh.U[k][4 * tc]);
+    const float le[4] = {l.x, l.y, l.z, l.w}, ve[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) acc[i][q] = fmaf(-le[i], ve[q], acc[i][q]);
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int r = 4 * tr + i, col = 4 * tc + q;
+      if (r < nr && col < w) A[(size_t)(c + col) * ld + r0 + r] = acc[i][q];
+    }
+}
+
+// The cluster kernel for m rows, or nothing when they do not fit: sub-panel width, blocks
+struct ClusterPlan {
+  const void* kernel = nullptr;
+  int width = 0, blocks = 0;
+  size_t smem = 0;
+};
+// the largest cluster of the variant that can be resident on this device (0: none); sets the
+// kernel's attributes, once per factorisation
+template <int W, int RPT> static int32_t cluster_setup_of(int* largest) {
+  const void* k = (const void*)&k_panel_cluster<W, RPT>;
+  const size_t smem = sizeof(ClusterShared<W, RPT>);
+  O3G_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  O3G_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  *largest = 0;
+  for (int c = kCpMax; c >= 1 && *largest == 0; c /= 2) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(c);
+    cfg.blockDim = dim3(kCpThreads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = c;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int nc = 0;
+    if (cudaOccupancyMaxActiveClusters(&nc, k, &cfg) == cudaSuccess && nc > 0) *largest = c;
+    else (void)cudaGetLastError();
+  }
+  return O3G_OK;
+}
+template <int W, int RPT> static bool cluster_fits(int m, int cmax, ClusterPlan* p) {
+  int c = 1;
+  while (c < cmax && c * kCpThreads * RPT < m) c *= 2;
+  if (cmax == 0 || c * kCpThreads * RPT < m) return false;
+  p->kernel = (const void*)&k_panel_cluster<W, RPT>;
+  p->width = W;
+  p->blocks = c;
+  p->smem = sizeof(ClusterShared<W, RPT>);
+  return true;
+}
+static int32_t launch_cluster_panel(const ClusterPlan& p, ClusterPanelArgs a, cudaStream_t st) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(p.blocks);
+  cfg.blockDim = dim3(kCpThreads);
+  cfg.dynamicSmemBytes = p.smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = p.blocks;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  void* args[] = {&a};
+  O3G_CUDA_TRY(cudaLaunchKernelExC(&cfg, p.kernel, args));
+  note_launch();
+  return O3G_OK;
+}
+
 // row interchanges p0..p1-1 (piv) applied to the columns [c0, c1) outside [s0, s1).  Each
 // block first composes the interchanges into one permutation of the rows they touch (the
 // np rows [p0, p1) and the distinct pivot rows below p1): slot s holds row rowof[s], and
@@ -1061,6 +1582,7 @@ extern "C" int32_t o3g_bem_factor(o3g_bem_t* h, void* stream) {
   O3G_CUDA_TRY(cudaFuncGetAttributes(&fa, k_panel_lu));
   const size_t max_smem = (size_t)optin - fa.sharedSizeBytes;
   O3G_CUDA_TRY(cudaFuncSetAttribute(k_panel_lu, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem));
+  // panels of up to 40,960 rows run in one cluster (k_panel_cluster); this sizes k_panel_lu
   int G = std::min(df.num_sms, 32 * kMaxKeysPerLane);
   int R = (n + G - 1) / G;
   size_t smem = ((size_t)kNb * R + 2 * kNb + 32) * sizeof(float);
@@ -1140,6 +1662,10 @@ extern "C" int32_t o3g_bem_factor(o3g_bem_t* h, void* stream) {
     note_launch();
   };
   auto at = [&](int r, int c) { return h->LU + (size_t)c * ld + r; };
+  int cmax = 0;
+  O3G_TRY((cluster_setup_of<kCpW, kCpRows>(&cmax)));
+  O3G_CUDA_TRY(cudaFuncSetAttribute(k_panel_next, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PanelNextShared)));
+  static_assert(kNb == 2 * kCpW && kCpW <= kNextMax, "at most one earlier sub-panel");
   // two-level right-looking LU: kNb-column panels inside kNbOuter-column outer panels; the
   // big trailing update of each outer panel has k = kNbOuter
   for (int K0 = 0; K0 < n; K0 += kNbOuter) {
@@ -1147,24 +1673,43 @@ extern "C" int32_t o3g_bem_factor(o3g_bem_t* h, void* stream) {
     for (int k0 = K0; k0 < K1; k0 += kNb) {
       const int jb = std::min(kNb, K1 - k0);
       const int m = n - k0;
-      int g = G;
-      int r = (m + g - 1) / g;
-      if (r < 32) {   // short panels: fewer blocks
-        g = (m + 31) / 32;
-        r = (m + g - 1) / g;
+      // the debug wait test (o3g_debug_wait_test) needs a kernel that polls
+      ClusterPlan cp;
+      if (!wait_test_on()) (void)cluster_fits<kCpW, kCpRows>(m, cmax, &cp);
+      if (cp.kernel) {
+        for (int c = k0; c < k0 + jb; c += cp.width) {
+          ClusterPanelArgs ca;
+          ca.A = h->LU; ca.ld = ld; ca.n = n; ca.k0 = k0; ca.c = c; ca.w = std::min(cp.width, k0 + jb - c);
+          ca.piv = h->piv; ca.singular = h->flags + 1; ca.err = h->flags;
+          ca.u = linv;
+          if (c > k0) {
+            k_panel_next<<<(n - c + kNextRows - 1) / kNextRows, 256, sizeof(PanelNextShared), st>>>(h->LU, ld, n, k0, c - k0,
+                                                                                               ca.w, linv);
+            note_launch();
+          }
+          O3G_TRY(launch_cluster_panel(cp, ca, st));
+          laswp(c, c + ca.w, K0, K1, c, c + ca.w);
+        }
+      } else {
+        int g = G;
+        int r = (m + g - 1) / g;
+        if (r < 32) {   // short panels: fewer blocks
+          g = (m + 31) / 32;
+          r = (m + g - 1) / g;
+        }
+        PanelArgs pa;
+        pa.A = h->LU; pa.ld = ld; pa.n = n; pa.k0 = k0; pa.jb = jb; pa.R = r;
+        pa.piv = h->piv; pa.keys = keys; pa.crows = crows; pa.drow = drow;
+        pa.singular = h->flags + 1;
+        pa.tag0 = (unsigned)(k0 / kNb + 1) << 7;   // panels numbered from 1: zeroed keys never match
+        pa.bar = make_barrier(h->flags);
+        void* args[] = {&pa};
+        const size_t sm = ((size_t)jb * r + 2 * jb + 32) * sizeof(float);
+        O3G_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)k_panel_lu, dim3(g), dim3(kPanelThreads), args, sm, st));
+        note_launch();
+        // interchanges inside the outer panel; the other columns get them once per outer panel
+        laswp(k0, k0 + jb, K0, K1, k0, k0 + jb);
       }
-      PanelArgs pa;
-      pa.A = h->LU; pa.ld = ld; pa.n = n; pa.k0 = k0; pa.jb = jb; pa.R = r;
-      pa.piv = h->piv; pa.keys = keys; pa.crows = crows; pa.drow = drow;
-      pa.singular = h->flags + 1;
-      pa.tag0 = (unsigned)(k0 / kNb + 1) << 7;   // panels numbered from 1: zeroed keys never match
-      pa.bar = make_barrier(h->flags);
-      void* args[] = {&pa};
-      const size_t sm = ((size_t)jb * r + 2 * jb + 32) * sizeof(float);
-      O3G_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)k_panel_lu, dim3(g), dim3(kPanelThreads), args, sm, st));
-      note_launch();
-      // interchanges inside the outer panel; the other columns get them once per outer panel
-      laswp(k0, k0 + jb, K0, K1, k0, k0 + jb);
       if (k0 + jb < K1) {
         trsm(k0, jb, k0 + jb, K1 - k0 - jb);
         O3G_TRY(gemm(n - k0 - jb, K1 - k0 - jb, jb, at(k0 + jb, k0), at(k0, k0 + jb), at(k0 + jb, k0 + jb)));
