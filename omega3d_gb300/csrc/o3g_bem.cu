@@ -570,101 +570,101 @@ __device__ __forceinline__ void panel_group(const ClusterPanelArgs& a, ClusterSh
 #pragma unroll 1
   for (int jj = 0; jj < B; ++jj) {
     if (jj < nb) {
-    const int cj = cg + jj, par = jj & 1;
-    // this thread's candidate, the warp's, the block's
-    unsigned key = 0u, mp = full;
-    int mq = 0;
+      const int cj = cg + jj, par = jj & 1;
+      // this thread's candidate, the warp's, the block's
+      unsigned key = 0u, mp = full;
+      int mq = 0;
 #pragma unroll
-    for (int q = 0; q < RPT; ++q) {
-      const float v = fabsf(x[q][0]);
-      const unsigned kq = pos[q] >= cj && v >= 0.f ? __float_as_uint(v) + 1u : 0u;   // NaN: no candidate
-      if (kq > key || (kq == key && kq != 0u && (unsigned)pos[q] < mp)) { key = kq; mp = (unsigned)pos[q]; mq = q; }
-    }
-    unsigned m = key, p = mp;
-    best_of(m, p);
-    // (wkey and wpos are double-buffered: a warp may be through this column's wait while
-    // another still reads them)
-    if (lane == 0) { sh.wkey[par][warp] = m; sh.wpos[par][warp] = p; }
-    const unsigned mw = m, pw_ = p;
-    __syncthreads();
-    m = lane < kCpWarps ? sh.wkey[par][lane] : 0u;
-    p = lane < kCpWarps ? sh.wpos[par][lane] : full;
-    best_of(m, p);
-    if (m != 0u ? (mw == m && pw_ == p) : warp == 0) {
-      // this warp holds the block's candidate: its window and head to every block
-      if (m != 0u && key == m && mp == p) {
+      for (int q = 0; q < RPT; ++q) {
+        const float v = fabsf(x[q][0]);
+        const unsigned kq = pos[q] >= cj && v >= 0.f ? __float_as_uint(v) + 1u : 0u;   // NaN: no candidate
+        if (kq > key || (kq == key && kq != 0u && (unsigned)pos[q] < mp)) { key = kq; mp = (unsigned)pos[q]; mq = q; }
+      }
+      unsigned m = key, p = mp;
+      best_of(m, p);
+      // (wkey and wpos are double-buffered: a warp may be through this column's wait while
+      // another still reads them)
+      if (lane == 0) { sh.wkey[par][warp] = m; sh.wpos[par][warp] = p; }
+      const unsigned mw = m, pw_ = p;
+      __syncthreads();
+      m = lane < kCpWarps ? sh.wkey[par][lane] : 0u;
+      p = lane < kCpWarps ? sh.wpos[par][lane] : full;
+      best_of(m, p);
+      if (m != 0u ? (mw == m && pw_ == p) : warp == 0) {
+        // this warp holds the block's candidate: its window and head to every block
+        if (m != 0u && key == m && mp == p) {
+#pragma unroll
+          for (int v = 0; v < B / 4; ++v) {
+            float4 r = make_float4(x[0][4 * v], x[0][4 * v + 1], x[0][4 * v + 2], x[0][4 * v + 3]);
+#pragma unroll
+            for (int q = 1; q < RPT; ++q)
+              if (mq == q) r = make_float4(x[q][4 * v], x[q][4 * v + 1], x[q][4 * v + 2], x[q][4 * v + 3]);
+            reinterpret_cast<float4*>(sh.cand[par])[v] = r;
+          }
+        }
+        __syncwarp();
+        const int to = lane & 15, h = lane >> 4;
+        if (to < (int)C) {
+          const unsigned bar = cluster_map(&sh.bar[par], to);
+          cluster_send4(cluster_map(&sh.xch[gp][jj][rank][4 * h], to), reinterpret_cast<const float4*>(sh.cand[par])[h], bar);
+          if (h == 0) cluster_send(cluster_map(&sh.head[gp][jj][rank], to), m, p, bar);
+        }
+      }
+      const unsigned bar = (unsigned)__cvta_generic_to_shared(&sh.bar[par]);
+      if (tid == 0) cluster_expect(bar, C * (B * 4 + 8));
+      if (!dead) dead = !cluster_wait(bar, (unsigned)((g0 + jj) >> 1) & 1u, a.err);
+      // the cluster's pivot, found by every warp alike
+      const uint2 hd = lane < (int)C ? sh.head[gp][jj][lane] : make_uint2(0u, full);
+      m = hd.x;
+      p = hd.y;
+      best_of(m, p);
+      const unsigned hit = __ballot_sync(full, m != 0u && hd.x == m && hd.y == p);
+      const unsigned wb = hit ? (unsigned)__ffs(hit) - 1u : 0u;
+      win |= wb << (4 * jj);
+      const float* u = sh.xch[gp][jj][wb];
+      // no finite candidate (or a wait that ran out): keep the row
+      const int pw = m != 0u && !dead && (int)p >= cj && (int)p < a.n ? (int)p : cj;
+      const float pv = m > 1u ? u[0] : 0.f;
+      if (rank == 0 && tid == 0) {
+        a.piv[cj] = pw;
+        if (m <= 1u && *a.singular == 0) *a.singular = cj + 1;
+      }
+#pragma unroll
+      for (int q = 0; q < RPT; ++q) {
+        if (pos[q] == cj) pos[q] = pw;
+        else if (pos[q] == pw) pos[q] = cj;
+      }
+      if (pv != 0.f) {
+        float ue[B];
 #pragma unroll
         for (int v = 0; v < B / 4; ++v) {
-          float4 r = make_float4(x[0][4 * v], x[0][4 * v + 1], x[0][4 * v + 2], x[0][4 * v + 3]);
-#pragma unroll
-          for (int q = 1; q < RPT; ++q)
-            if (mq == q) r = make_float4(x[q][4 * v], x[q][4 * v + 1], x[q][4 * v + 2], x[q][4 * v + 3]);
-          reinterpret_cast<float4*>(sh.cand[par])[v] = r;
+          const float4 uv = reinterpret_cast<const float4*>(u)[v];
+          ue[4 * v] = uv.x; ue[4 * v + 1] = uv.y; ue[4 * v + 2] = uv.z; ue[4 * v + 3] = uv.w;
         }
-      }
-      __syncwarp();
-      const int to = lane & 15, h = lane >> 4;
-      if (to < (int)C) {
-        const unsigned bar = cluster_map(&sh.bar[par], to);
-        cluster_send4(cluster_map(&sh.xch[gp][jj][rank][4 * h], to), reinterpret_cast<const float4*>(sh.cand[par])[h], bar);
-        if (h == 0) cluster_send(cluster_map(&sh.head[gp][jj][rank], to), m, p, bar);
-      }
-    }
-    const unsigned bar = (unsigned)__cvta_generic_to_shared(&sh.bar[par]);
-    if (tid == 0) cluster_expect(bar, C * (B * 4 + 8));
-    if (!dead) dead = !cluster_wait(bar, (unsigned)((g0 + jj) >> 1) & 1u, a.err);
-    // the cluster's pivot, found by every warp alike
-    const uint2 hd = lane < (int)C ? sh.head[gp][jj][lane] : make_uint2(0u, full);
-    m = hd.x;
-    p = hd.y;
-    best_of(m, p);
-    const unsigned hit = __ballot_sync(full, m != 0u && hd.x == m && hd.y == p);
-    const unsigned wb = hit ? (unsigned)__ffs(hit) - 1u : 0u;
-    win |= wb << (4 * jj);
-    const float* u = sh.xch[gp][jj][wb];
-    // no finite candidate (or a wait that ran out): keep the row
-    const int pw = m != 0u && !dead && (int)p >= cj && (int)p < a.n ? (int)p : cj;
-    const float pv = m > 1u ? u[0] : 0.f;
-    if (rank == 0 && tid == 0) {
-      a.piv[cj] = pw;
-      if (m <= 1u && *a.singular == 0) *a.singular = cj + 1;
-    }
+        // the finished columns at the window's end take no update
 #pragma unroll
-    for (int q = 0; q < RPT; ++q) {
-      if (pos[q] == cj) pos[q] = pw;
-      else if (pos[q] == pw) pos[q] = cj;
-    }
-    if (pv != 0.f) {
-      float ue[B];
+        for (int k = 1; k < B; ++k)
+          if (k >= B - jj) ue[k] = 0.f;
+        // x / pv by the reciprocal and one correction (the quotient to within an ulp) where nothing
+        // overflows on the way; the division itself otherwise
+        const float ap = fabsf(pv);
+        const bool mid = ap > 1e-30f && ap < 1e30f;
+        const float rp = mid ? __frcp_rn(pv) : 0.f;
 #pragma unroll
-      for (int v = 0; v < B / 4; ++v) {
-        const float4 uv = reinterpret_cast<const float4*>(u)[v];
-        ue[4 * v] = uv.x; ue[4 * v + 1] = uv.y; ue[4 * v + 2] = uv.z; ue[4 * v + 3] = uv.w;
-      }
-      // the finished columns at the window's end take no update
+        for (int q = 0; q < RPT; ++q)
+          if (pos[q] > cj) {
+            float l;
+            if (mid) {
+              l = x[q][0] * rp;
+              l = fmaf(fmaf(-l, pv, x[q][0]), rp, l);
+            } else {
+              l = x[q][0] / pv;
+            }
+            x[q][0] = l;
 #pragma unroll
-      for (int k = 1; k < B; ++k)
-        if (k >= B - jj) ue[k] = 0.f;
-      // x / pv by the reciprocal and one correction (the quotient to within an ulp) where nothing
-      // overflows on the way; the division itself otherwise
-      const float ap = fabsf(pv);
-      const bool mid = ap > 1e-30f && ap < 1e30f;
-      const float rp = mid ? __frcp_rn(pv) : 0.f;
-#pragma unroll
-      for (int q = 0; q < RPT; ++q)
-        if (pos[q] > cj) {
-          float l;
-          if (mid) {
-            l = x[q][0] * rp;
-            l = fmaf(fmaf(-l, pv, x[q][0]), rp, l);
-          } else {
-            l = x[q][0] / pv;
+            for (int k = 1; k < B; ++k) x[q][k] = fmaf(-l, ue[k], x[q][k]);
           }
-          x[q][0] = l;
-#pragma unroll
-          for (int k = 1; k < B; ++k) x[q][k] = fmaf(-l, ue[k], x[q][k]);
-        }
-    }
+      }
     }
 #pragma unroll
     for (int q = 0; q < RPT; ++q) {
@@ -1121,31 +1121,23 @@ __global__ void k_permute_to_float(const double* r, const int* perm, float* y, i
   if (i < n) y[i] = (float)r[perm[i]];
 }
 
-// sum_m col[m*ld] * yd[m] for m < jb; the full-width case is unrolled so every load of the
-// row is in flight at once (the loop is latency-bound otherwise)
-__device__ __forceinline__ float panel_dot(const float* __restrict__ col, long long ld, const float* yd, int jb) {
-  if (jb == kNb) {
-    float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-    for (int m = 0; m < kNb; ++m) s[m & 7] = fmaf(__ldg(col + (size_t)m * ld), yd[m], s[m & 7]);
-    return ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
-  }
-  float s = 0.f;
-  for (int m = 0; m < jb; ++m) s = fmaf(col[(size_t)m * ld], yd[m], s);
-  return s;
-}
-
-// Inverses of the diagonal kNb x kNb blocks of the factors, one block per CUDA block:
-// Linv (unit lower) and Uinv (upper) column-major at dinv + kb*2*kNb*kNb (+kNb*kNb).
-// Columns of the identity are solved by one warp each (forward / back substitution).
+// Inverses of the diagonal blocks of the factors.  The solves use blocks of kDb columns: block b
+// has its unit lower inverse at dinv + b 2 kDb^2 and its upper one kDb^2 further, both
+// column-major with leading dimension kDb.  k_diag_inverses inverts the kNb x kNb blocks on
+// their diagonals (one per CUDA block: columns of the identity, solved by one warp each),
+// k_diag_merge fills in the blocks beside them.  The other triangles off those blocks are never
+// written nor read.
+constexpr int kDb = 512;
+constexpr int kDbSub = kDb / kNb;
+__host__ __device__ inline size_t dinv_floats(int n) { return (size_t)((n + kDb - 1) / kDb) * 2 * kDb * kDb; }
 __global__ void __launch_bounds__(256) k_diag_inverses(const float* __restrict__ LU, long long ld, int n,
                                                        float* __restrict__ dinv) {
   extern __shared__ float D[];   // [jb][jb] diagonal block
   const int kb = blockIdx.x, k0 = kb * kNb, jb = min(kNb, n - k0);
   stage_in(D, jb, LU + (size_t)k0 * ld + k0, ld, jb, jb);
   __syncthreads();
-  float* Li = dinv + (size_t)kb * 2 * kNb * kNb;
-  float* Ui = Li + (size_t)kNb * kNb;
+  float* Li = dinv + (size_t)(kb / kDbSub) * 2 * kDb * kDb + (size_t)(kb % kDbSub) * kNb * (kDb + 1);
+  float* Ui = Li + (size_t)kDb * kDb;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int c = warp; c < jb; c += blockDim.x / 32) {
     float x[kNb / 32];
@@ -1163,7 +1155,7 @@ __global__ void __launch_bounds__(256) k_diag_inverses(const float* __restrict__
 #pragma unroll
     for (int q = 0; q < kNb / 32; ++q) {
       const int m = q * 32 + lane;
-      if (m < kNb) Li[(size_t)c * kNb + m] = m < jb ? x[q] : 0.f;
+      if (m < kNb) Li[(size_t)c * kDb + m] = m < jb ? x[q] : 0.f;
     }
     // U x = e_c
 #pragma unroll
@@ -1180,66 +1172,95 @@ __global__ void __launch_bounds__(256) k_diag_inverses(const float* __restrict__
 #pragma unroll
     for (int q = 0; q < kNb / 32; ++q) {
       const int m = q * 32 + lane;
-      if (m < kNb) Ui[(size_t)c * kNb + m] = m < jb ? x[q] : 0.f;
+      if (m < kNb) Ui[(size_t)c * kDb + m] = m < jb ? x[q] : 0.f;
     }
   }
 }
 
-// yd = Dinv y[k0 : k0+jb] (Dinv kNb x kNb column-major) by the whole block
-__device__ __forceinline__ void diag_apply(const float* __restrict__ Dinv, const float* y, int jb, float* yin,
-                                           float* part, float* yd) {
-  if (threadIdx.x < jb) yin[threadIdx.x] = y[threadIdx.x];
-  __syncthreads();
-  constexpr int kQ = kSolveThreads / kNb;   // 8 column chunks
-  const int m = threadIdx.x % kNb, q = threadIdx.x / kNb;
-  float s = 0.f;
-  if (m < jb) {
-    for (int k = q * (kNb / kQ); k < (q + 1) * (kNb / kQ); ++k)
-      if (k < jb) s = fmaf(__ldg(Dinv + (size_t)k * kNb + m), yin[k], s);
-  }
-  part[q * kNb + m] = s;
-  __syncthreads();
-  if (threadIdx.x < jb) {
-    float t = 0.f;
+// acc (8 x 8 of a 128 x 128 product per thread, 256 threads as 16 x 16) += A B over k < 128:
+// A(r, k) at a + k lda + r (rows < ar, columns < ac; zero beyond), B from b(k, c)
+template <class BLoad>
+__device__ __forceinline__ void merge_gemm(float (*acc)[8], const float* __restrict__ a, long long lda, int ar, int ac,
+                                           const BLoad& b, float (*As)[kNb + 4], float (*Bs)[kNb + 4]) {
+  const int tid = threadIdx.x, tr = tid & 15, tc = tid >> 4;
+  for (int k0 = 0; k0 < kNb; k0 += 16) {
+    float va[8], vb[8];
 #pragma unroll
-    for (int qq = 0; qq < kQ; ++qq) t += part[qq * kNb + threadIdx.x];
-    yd[threadIdx.x] = t;
+    for (int q = 0; q < 8; ++q) {
+      const int e = tid + 256 * q;
+      const int r = e % kNb, ka = k0 + e / kNb;
+      va[q] = r < ar && ka < ac ? a[(size_t)ka * lda + r] : 0.f;
+      vb[q] = b(k0 + e % 16, e / 16);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int e = tid + 256 * q;
+      As[e / kNb][e % kNb] = va[q];
+      Bs[e % 16][e / 16] = vb[q];
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (int kk = 0; kk < 16; ++kk) {
+      float x[8], y[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        x[q] = As[kk][tr + 16 * q];
+        y[q] = Bs[kk][tc + 16 * q];
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int q = 0; q < 8; ++q) acc[i][q] = fmaf(x[i], y[q], acc[i][q]);
+    }
   }
   __syncthreads();
 }
 
-// y[i] -= sum_m M(i, k0+m) yd[m] for the rows [i0, i1) of this block: the 128 columns are
-// split in 4 chunks of 32 so every thread of the block has loads in flight (one row per
-// thread leaves most threads idle and each row latency-bound); partials meet in `part`
-__device__ __forceinline__ void update_rows(const float* __restrict__ LU, long long ld, int k0, int jb, int i0, int i1,
-                                            const float* yd, float* y, float* part) {
-  const int nr = i1 - i0;
-  if (nr <= 0) return;
-  if (jb != kNb) {
-    for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) y[i] -= panel_dot(LU + (size_t)k0 * ld + i, ld, yd, jb);
-    return;
-  }
-  constexpr int kChunks = 4, kW = kNb / kChunks;
-  for (int r0 = 0; r0 < nr; r0 += kSolveThreads / kChunks) {
-    const int rows = min(kSolveThreads / kChunks, nr - r0);
-    const int q = threadIdx.x / (kSolveThreads / kChunks), r = threadIdx.x % (kSolveThreads / kChunks);
-    if (r < rows) {
-      const float* col = LU + (size_t)(k0 + q * kW) * ld + i0 + r0 + r;
-      float s[4] = {0.f, 0.f, 0.f, 0.f};
+// The kNb x kNb blocks at distance d from the diagonal of every kDb block's inverses (d = 1, 2,
+// ... in turn): X_ij = -X_ii sum_{j <= k < i} L_ik X_kj, and for the upper factor
+// Y_ij = -Y_ii sum_{i < k <= j} U_ik Y_kj.  One block each; blockIdx.y: lower, upper.
+struct MergeShared {
+  float As[16][kNb + 4], Bs[16][kNb + 4];
+  float T[kNb][kNb + 1];   // [column][row]
+};
+__global__ void __launch_bounds__(256) k_diag_merge(const float* __restrict__ LU, long long ld, int n, float* dinv,
+                                                    int d) {
+  extern __shared__ __align__(16) char mgsm[];
+  MergeShared& sh = *reinterpret_cast<MergeShared*>(mgsm);
+  const int per = kDbSub - d, b = blockIdx.x / per, t = blockIdx.x % per;
+  const bool lower = blockIdx.y == 0;
+  const int i = lower ? t + d : t, j = lower ? t : t + d;
+  const int o = b * kDb;                                   // first row and column of the kDb block
+  if (o + kNb * max(i, j) >= n) return;
+  float* X = dinv + (size_t)b * 2 * kDb * kDb + (lower ? 0 : (size_t)kDb * kDb);
+  const int tid = threadIdx.x, tr = tid & 15, tc = tid >> 4;
+  float acc[8][8];
 #pragma unroll
-      for (int m = 0; m < kW; ++m) s[m & 3] = fmaf(__ldg(col + (size_t)m * ld), yd[q * kW + m], s[m & 3]);
-      part[q * (kSolveThreads / kChunks) + r] = (s[0] + s[1]) + (s[2] + s[3]);
-    }
-    __syncthreads();
-    if (threadIdx.x < rows) {
-      const int rr = threadIdx.x;
-      float t = 0.f;
+  for (int e = 0; e < 8; ++e)
 #pragma unroll
-      for (int qq = 0; qq < kChunks; ++qq) t += part[qq * (kSolveThreads / kChunks) + rr];
-      y[i0 + r0 + rr] -= t;
-    }
-    __syncthreads();
+    for (int q = 0; q < 8; ++q) acc[e][q] = 0.f;
+  const int ar = min(kNb, n - (o + kNb * i));
+  for (int k = lower ? j : i + 1; k <= (lower ? i - 1 : j); ++k) {
+    const float* xb = X + (size_t)kNb * j * kDb + kNb * k;
+    merge_gemm(acc, LU + (size_t)(o + kNb * k) * ld + o + kNb * i, ld, ar, min(kNb, n - (o + kNb * k)),
+               [&](int kk, int c) { return xb[(size_t)c * kDb + kk]; }, sh.As, sh.Bs);
   }
+#pragma unroll
+  for (int e = 0; e < 8; ++e)
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      sh.T[tc + 16 * q][tr + 16 * e] = acc[e][q];
+      acc[e][q] = 0.f;
+    }
+  __syncthreads();
+  merge_gemm(acc, X + (size_t)kNb * i * (kDb + 1), kDb, kNb, kNb, [&](int kk, int c) { return sh.T[c][kk]; }, sh.As,
+             sh.Bs);
+  float* out = X + (size_t)kNb * j * kDb + kNb * i;
+#pragma unroll
+  for (int e = 0; e < 8; ++e)
+#pragma unroll
+    for (int q = 0; q < 8; ++q) out[(size_t)(tc + 16 * q) * kDb + tr + 16 * e] = -acc[e][q];
 }
 
 struct TrsvArgs {
@@ -1247,47 +1268,142 @@ struct TrsvArgs {
   const float* dinv;
   long long ld;
   int n;
-  float* y;     // right-hand side, overwritten by the partial updates
-  float* out;   // the solution: each segment, once final (never read by the kernel)
+  float* y;     // K right-hand sides (column c at c n), overwritten by the partial updates
+  float* out;   // the solutions: each segment, once final
   Barrier bar;
 };
 
-// forward substitution with the unit lower factor: per block column, every block applies
-// the block's inverse to the (final) y segment, then updates its share of the rows below;
-// block 0 stores the solved segment in `out`, which no block reads, so it cannot overtake
-// another block still reading that segment of y
-__global__ void __launch_bounds__(kSolveThreads) k_trsv_lower(TrsvArgs a) {
-  __shared__ float yd[kNb], yin[kNb];
-  __shared__ float part[kSolveThreads];
-  const int G = gridDim.x;
-  for (int k0 = 0; k0 < a.n; k0 += kNb) {
-    const int jb = min(kNb, a.n - k0);
-    diag_apply(a.dinv + (size_t)(k0 / kNb) * 2 * kNb * kNb, a.y + k0, jb, yin, part, yd);
-    const int rest = a.n - k0 - jb;
-    const int chunk = (rest + G - 1) / G;
-    const int i0 = k0 + jb + blockIdx.x * chunk, i1 = min(a.n, i0 + chunk);
-    update_rows(a.LU, a.ld, k0, jb, i0, i1, yd, a.y, part);
-    if (blockIdx.x == 0 && threadIdx.x < jb) a.out[k0 + threadIdx.x] = yd[threadIdx.x];
+// L w = y (LOWER) or U x = w for K right-hand sides, kDb columns at a time.  What bounds it is
+// latency: per step the segment is multiplied by its block's inverse (a few rows per CUDA block),
+// a grid barrier, the other rows take the segment's columns of the factor (each block its share
+// of rows), a grid barrier.  The factor's elements are loaded before the barriers they do not
+// depend on.  kDb 512: 128 columns a step, every block applying the whole 128 x 128 inverse for
+// itself, took 8-10 us a step; 1024 would double the memory of the inverses (n kDb 8 bytes) to
+// save a few barriers.  A whole solve with 3 refinements, before and after: n = 640 0.44 -> 0.36
+// ms, 2,560 0.99 -> 0.56, 10,240 5.41 -> 1.59, 15,360 8.12 -> 2.56; the inverses cost 0.1 ms per factorisation.
+constexpr int kTrRows = 64, kTrChunks = kSolveThreads / kTrRows, kTrCols = kDb / kTrChunks;
+constexpr size_t trsv_smem(int K) { return (size_t)K * (kDb + kSolveThreads) * sizeof(float); }
+template <int K, bool LOWER>
+__global__ void __launch_bounds__(kSolveThreads) k_trsv(TrsvArgs a) {
+  extern __shared__ float trsm[];
+  float* yd = trsm;               // [K][kDb]
+  float* part = trsm + K * kDb;   // [K][kTrChunks][kTrRows]
+  const int G = gridDim.x, tid = threadIdx.x, n = a.n;
+  const int nblk = (n + kDb - 1) / kDb;
+  for (int s = 0; s < nblk; ++s) {
+    const int b = LOWER ? s : nblk - 1 - s;
+    const int k0 = b * kDb, jb = min(kDb, n - k0);
+    const float* D = a.dinv + (size_t)b * 2 * kDb * kDb + (LOWER ? 0 : (size_t)kDb * kDb);
+    // this block's rows of the update, and their elements for the first kTrRows of them
+    const int lo = LOWER ? k0 + jb : 0, hi = LOWER ? n : k0;
+    const int share = (hi - lo + G - 1) / G;
+    const int i0 = lo + blockIdx.x * share, i1 = min(hi, i0 + share);
+    const int r = tid % kTrRows, q = tid / kTrRows;
+    float m[kTrCols];
+    auto load = [&](int i) {
+#pragma unroll
+      for (int t = 0; t < kTrCols; ++t) {
+        const int col = q * kTrCols + t;
+        m[t] = i < i1 && col < jb ? __ldg(a.LU + (size_t)(k0 + col) * a.ld + i) : 0.f;
+      }
+    };
+    load(i0 + r);
+    // rows of the block's inverse times the segment: 4 rows at a time, a thread per row and pair
+    // of columns
+    const int rpb = (jb + G - 1) / G;
+    const int d1 = min(jb, (int)(blockIdx.x + 1) * rpb);
+    for (int d0 = blockIdx.x * rpb; d0 < d1; d0 += 4) {
+      const int row = d0 + (tid & 3);
+      float v[K];
+#pragma unroll
+      for (int c = 0; c < K; ++c) v[c] = 0.f;
+#pragma unroll
+      for (int h = 0; h < kDb / (kSolveThreads / 4); ++h) {
+        const int col = (tid >> 2) + h * (kSolveThreads / 4);
+        const bool in = row < d1 && col < jb && (LOWER ? col <= row : col >= row);
+        const float dv = in ? __ldg(D + (size_t)col * kDb + row) : 0.f;
+        if (in)
+#pragma unroll
+          for (int c = 0; c < K; ++c) v[c] = fmaf(dv, __ldcg(a.y + (size_t)c * n + k0 + col), v[c]);
+      }
+#pragma unroll
+      for (int c = 0; c < K; ++c) {
+#pragma unroll
+        for (int o = 4; o < 32; o <<= 1) v[c] += __shfl_xor_sync(0xffffffffu, v[c], o);
+        if ((tid & 31) < 4) part[(c * 32 + (tid >> 5)) * 4 + (tid & 3)] = v[c];
+      }
+      __syncthreads();
+      if (tid < 4 * K) {
+        const int c = tid >> 2, rr = d0 + (tid & 3);
+        float t = 0.f;
+#pragma unroll 8
+        for (int w = 0; w < 32; ++w) t += part[(c * 32 + w) * 4 + (tid & 3)];
+        if (rr < d1) __stcg(a.out + (size_t)c * n + k0 + rr, t);
+      }
+      __syncthreads();
+    }
+    if (hi <= lo) break;   // the last segment (the same in every block)
+    if (!grid_sync(a.bar)) return;
+    for (int e = tid; e < K * jb; e += kSolveThreads) {
+      const int c = e / jb, k = e - c * jb;
+      yd[c * kDb + k] = __ldcg(a.out + (size_t)c * n + k0 + k);
+    }
+    for (int r0 = i0; r0 < i1; r0 += kTrRows) {
+      if (r0 > i0) load(r0 + r);
+      __syncthreads();
+      float v[K];
+#pragma unroll
+      for (int c = 0; c < K; ++c) v[c] = 0.f;
+#pragma unroll
+      for (int t = 0; t < kTrCols; ++t)
+#pragma unroll
+        for (int c = 0; c < K; ++c) v[c] = fmaf(m[t], q * kTrCols + t < jb ? yd[c * kDb + q * kTrCols + t] : 0.f, v[c]);
+#pragma unroll
+      for (int c = 0; c < K; ++c) part[(c * kTrChunks + q) * kTrRows + r] = v[c];
+      __syncthreads();
+      for (int e = tid; e < K * kTrRows; e += kSolveThreads) {
+        const int c = e / kTrRows, rr = e % kTrRows;
+        if (r0 + rr < i1) {
+          float t = 0.f;
+#pragma unroll
+          for (int w = 0; w < kTrChunks; ++w) t += part[(c * kTrChunks + w) * kTrRows + rr];
+          float* yp = a.y + (size_t)c * n + r0 + rr;
+          __stcg(yp, __ldcg(yp) - t);
+        }
+      }
+    }
     if (!grid_sync(a.bar)) return;
   }
 }
 
-// back substitution with the upper factor
-__global__ void __launch_bounds__(kSolveThreads) k_trsv_upper(TrsvArgs a) {
-  __shared__ float yd[kNb], yin[kNb];
-  __shared__ float part[kSolveThreads];
-  const int G = gridDim.x;
-  const int nblk = (a.n + kNb - 1) / kNb;
-  for (int kb = nblk - 1; kb >= 0; --kb) {
-    const int k0 = kb * kNb, jb = min(kNb, a.n - k0);
-    diag_apply(a.dinv + (size_t)kb * 2 * kNb * kNb + (size_t)kNb * kNb, a.y + k0, jb, yin, part, yd);
-    const int chunk = (k0 + G - 1) / G;
-    const int i0 = blockIdx.x * chunk, i1 = min(k0, i0 + chunk);
-    update_rows(a.LU, a.ld, k0, jb, i0, i1, yd, a.y, part);
-    if (blockIdx.x == 0 && threadIdx.x < jb) a.out[k0 + threadIdx.x] = yd[threadIdx.x];
-    if (!grid_sync(a.bar)) return;
+// both solves for K right-hand sides: lower.y -> lower.out = upper.y -> upper.out
+template <int K>
+static int32_t launch_trsv(const TrsvArgs& lower, const TrsvArgs& upper, int G, cudaStream_t st) {
+  const void* ks[2] = {(const void*)&k_trsv<K, true>, (const void*)&k_trsv<K, false>};
+  TrsvArgs args[2] = {lower, upper};
+  for (int e = 0; e < 2; ++e) {
+    void* av[] = {&args[e]};
+    O3G_CUDA_TRY(cudaFuncSetAttribute(ks[e], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trsv_smem(K)));
+    O3G_CUDA_TRY(zero_barrier(lower.bar.err, st));
+    O3G_CUDA_TRY(cudaLaunchCooperativeKernel(ks[e], dim3(G), dim3(kSolveThreads), av, trsv_smem(K), st));
+  }
+  note_launch(2);
+  return O3G_OK;
+}
+static int32_t trsv(int K, const TrsvArgs& lower, const TrsvArgs& upper, int G, cudaStream_t st) {
+  switch (K) {
+    case 1: return launch_trsv<1>(lower, upper, G, st);
+    case 2: return launch_trsv<2>(lower, upper, G, st);
+    case 3: return launch_trsv<3>(lower, upper, G, st);
+    case 4: return launch_trsv<4>(lower, upper, G, st);
+    case 5: return launch_trsv<5>(lower, upper, G, st);
+    case 6: return launch_trsv<6>(lower, upper, G, st);
+    case 7: return launch_trsv<7>(lower, upper, G, st);
+    default: return launch_trsv<8>(lower, upper, G, st);
   }
 }
+// one block per SM (1024 threads and at most 48 KB each: always resident together)
+static int trsv_grid(int num_sms) { return num_sms; }
 
 __global__ void k_axpy_f2d(double* x, const float* d, int n) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1491,7 +1607,7 @@ extern "C" int32_t o3g_bem_create(int64_t n, o3g_bem_t** out) {
   if (e == cudaSuccess) e = o3g::dev_alloc((void**)&h->piv, n * sizeof(int));
   if (e == cudaSuccess) e = o3g::dev_alloc((void**)&h->perm, n * sizeof(int));
   if (e == cudaSuccess) e = o3g::dev_alloc((void**)&h->flags, 64 * sizeof(int));
-  if (e == cudaSuccess) e = o3g::dev_alloc((void**)&h->dinv, (size_t)((n + kNb - 1) / kNb) * 2 * kNb * kNb * sizeof(float));
+  if (e == cudaSuccess) e = o3g::dev_alloc((void**)&h->dinv, dinv_floats((int)n) * sizeof(float));
   if (e != cudaSuccess) {
     (void)cudaGetLastError();
     set_error_cuda("o3g_bem_create: cudaMalloc", e);
@@ -1730,7 +1846,11 @@ extern "C" int32_t o3g_bem_factor(o3g_bem_t* h, void* stream) {
     const size_t dsm = (size_t)kNb * kNb * sizeof(float);
     O3G_CUDA_TRY(cudaFuncSetAttribute(k_diag_inverses, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsm));
     k_diag_inverses<<<(n + kNb - 1) / kNb, 256, dsm, st>>>(h->LU, ld, n, h->dinv);
-    note_launch();
+    O3G_CUDA_TRY(cudaFuncSetAttribute(k_diag_merge, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MergeShared)));
+    const int nbig = (n + kDb - 1) / kDb;
+    for (int d = 1; d < kDbSub && n > d * kNb; ++d)
+      k_diag_merge<<<dim3(nbig * (kDbSub - d), 2), 256, sizeof(MergeShared), st>>>(h->LU, ld, n, h->dinv, d);
+    note_launch(kDbSub);
   }
   tm.end(st);
   O3G_CUDA_TRY(cudaGetLastError());
@@ -1808,20 +1928,13 @@ extern "C" int32_t o3g_bem_solve(o3g_bem_t* h, const float* b, float* x, double*
   O3G_CUDA_TRY(cudaMemsetAsync(xd, 0, (size_t)n * 8, st));
   O3G_CUDA_TRY(cudaMemcpyAsync(rd, bd, (size_t)n * 8, cudaMemcpyDeviceToDevice, st));
   O3G_CUDA_TRY(cudaMemsetAsync(h->flags, 0, 4 * sizeof(int), st));
-  // cooperative solve kernels: one block per SM
-  int G = df.num_sms;
-  int per_sm = 0;
-  const size_t dsm = 0;
-  O3G_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trsv_lower, kSolveThreads, dsm));
-  if (per_sm < 1) return O3G_ERR_CUDA;
+  const int G = trsv_grid(df.num_sms);
   // L w = P r (y -> w; xh is free between the products), then U y = w (w -> y)
   TrsvArgs ta, tb;
   ta.LU = h->LU; ta.dinv = h->dinv; ta.ld = ld; ta.n = n; ta.y = y; ta.out = xh;
   ta.bar = make_barrier(h->flags);
   tb = ta;
   tb.y = xh; tb.out = y;
-  void* targs[] = {&ta};
-  void* tbargs[] = {&tb};
   std::vector<double> hn((size_t)nrb);
   double rel = 1.0, bnorm = 0.0;
   int it = 0;
@@ -1844,12 +1957,9 @@ extern "C" int32_t o3g_bem_solve(o3g_bem_t* h, const float* b, float* x, double*
     rel = bnorm > 0.0 ? std::sqrt(rr) / bnorm : std::sqrt(rr);
     if (rel <= tol || it == max_iter) break;
     k_permute_to_float<<<nrb, 256, 0, st>>>(rd, h->perm, y, n);
-    O3G_CUDA_TRY(zero_barrier(h->flags, st));
-    O3G_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)k_trsv_lower, dim3(G), dim3(kSolveThreads), targs, dsm, st));
-    O3G_CUDA_TRY(zero_barrier(h->flags, st));
-    O3G_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)k_trsv_upper, dim3(G), dim3(kSolveThreads), tbargs, dsm, st));
+    O3G_TRY(trsv(1, ta, tb, G, st));
     k_axpy_f2d<<<nrb, 256, 0, st>>>(xd, y, n);
-    note_launch(4);
+    note_launch(2);
   }
   tm.end(st);
   int fl = 0;
@@ -2336,124 +2446,6 @@ __global__ void k_permute_to_float_multi(const double* r, const int* perm, float
   if (i < n) y[(size_t)c * n + i] = ((mask >> c) & 1u) ? (float)r[(size_t)c * n + perm[i]] : 0.f;
 }
 
-template <int K>
-__device__ __forceinline__ void diag_apply_multi(const float* __restrict__ Dinv, const float* y, int n, int jb,
-                                                 float (*yin)[kNb], float* part, float (*yd)[kNb]) {
-  for (int e = threadIdx.x; e < K * jb; e += blockDim.x) yin[e / jb][e % jb] = y[(size_t)(e / jb) * n + e % jb];
-  __syncthreads();
-  constexpr int kQ = kSolveThreads / kNb;
-  const int m = threadIdx.x % kNb, q = threadIdx.x / kNb;
-  float s[K];
-#pragma unroll
-  for (int c = 0; c < K; ++c) s[c] = 0.f;
-  if (m < jb) {
-    for (int k = q * (kNb / kQ); k < (q + 1) * (kNb / kQ); ++k)
-      if (k < jb) {
-        const float d = __ldg(Dinv + (size_t)k * kNb + m);
-#pragma unroll
-        for (int c = 0; c < K; ++c) s[c] = fmaf(d, yin[c][k], s[c]);
-      }
-  }
-#pragma unroll
-  for (int c = 0; c < K; ++c) part[(c * kQ + q) * kNb + m] = s[c];
-  __syncthreads();
-  for (int e = threadIdx.x; e < K * jb; e += blockDim.x) {
-    const int c = e / jb, tt = e % jb;
-    float v = 0.f;
-#pragma unroll
-    for (int qq = 0; qq < kQ; ++qq) v += part[(c * kQ + qq) * kNb + tt];
-    yd[c][tt] = v;
-  }
-  __syncthreads();
-}
-
-template <int K>
-__device__ __forceinline__ void update_rows_multi(const float* __restrict__ LU, long long ld, int n, int k0, int jb,
-                                                  int i0, int i1, float (*yd)[kNb], float* y, float* part) {
-  const int nr = i1 - i0;
-  if (nr <= 0) return;
-  if (jb != kNb) {
-    for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
-      float s[K];
-#pragma unroll
-      for (int c = 0; c < K; ++c) s[c] = 0.f;
-      for (int m = 0; m < jb; ++m) {
-        const float a = LU[(size_t)(k0 + m) * ld + i];
-#pragma unroll
-        for (int c = 0; c < K; ++c) s[c] = fmaf(a, yd[c][m], s[c]);
-      }
-#pragma unroll
-      for (int c = 0; c < K; ++c) y[(size_t)c * n + i] -= s[c];
-    }
-    return;
-  }
-  constexpr int kChunks = 4, kW = kNb / kChunks, kRows = kSolveThreads / kChunks;
-  for (int r0 = 0; r0 < nr; r0 += kRows) {
-    const int rows = min(kRows, nr - r0);
-    const int q = threadIdx.x / kRows, r = threadIdx.x % kRows;
-    if (r < rows) {
-      const float* col = LU + (size_t)(k0 + q * kW) * ld + i0 + r0 + r;
-      float s[K];
-#pragma unroll
-      for (int c = 0; c < K; ++c) s[c] = 0.f;
-#pragma unroll 8
-      for (int m = 0; m < kW; ++m) {
-        const float a = __ldg(col + (size_t)m * ld);
-#pragma unroll
-        for (int c = 0; c < K; ++c) s[c] = fmaf(a, yd[c][q * kW + m], s[c]);
-      }
-#pragma unroll
-      for (int c = 0; c < K; ++c) part[(c * kChunks + q) * kRows + r] = s[c];
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < K * rows; e += blockDim.x) {
-      const int c = e / rows, rr = e % rows;
-      float v = 0.f;
-#pragma unroll
-      for (int qq = 0; qq < kChunks; ++qq) v += part[(c * kChunks + qq) * kRows + rr];
-      y[(size_t)c * n + i0 + r0 + rr] -= v;
-    }
-    __syncthreads();
-  }
-}
-
-// L w = y and U x = w for K right-hand sides (y, out: K vectors of n, column c at c n)
-template <int K>
-__global__ void __launch_bounds__(kSolveThreads) k_trsv_lower_multi(TrsvArgs a) {
-  __shared__ float yd[K][kNb], yin[K][kNb];
-  __shared__ float part[K * kSolveThreads];
-  const int G = gridDim.x;
-  for (int k0 = 0; k0 < a.n; k0 += kNb) {
-    const int jb = min(kNb, a.n - k0);
-    diag_apply_multi<K>(a.dinv + (size_t)(k0 / kNb) * 2 * kNb * kNb, a.y + k0, a.n, jb, yin, part, yd);
-    const int rest = a.n - k0 - jb;
-    const int chunk = (rest + G - 1) / G;
-    const int i0 = k0 + jb + blockIdx.x * chunk, i1 = min(a.n, i0 + chunk);
-    update_rows_multi<K>(a.LU, a.ld, a.n, k0, jb, i0, i1, yd, a.y, part);
-    if (blockIdx.x == 0)
-      for (int e = threadIdx.x; e < K * jb; e += blockDim.x) a.out[(size_t)(e / jb) * a.n + k0 + e % jb] = yd[e / jb][e % jb];
-    if (!grid_sync(a.bar)) return;
-  }
-}
-
-template <int K>
-__global__ void __launch_bounds__(kSolveThreads) k_trsv_upper_multi(TrsvArgs a) {
-  __shared__ float yd[K][kNb], yin[K][kNb];
-  __shared__ float part[K * kSolveThreads];
-  const int G = gridDim.x;
-  const int nblk = (a.n + kNb - 1) / kNb;
-  for (int kb = nblk - 1; kb >= 0; --kb) {
-    const int k0 = kb * kNb, jb = min(kNb, a.n - k0);
-    diag_apply_multi<K>(a.dinv + (size_t)kb * 2 * kNb * kNb + (size_t)kNb * kNb, a.y + k0, a.n, jb, yin, part, yd);
-    const int chunk = (k0 + G - 1) / G;
-    const int i0 = blockIdx.x * chunk, i1 = min(k0, i0 + chunk);
-    update_rows_multi<K>(a.LU, a.ld, a.n, k0, jb, i0, i1, yd, a.y, part);
-    if (blockIdx.x == 0)
-      for (int e = threadIdx.x; e < K * jb; e += blockDim.x) a.out[(size_t)(e / jb) * a.n + k0 + e % jb] = yd[e / jb][e % jb];
-    if (!grid_sync(a.bar)) return;
-  }
-}
-
 // the products b_c - A x_c (b given) or A x_c for K vectors in one pass over A, with the
 // squared norms of the results on the host (synchronises) when norm2 is given
 static int32_t matvec_multi(o3g_bem_t* h, int K, const DIn& x, const DIn& b, const DOut& y, float* xh, float* xl,
@@ -2495,58 +2487,6 @@ static int32_t matvec_multi(o3g_bem_t* h, int K, const DIn& x, const DIn& b, con
     for (int c = 0; c < K; ++c)
       for (int k = 0; k < nrb; ++k) (*norm2)[c] += hn[(size_t)c * nrb + k];
   }
-  return O3G_OK;
-}
-
-template <int K>
-static int32_t launch_trsv_multi(const TrsvArgs& lower, const TrsvArgs& upper, int G, cudaStream_t st) {
-  TrsvArgs a = lower, b = upper;
-  void* aa[] = {&a};
-  void* bb[] = {&b};
-  int* flags = reinterpret_cast<int*>(a.bar.err);
-  O3G_CUDA_TRY(zero_barrier(flags, st));
-  O3G_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)k_trsv_lower_multi<K>, dim3(G), dim3(kSolveThreads), aa, 0,
-                                           st));
-  O3G_CUDA_TRY(zero_barrier(flags, st));
-  O3G_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)k_trsv_upper_multi<K>, dim3(G), dim3(kSolveThreads), bb, 0,
-                                           st));
-  note_launch(2);
-  return O3G_OK;
-}
-
-static int32_t trsv_multi(int K, const TrsvArgs& lower, const TrsvArgs& upper, int G, cudaStream_t st) {
-  switch (K) {
-    case 1: return launch_trsv_multi<1>(lower, upper, G, st);
-    case 2: return launch_trsv_multi<2>(lower, upper, G, st);
-    case 3: return launch_trsv_multi<3>(lower, upper, G, st);
-    case 4: return launch_trsv_multi<4>(lower, upper, G, st);
-    case 5: return launch_trsv_multi<5>(lower, upper, G, st);
-    case 6: return launch_trsv_multi<6>(lower, upper, G, st);
-    case 7: return launch_trsv_multi<7>(lower, upper, G, st);
-    default: return launch_trsv_multi<8>(lower, upper, G, st);
-  }
-}
-
-// blocks per SM of the K-vector solve kernels (their shared memory grows with K)
-static int32_t trsv_multi_grid(int K, int num_sms, int* G) {
-  int per_sm = 0;
-  cudaError_t e;
-  switch (K) {
-    case 1: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trsv_lower_multi<1>, kSolveThreads, 0); break;
-    case 2: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trsv_lower_multi<2>, kSolveThreads, 0); break;
-    case 3: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trsv_lower_multi<3>, kSolveThreads, 0); break;
-    case 4: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trsv_lower_multi<4>, kSolveThreads, 0); break;
-    case 5: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trsv_lower_multi<5>, kSolveThreads, 0); break;
-    case 6: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trsv_lower_multi<6>, kSolveThreads, 0); break;
-    case 7: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trsv_lower_multi<7>, kSolveThreads, 0); break;
-    default: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trsv_lower_multi<8>, kSolveThreads, 0); break;
-  }
-  O3G_CUDA_TRY(e);
-  if (per_sm < 1) {
-    set_error("o3g_bem_solve_many: the solve kernel does not fit on an SM");
-    return O3G_ERR_CUDA;
-  }
-  *G = num_sms;   // one block per SM, as the single-vector solve
   return O3G_OK;
 }
 
@@ -2618,8 +2558,7 @@ extern "C" int32_t o3g_bem_solve_many(o3g_bem_t* h, int32_t nrhs, const float* B
       rout.p[c] = rd + (size_t)c * n;
     }
     DIn none{};
-    int G = 0;
-    O3G_TRY(trsv_multi_grid(K, df.num_sms, &G));
+    const int G = trsv_grid(df.num_sms);
     TrsvArgs lo, up;
     lo.LU = h->LU; lo.dinv = h->dinv; lo.ld = ld; lo.n = n; lo.y = y; lo.out = w;
     lo.bar = make_barrier(h->flags);
@@ -2642,7 +2581,7 @@ extern "C" int32_t o3g_bem_solve_many(o3g_bem_t* h, int32_t nrhs, const float* B
       if (!active) break;
       k_permute_to_float_multi<<<dim3(nrb, K), 256, 0, st>>>(rd, h->perm, y, n, active);
       note_launch();
-      O3G_TRY(trsv_multi(K, lo, up, G, st));
+      O3G_TRY(trsv(K, lo, up, G, st));
       k_axpy_f2d<<<(unsigned)((knn + 255) / 256), 256, 0, st>>>(xd, y, (int)knn);
       note_launch();
     }
