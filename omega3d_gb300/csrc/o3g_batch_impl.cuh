@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(kBlock, PairMinBlocks<C, MODE, GRADS, TPT>::va
   constexpr int NP = ACC ? 2 * NC : NC;
   constexpr int TB = kBlock * TPT;
   static_assert(std::is_same<T, float>::value, "the batched sums are FP32 (packed pair arithmetic)");
-  __shared__ float4 QB[2][5][kBlock / 2];   // staged tiles as source pairs, double-buffered
+  __shared__ float4 QB[2][4][kBlock / 2];   // staged tiles as source pairs, double-buffered
   __shared__ int s_item, s_last;
   // the Gaussian core's polynomial table, read from shared memory by the near-field pairs
   __shared__ __align__(16) float gsh[C == CORE_GAUSS ? kGaussTab : 1];

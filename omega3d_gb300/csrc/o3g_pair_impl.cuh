@@ -238,7 +238,8 @@ __device__ __forceinline__ void sweep_tile(const V4<T>* sp, const V4<T>* sw, con
 // ---- packed FP32: two sources per instruction (FFMA2 / FADD2 / FMUL2 on float2) -----------
 // What bounds these kernels is the FMA pipe: RM plain with gradients takes 34 packed
 // operations and two MUFU per pair of sources, 34 cycles per pair and warp scheduler at two
-// cycles each, and runs at 41 (65,536 particles, one GB300; was 47 with 37 operations).
+// cycles each, and runs at 41 (65,536 particles, one GB300; was 47 with 37 operations), RM
+// compensated at 50 (60).
 // The rest is the register file: a micro-benchmark of FFMA2 alone takes 2.1 cycles when one
 // operand is the previous instruction's, 2.95 with three new ones (FMUL2, FADD2 2.1; a
 // scalar FFMA 1.08), so the accumulations below are written in runs that share an operand.
@@ -249,28 +250,28 @@ __device__ __forceinline__ void sweep_tile(const V4<T>* sp, const V4<T>* sw, con
 // shared memory as pairs of sources (2p, 2p+1), component-major so every load yields
 // float2 operands directly:
 //   Q[0][p] = (-x0, -x1, -y0, -y1)    Q[1][p] = (-z0, -z1, c0, c1)     (c: core parameter)
-//   Q[2][p] = (wx0, wx1, wy0, wy1)    Q[3][p] = (wz0, wz1, -wx0, -wx1)
-//   Q[4][p] = (-wy0, -wy1, -wz0, -wz1)
-// (negated copies turn the separations and the cross products' differences into adds
-// and fused multiply-adds).
+//   Q[2][p] = (wx0, wx1, wy0, wy1)    Q[3][p] = (wz0, wz1)             (8 of its 16 bytes)
+// (negated positions turn the separations into adds; the cross products' differences negate
+// a register operand, which costs nothing).  Rows are worth saving: a broadcast read still returns
+// 16 bytes to each of 32 lanes, four cycles of the SM's 128 bytes a cycle, so five rows with one
+// target per thread took 80 of the 104 cycles that four schedulers' pairs take.
 __device__ __forceinline__ void stage_pair(const V4<float>& s, const V4<float>& w, float4 (*Q)[kBlock / 2], int j) {
   const int p = j >> 1, h = j & 1;
   float* q0 = reinterpret_cast<float*>(&Q[0][p]);
   float* q1 = reinterpret_cast<float*>(&Q[1][p]);
   float* q2 = reinterpret_cast<float*>(&Q[2][p]);
   float* q3 = reinterpret_cast<float*>(&Q[3][p]);
-  float* q4 = reinterpret_cast<float*>(&Q[4][p]);
   q0[h] = -s.x; q0[2 + h] = -s.y;
   q1[h] = -s.z; q1[2 + h] = s.w;
   q2[h] = w.x;  q2[2 + h] = w.y;
-  q3[h] = w.z;  q3[2 + h] = -w.x;
-  q4[h] = -w.y; q4[2 + h] = -w.z;
+  q3[h] = w.z;
 }
 
 __device__ __forceinline__ float2 f2lo(const float4& q) { return make_float2(q.x, q.y); }
 __device__ __forceinline__ float2 f2hi(const float4& q) { return make_float2(q.z, q.w); }
 
 __device__ __forceinline__ float2 f2(float v) { return make_float2(v, v); }
+__device__ __forceinline__ float2 neg2(const float2& v) { return make_float2(-v.x, -v.y); }
 
 // x^(-1/2) (rs), x^(-1) (s2) and x^(-3/2) (r3) of two lanes.  ACC: one Newton step whose
 // residual e = 1 - x s2 is formed from the rounded square s2 = rs^2 by one fma, so the
@@ -383,23 +384,27 @@ __device__ __forceinline__ void core2(const float2& dx, const float2& dy, const 
   }
 }
 
-// one target (tt = (x,x), (y,y), (z,z), (c,c)) against the source pair of q0..q4; a[] as in
+// one target (tt = (x,x), (y,y), (z,z), (c,c)) against the source pair of q0..q2, wz; a[] as in
 // pair_g / pair_v, one float2 lane per source.  NO_ZZ: a[11] is left out (fold_grads).
 template <int C, bool ACC, bool HAVE_TR, bool GRADS, bool NO_ZZ>
 __device__ __forceinline__ void pair2(const float2* tt, const float4& q0, const float4& q1, const float4& q2,
-                                      const float4& q3, const float4& q4, float2* a, const float* gtab) {
+                                      const float2& wz, float2* a, const float* gtab) {
   const float2 dx = __fadd2_rn(tt[0], f2lo(q0));
   const float2 dy = __fadd2_rn(tt[1], f2hi(q0));
   const float2 dz = __fadd2_rn(tt[2], f2lo(q1));
   const float2 cst = HAVE_TR && C != CORE_SING ? __fadd2_rn(f2hi(q1), tt[3]) : f2hi(q1);
   float2 r3, b3;
   core2<C, ACC, GRADS>(dx, dy, dz, cst, gtab, r3, b3);
-  const float2 wx = f2lo(q2), wy = f2hi(q2), wz = f2lo(q3);
-  const float2 nwx = f2hi(q3), nwy = f2lo(q4), nwz = f2hi(q4);
-  float2 cx = __fmul2_rn(dy, nwz), cy = __fmul2_rn(dx, wz), cz = __fmul2_rn(dx, nwy);
-  cx = __ffma2_rn(dz, wy, cx);    // dz wy - dy wz
-  cy = __ffma2_rn(dz, nwx, cy);   // dx wz - dz wx
-  cz = __ffma2_rn(dy, wx, cz);    // dy wx - dx wy
+  const float2 wx = f2lo(q2), wy = f2hi(q2);
+  // which operands carry the signs decides the register assignment: at 65,536 particles (RM) the
+  // compensated kernel takes 49.7 cycles per pair with the strengths negated and 53.3 with the
+  // separations, the plain one 42.4 and 41.2 (51.5 and 41.3 with five staged rows)
+  const float2 ndx = ACC ? dx : neg2(dx), ndy = ACC ? dy : neg2(dy), ndz = ACC ? dz : neg2(dz);
+  const float2 nwx = ACC ? neg2(wx) : wx, nwy = ACC ? neg2(wy) : wy, nwz = ACC ? neg2(wz) : wz;
+  float2 cx = __fmul2_rn(ndy, nwz), cy = __fmul2_rn(dx, wz), cz = __fmul2_rn(ndx, nwy);
+  cx = __ffma2_rn(dz, wy, cx);     // dz wy - dy wz
+  cy = __ffma2_rn(ndz, nwx, cy);   // dx wz - dz wx
+  cz = __ffma2_rn(dy, wx, cz);     // dy wx - dx wy
   a[0] = __ffma2_rn(r3, cx, a[0]);
   a[1] = __ffma2_rn(r3, cy, a[1]);
   a[2] = __ffma2_rn(r3, cz, a[2]);
@@ -438,10 +443,11 @@ __device__ __forceinline__ void sweep_pairs(const float4 (*Q)[kBlock / 2], int p
 #pragma unroll UN
     for (int j = j0; j < j0 + FOLD; ++j) {
       const int p = p0 + j;
-      const float4 q0 = Q[0][p], q1 = Q[1][p], q2 = Q[2][p], q3 = Q[3][p], q4 = Q[4][p];
+      const float4 q0 = Q[0][p], q1 = Q[1][p], q2 = Q[2][p];
+      const float2 wz = *reinterpret_cast<const float2*>(&Q[3][p]);
 #pragma unroll
       for (int k = 0; k < TPT; ++k)
-        pair2<C, ACC, HAVE_TR, GRADS, ACC>(tt[k], q0, q1, q2, q3, q4, acc[k], gtab);
+        pair2<C, ACC, HAVE_TR, GRADS, ACC>(tt[k], q0, q1, q2, wz, acc[k], gtab);
     }
     if (ACC) {
 #pragma unroll
@@ -618,10 +624,11 @@ __global__ void __launch_bounds__(kBlock) k_pair(const PairArgs<T, O> a) {
 }
 
 // Blocks per SM asked of the compiler (0: its own choice).  The compensated Gaussian kernel
-// with gradients would take 124 registers (4 blocks); held to 5 blocks it spills 40 bytes outside the
-// pair loops and the 262,144-particle cloud goes from 102.8 to 98.0 ms (115.8 ms before
-// gauss2's table, rsq2 and the factored gradient).  RM compensated takes 90 (5 blocks) by
-// itself; 6 blocks (80 registers) were slower (5.58 against 5.49 ms at 65,536 particles).
+// with gradients would take 124 registers (4 blocks); held to 5 blocks it spills 8 bytes outside the
+// pair loops and a 262,144-particle cloud takes 97.4 ms (4 blocks, with five staged rows: 102.8
+// against 98.0; 111 before gauss2's table, rsq2, the factored gradient and the four rows).  Two
+// targets per thread read half the rows but leave 3 blocks: RM 50.8 cycles per pair against
+// 49.7, Gaussian 62.7 against 62.5.
 // The plain kernels with two targets per thread are held to the 128 registers of 4 blocks
 // (the batched ones would take 130 to 159).
 template <int C, int MODE, bool GRADS, int TPT> struct PairMinBlocks {
@@ -642,7 +649,7 @@ __global__ void __launch_bounds__(kBlock, PairMinBlocks<C, MODE, GRADS, TPT>::va
   constexpr int NA = GRADS ? 15 : 3;
   constexpr int NC = GRADS ? 12 : 3;
   constexpr int NH = ACC ? NC : 1;
-  __shared__ float4 QB[2][5][kBlock / 2];
+  __shared__ float4 QB[2][4][kBlock / 2];
   // the Gaussian core's polynomial table, read from shared memory by the near-field pairs
   __shared__ __align__(16) float gsh[C == CORE_GAUSS ? kGaussTab : 1];
   const float* gtab = nullptr;
