@@ -24,7 +24,7 @@
 //     lanes have a close panel at the same time, and their trees have 4 to 64 leaves.
 // The owner adds its nodes' sums in queue order: results do not depend on scheduling.
 // Measured (one GB300), 5,120 panels on 262,144 points with gradients, compensated: 4.32 ->
-// 2.43 ms; 100,000 particles on 20,480 panels: 3.05 -> 1.41 ms.
+// 2.23 ms; 100,000 particles on 20,480 panels: 3.05 -> 1.34 ms (2.43 and 1.41 with six rows a tile).
 //
 #include "o3g_pair_impl.cuh"
 
@@ -41,11 +41,11 @@ constexpr int kFoldTiles = 4;     // tiles between two folds of the compensated 
 __host__ __device__ constexpr int queue_cap(int tpt, int maxlev) {
   return 31 + 64 * tpt + 96 * (maxlev > 1 ? maxlev - 1 : 0) + 128;
 }
-constexpr int kRows = 6;          // float4 rows of a staged tile
+constexpr int kRows = 4;          // float4 rows of a staged tile
 
 // A tile of kPW panels or particles, as pairs, component-major (kRows rows of kPW / 2 float4):
 //   0: (-x0, -x1, -y0, -y1)   1: (-z0, -z1, t0, t1)   2: (sx0, sx1, sy0, sy1)
-//   3: (sz0, sz1, -sx0, -sx1) 4: (-sy0, -sy1, -sz0, -sz1)   5: (q0, q1, -, -)
+//   3: (sz0, sz1, q0, q1)
 // position (a panel's centroid), squared far threshold, strength, source strength.
 __device__ __forceinline__ void store_row(float4* tiles, int j, float x, float y, float z, float t, float sx, float sy,
                                           float sz, float q) {
@@ -54,9 +54,7 @@ __device__ __forceinline__ void store_row(float4* tiles, int j, float x, float y
   b[0] = -x;          b[2] = -y;
   b[R] = -z;          b[R + 2] = t;
   b[2 * R] = sx;      b[2 * R + 2] = sy;
-  b[3 * R] = sz;      b[3 * R + 2] = -sx;
-  b[4 * R] = -sy;     b[4 * R + 2] = -sz;
-  b[5 * R] = q;       b[5 * R + 2] = 0.f;
+  b[3 * R] = sz;      b[3 * R + 2] = q;
 }
 
 struct PanelNear {
@@ -110,12 +108,12 @@ __device__ __forceinline__ Tri child(const Tri& t, int c) {
 // a[12..14] r3 s, a[15] r3 q; kernel_0vs_0pg with sr = 0 (Kernels.h:294-345).
 template <bool GRADS, bool SRC> struct PanelSums { static constexpr int n = GRADS ? (SRC ? 16 : 15) : 3; };
 
-// the pair of panels (particles) of rows q0..q5 on one target tt = (x,x), (y,y), (z,z); `t2` the
+// the pair of panels (particles) of rows q0..q2, (wz, qs) on one target tt = (x,x), (y,y), (z,z); `t2` the
 // far thresholds; nx, ny: the pairs that are left out.  The warp votes first: almost always no
 // lane has a near pair and nothing is selected.
 template <bool GRADS, bool SRC, bool ACC>
 __device__ __forceinline__ void far_pair(const float2* tt, const float4& q0, const float4& q1, const float4& q2,
-                                         const float4& q3, const float4& q4, const float2& qs, const float2& t2,
+                                         const float2& wz, const float2& qs, const float2& t2,
                                          float2* a, bool& nx, bool& ny, bool& any) {
   const float2 dx = __fadd2_rn(tt[0], f2lo(q0));
   const float2 dy = __fadd2_rn(tt[1], f2hi(q0));
@@ -131,17 +129,19 @@ __device__ __forceinline__ void far_pair(const float2* tt, const float4& q0, con
     s2 = make_float2(nx ? 0.f : s2.x, ny ? 0.f : s2.y);
     any = true;
   }
-  const float2 wx = f2lo(q2), wy = f2hi(q2), wz = f2lo(q3);
-  const float2 nwx = f2hi(q3), nwy = f2lo(q4), nwz = f2hi(q4);
-  float2 cx = __fmul2_rn(dy, nwz), cy = __fmul2_rn(dx, wz), cz = __fmul2_rn(dx, nwy);
+  // signs on register operands, as pair2
+  const float2 wx = f2lo(q2), wy = f2hi(q2);
+  const float2 ndx = ACC ? dx : neg2(dx), ndy = ACC ? dy : neg2(dy), ndz = ACC ? dz : neg2(dz);
+  const float2 nwx = ACC ? neg2(wx) : wx, nwy = ACC ? neg2(wy) : wy, nwz = ACC ? neg2(wz) : wz;
+  float2 cx = __fmul2_rn(ndy, nwz), cy = __fmul2_rn(dx, wz), cz = __fmul2_rn(ndx, nwy);
   if (SRC) {
     cx = __ffma2_rn(dx, qs, cx);
     cy = __ffma2_rn(dy, qs, cy);
     cz = __ffma2_rn(dz, qs, cz);
   }
-  cx = __ffma2_rn(dz, wy, cx);    // dz wy - dy wz
-  cy = __ffma2_rn(dz, nwx, cy);   // dx wz - dz wx
-  cz = __ffma2_rn(dy, wx, cz);    // dy wx - dx wy
+  cx = __ffma2_rn(dz, wy, cx);     // dz wy - dy wz
+  cy = __ffma2_rn(ndz, nwx, cy);   // dx wz - dz wx
+  cz = __ffma2_rn(dy, wx, cz);     // dy wx - dx wy
   a[0] = __ffma2_rn(r3, cx, a[0]);
   a[1] = __ffma2_rn(r3, cy, a[1]);
   a[2] = __ffma2_rn(r3, cz, a[2]);
@@ -162,7 +162,7 @@ __device__ __forceinline__ void far_pair(const float2* tt, const float4& q0, con
     a[6] = __ffma2_rn(dy, cx, a[6]);
     a[9] = __ffma2_rn(dz, cx, a[9]);
     a[10] = __ffma2_rn(dz, cy, a[10]);
-    a[11] = __ffma2_rn(dz, cz, a[11]);
+    if (SRC || !ACC) a[11] = __ffma2_rn(dz, cz, a[11]);   // fold_grads' NO_ZZ otherwise
   }
 }
 
@@ -196,10 +196,10 @@ __device__ __forceinline__ void leaf(float dx, float dy, float dz, float sx, flo
 }
 
 // the 3 or 12 results from a thread's sums
-template <bool GRADS, bool SRC>
+template <bool GRADS, bool SRC, bool NO_ZZ = false>
 __device__ __forceinline__ void panel_fold(float* a) {
   if (!GRADS) return;
-  fold_grads<CORE_SING>(a);
+  fold_grads<CORE_SING, NO_ZZ>(a);
   if (SRC) {
     a[3] += a[15];
     a[7] += a[15];
@@ -235,8 +235,8 @@ template <bool GRADS, bool SRC, bool ACC> struct NodeSums {
 };
 // In dynamic shared memory: two staged tiles, then the nodes' sums, the owners' masks and the
 // nodes.
-template <int NR, int NV, int TPT> struct WarpShared {
-  float4 buf[2][NR][kPW / 2];
+template <int NV, int TPT> struct WarpShared {
+  float4 buf[2][kRows][kPW / 2];
   float sums[NV][32];      // the nodes' sums, by the lane that computed them
   unsigned mine[TPT][32];  // per owner: the lanes whose sums are its own
   uint2 node[1];           // queue_cap(TPT, maxlev) of them
@@ -323,7 +323,6 @@ __device__ __forceinline__ void sweep_panels(const float4* __restrict__ tiles, i
                                              float (*lo)[GRADS ? 12 : 3], const Fetch& fetch) {
   constexpr int NS = PanelSums<GRADS, SRC>::n;
   constexpr int NC = GRADS ? 12 : 3;
-  constexpr int NR = SRC ? kRows : kRows - 1;
   constexpr int HALF = kPW / 2;
   constexpr unsigned full = 0xffffffffu;
   const int lane = threadIdx.x;
@@ -332,9 +331,8 @@ __device__ __forceinline__ void sweep_panels(const float4* __restrict__ tiles, i
     const float4* g = tiles + (size_t)tile * (kRows * HALF);
     const unsigned d = (unsigned)__cvta_generic_to_shared(&q.buf[b][0][0]);
 #pragma unroll
-    for (int e = 0; e < NR * HALF; e += kPW)
-      if (e + lane < NR * HALF)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 16u * (e + lane)), "l"(g + e + lane) : "memory");
+    for (int e = 0; e < kRows * HALF; e += kPW)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 16u * (e + lane)), "l"(g + e + lane) : "memory");
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
   if (t0 < t1) stage(t0, 0);
@@ -346,14 +344,21 @@ __device__ __forceinline__ void sweep_panels(const float4* __restrict__ tiles, i
     const float4 (*Q)[HALF] = q.buf[cur];
 #pragma unroll 1
     for (int p = 0; p < HALF; ++p) {
-      const float4 q0 = Q[0][p], q1 = Q[1][p], q2 = Q[2][p], q3 = Q[3][p], q4 = Q[4][p];
-      const float2 qs = SRC ? f2lo(Q[NR - 1][p]) : f2(0.f);
+      const float4 q0 = Q[0][p], q1 = Q[1][p], q2 = Q[2][p];
+      float2 wz, qs = f2(0.f);
+      if (SRC) {
+        const float4 q3 = Q[3][p];
+        wz = f2lo(q3);
+        qs = f2hi(q3);
+      } else {
+        wz = *reinterpret_cast<const float2*>(&Q[3][p]);
+      }
       bool nx[TPT], ny[TPT];
       const bool last = tile + 1 == t1 && p + 1 == HALF;
       bool any = last && cnt > 0;
 #pragma unroll
       for (int k = 0; k < TPT; ++k)
-        far_pair<GRADS, SRC, ACC>(tt[k], q0, q1, q2, q3, q4, qs, OWN_T ? f2(own2[k]) : f2hi(q1), a[k], nx[k], ny[k],
+        far_pair<GRADS, SRC, ACC>(tt[k], q0, q1, q2, wz, qs, OWN_T ? f2(own2[k]) : f2hi(q1), a[k], nx[k], ny[k],
                                   any);
       if (any) {
 #pragma unroll
@@ -380,7 +385,7 @@ __device__ __forceinline__ void sweep_panels(const float4* __restrict__ tiles, i
           v[c] = a[k][c].x + a[k][c].y;
           a[k][c] = f2(0.f);
         }
-        panel_fold<GRADS, SRC>(v);
+        panel_fold<GRADS, SRC, !SRC>(v);
         fold_tile<NC>(v, hi[k], lo[k]);
       }
     }
@@ -469,7 +474,7 @@ __global__ void __launch_bounds__(kPW) k_panpt(const float4* __restrict__ tiles,
                                                OutPtrs<float> out) {
   constexpr int NC = GRADS ? 12 : 3;
   constexpr int NS = PanelSums<GRADS, SRC>::n;
-  using Shared = WarpShared<SRC ? kRows : kRows - 1, NodeSums<GRADS, SRC, ACC>::n, TPT>;
+  using Shared = WarpShared<NodeSums<GRADS, SRC, ACC>::n, TPT>;
   extern __shared__ __align__(16) char smem[];
   Shared& sh = *reinterpret_cast<Shared*>(smem);
   const int i0 = blockIdx.x * (kPW * TPT) + threadIdx.x;
@@ -531,7 +536,7 @@ __global__ void __launch_bounds__(kPW) k_ptpan(const float4* __restrict__ cen, c
                                                int np, const float4* __restrict__ tiles, int ntiles,
                                                int tiles_per_split, int maxlev, float* partial, int np_pad,
                                                OutPtrs<float> out) {
-  using Shared = WarpShared<kRows - 1, 3, TPT>;
+  using Shared = WarpShared<3, TPT>;
   extern __shared__ __align__(16) char smem[];
   Shared& sh = *reinterpret_cast<Shared*>(smem);
   const int w0 = blockIdx.x * (kPW * TPT);
@@ -583,7 +588,7 @@ __global__ void k_pack_particles(int n, int n_pad, const float* __restrict__ x, 
 template <bool GRADS, bool SRC, bool ACC, int TPT>
 static void panpt_kernel_of(int maxlev, const void** k, size_t* smem) {
   *k = (const void*)&k_panpt<GRADS, SRC, ACC, TPT>;
-  *smem = WarpShared<SRC ? kRows : kRows - 1, NodeSums<GRADS, SRC, ACC>::n, TPT>::bytes(maxlev);
+  *smem = WarpShared<NodeSums<GRADS, SRC, ACC>::n, TPT>::bytes(maxlev);
 }
 template <bool SRC, bool ACC>
 static void panpt_kernel(bool grads, int tpt, int maxlev, const void** k, size_t* smem) {
@@ -594,7 +599,7 @@ static void panpt_kernel(bool grads, int tpt, int maxlev, const void** k, size_t
 template <int TPT>
 static void ptpan_kernel(bool comp, int maxlev, const void** k, size_t* smem) {
   *k = comp ? (const void*)&k_ptpan<true, TPT> : (const void*)&k_ptpan<false, TPT>;
-  *smem = WarpShared<kRows - 1, 3, TPT>::bytes(maxlev);
+  *smem = WarpShared<3, TPT>::bytes(maxlev);
 }
 
 // Splits the swept tiles over blockIdx.y: up to 4 waves of resident blocks (their near work
