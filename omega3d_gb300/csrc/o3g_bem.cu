@@ -416,24 +416,29 @@ __global__ void __launch_bounds__(kPanelThreads) k_panel_lu(PanelArgs a) {
 // What bounds a panel is latency: one pivot exchange per column.  Through global memory
 // (k_panel_lu, 152 blocks) it costs 3.1 us a column; among the 16 blocks of one cluster the
 // candidates travel through distributed shared memory behind the hardware's cluster barrier.
-// The rows then have to fit 16 SMs: each thread keeps RPT = 2 rows of W = 64 columns in
-// registers, so up to 10,240 rows fit; a kNb-column panel is factored W columns at a time
-// (k_panel_next brings the second half up to date).  More rows than that go to k_panel_lu.
+// The rows then have to fit 16 SMs: 640 rows of W = 64 columns in a block's registers, so up to
+// 10,240 rows fit; a kNb-column panel is factored W columns at a time (k_panel_next brings the
+// second half up to date).  More rows than that go to k_panel_lu.
 //
-// Rows do not move while the sub-panel is factored: each thread tracks the position its row has
+// Rows do not move while the sub-panel is factored: each thread tracks the position its rows have
 // after the interchanges so far (LAPACK's order); the sub-panel's rows are stored there at
 // the end, and k_laswp moves the other columns'.  Pivot choice: largest |value|, lowest position on ties.
-// Inside, columns go in groups of kCpGroup.  Per column only the group's columns are touched:
-// the warps' candidates (redux), the block's candidate window sent to every block of the
-// cluster (st.async, which counts its bytes on the receiver's mbarrier), the same winner found
-// by every warp, the rank-1 update of the window.  Per group the pivot rows' other columns are
-// sent to every block, solved against the group's L (U12), and the rows take the rank-8 update
-// from registers and shared memory.
-// Measured (one GB300), factorisation at n = 10,240: 43.2 -> 31.5 ms.  Not kept: full
-// rows in every exchange with a rank-1 update of the whole width per column (2.3 us a column:
-// 500 instructions per warp and column, in series), the same fully unrolled (2.8 us: 300 KB of
-// code, fetched once), a cluster barrier instead of mbarriers (its release waits for the
-// finished columns' global stores).
+// Inside, columns go in groups of kCpGroup.  Per column only the group's columns are touched, a
+// thread holding two rows of them: the warps' candidates (redux), the best of them sent by warp 0 to
+// every block of the cluster (st.async, which counts its bytes on the receiver's mbarrier), the
+// same winner found by every warp, the rank-1 update of the window.  Per group the pivot rows'
+// later columns are sent to every block, solved against the group's L (U12), and the columns right
+// of the group, held as tiles of 4 rows x 4 columns per thread and chunk, take the rank-8 update: a
+// tile reads 4 multipliers and 4 elements of U for 16 products, and a broadcast read of shared
+// memory costs as much as 32 different words (two full rows per thread: 58 reads for 112
+// products, and this update a fifth of the kernel).
+// Measured (one GB300), 64 columns: 112 -> 86 us (one warp's instructions in series are what
+// is left: 150 a column); factorisation at n = 10,240: 43.2 -> 29.3 ms.  Not kept: full
+// rows in every exchange with a rank-1 update of the whole width per column (2.3 us a column),
+// the column's code unrolled (by 8: 108 against 97 us; fetching it takes longer than running
+// it), a block barrier and a second search by every warp before the exchange (112 against
+// 97 us), a cluster barrier instead of mbarriers (its release waits for the finished columns'
+// global stores).
 constexpr int kCpThreads = 320;
 constexpr int kCpWarps = kCpThreads / 32;
 constexpr int kCpMax = 16;                  // blocks per cluster
@@ -450,16 +455,19 @@ struct ClusterPanelArgs {
   const float* u;         // the rows of U above the sub-panel, (c - k0) x w column-major (k_panel_next)
 };
 template <int W, int RPT> struct ClusterShared {
-  static constexpr int R = W - kCpGroup;          // columns right of a group
+  static constexpr int R = W - kCpGroup;          // columns right of the first group
+  static constexpr int rows_n = RPT * kCpThreads; // rows of a block
   float xch[2][kCpGroup][kCpMax][kCpGroup];       // the blocks' candidate windows, by group parity and column
-  float rows[2][kCpGroup][R];                     // the pivot rows' other columns, by group parity
+  float rows[2][kCpGroup][R];                     // the pivot rows' later columns, by group parity
   float u12[2][kCpGroup][R];                      // the same after the solve
   float own[kCpGroup][R];                         // those that this block sends
-  float cand[2][kCpGroup];                        // this block's candidate window, by column parity
+  float cand[kCpWarps][kCpGroup];                 // the warps' candidate windows
+  float l[kCpGroup][rows_n];                      // the group's multipliers, 0 where a row takes no update
+  float4 turn[2][rows_n];                         // the next group's columns, from tiles to rows
   uint2 head[2][kCpGroup][kCpMax];                // candidates' |value| bits + 1 (0: none) and positions
+  uint2 whead[kCpWarps];                          // the warps'
   unsigned long long bar[3];                      // mbarriers: a column's candidates (by parity), a group's rows
-  unsigned wkey[2][kCpWarps], wpos[2][kCpWarps];
-  int ownk[kCpGroup];                             // the last group (+ 1) whose k-th pivot row is in this block
+  int prow[kCpGroup];                             // the group's k-th pivot row, if it is one of this block's (-1)
   float done[W * RPT * kCpThreads];               // the finished columns
 };
 __device__ __forceinline__ unsigned cluster_rank() {
@@ -496,74 +504,85 @@ __device__ __forceinline__ void cluster_send4(unsigned dst, const float4& v, uns
                "r"(bar)
                : "memory");
 }
-// the largest key of the lanes and the lowest position among those that have it (0: none)
-__device__ __forceinline__ void best_of(unsigned& key, unsigned& pos) {
+// the lane with the largest key and, among those that have it, the lowest position (distinct
+// but for keys of 0)
+__device__ __forceinline__ int best_lane(unsigned key, unsigned pos, unsigned& m) {
   constexpr unsigned full = 0xffffffffu;
-  const unsigned m = __reduce_max_sync(full, key);
-  const unsigned eq = __ballot_sync(full, m != 0u && key == m);
-  // one lane, almost always
-  pos = __popc(eq) == 1 ? __shfl_sync(full, pos, __ffs(eq) - 1) : __reduce_min_sync(full, m != 0u && key == m ? pos : full);
-  key = m;
+  m = __reduce_max_sync(full, key);
+  unsigned eq = __ballot_sync(full, key == m);
+  if ((eq & (eq - 1u)) != 0u && m != 0u) {
+    const unsigned p = __reduce_min_sync(full, key == m ? pos : full);
+    eq = __ballot_sync(full, key == m && pos == p);
+  }
+  return __ffs(eq) - 1;
 }
 // waits (bounded) for the mbarrier's phase; every thread for itself.  All blocks of a cluster are
 // resident, so it can only run out if one of them faults.
 __device__ __forceinline__ bool cluster_wait(unsigned bar, unsigned parity, int* err) {
-  for (unsigned it = 0; it < (1u << 21); ++it) {   // each try suspends for 1 us at most
-    unsigned done;
+  unsigned done = 0u;
+  // polled first (a suspended wait wakes up later), then with suspensions of up to 1 us
+  for (int it = 0; it < 4096 && !done; ++it)
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(done)
+                 : "r"(bar), "r"(parity)
+                 : "memory");
+  for (unsigned it = 0; it < (1u << 21) && !done; ++it)
     asm volatile(
         "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 1000;\n\tselp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(done)
         : "r"(bar), "r"(parity)
         : "memory");
-    if (done) return true;
-  }
+  if (done) return true;
   atomicExch(err, 1);
   return false;
 }
 
-// rank-kCpGroup update of the columns [kCpGroup, V) of the rows' windows: row by row the
-// multipliers are x[q][0..kCpGroup), but a pivot row of this group takes only the earlier ones
-// and a finished row none.  (Rolled over k, the multipliers turning through x[.][0].)
-template <int V, int W, int RPT>
-__device__ __forceinline__ void panel_update(float (*x)[W], const int* pos, int cg, const float (*u12)[W - kCpGroup]) {
-  constexpr int B = kCpGroup;
+// A block's rows right of the group: warp w holds the rows 128 (w % 5) + lane + 32 i, i < 4, and of
+// every group's 8 columns the half w / 5 (chunk c: columns 8 (c + 1) + 4 (w / 5) .. + 3).
+template <int W> struct PanelTile {
+  static constexpr int NCH = W / kCpGroup - 1;
+  float4 y[4][NCH];
+};
+// their rank-kCpGroup update after group g: y -= l u
+template <int W, class Shared>
+__device__ __forceinline__ void panel_update(PanelTile<W>& t, const Shared& sh, int g, int gp, int rb, int cb) {
+  constexpr int kHalfK = kCpGroup / 2;   // multipliers in registers at a time
+  const int lane = threadIdx.x & 31;
 #pragma unroll 1
-  for (int k = 0; k < B; ++k) {
-    float l[RPT];
+  for (int k0 = 0; k0 < kCpGroup; k0 += kHalfK) {
+    float l[kHalfK][4];
 #pragma unroll
-    for (int q = 0; q < RPT; ++q) l[q] = pos[q] > cg + k ? x[q][0] : 0.f;
+    for (int k = 0; k < kHalfK; ++k)
 #pragma unroll
-    for (int v = 0; v < (V - B) / 4; ++v) {
-      const float4 u = reinterpret_cast<const float4*>(u12[k])[v];
+      for (int i = 0; i < 4; ++i) l[k][i] = -sh.l[k0 + k][128 * rb + lane + 32 * i];
 #pragma unroll
-      for (int q = 0; q < RPT; ++q) {
-        float* y = &x[q][B + 4 * v];
-        y[0] = fmaf(-l[q], u.x, y[0]);
-        y[1] = fmaf(-l[q], u.y, y[1]);
-        y[2] = fmaf(-l[q], u.z, y[2]);
-        y[3] = fmaf(-l[q], u.w, y[3]);
-      }
-    }
+    for (int c = 0; c < PanelTile<W>::NCH; ++c)
+      if (c >= g)
 #pragma unroll
-    for (int q = 0; q < RPT; ++q) {
-      const float t = x[q][0];
+        for (int k = 0; k < kHalfK; ++k) {
+          const float4 u = *reinterpret_cast<const float4*>(&sh.u12[gp][k0 + k][8 * c + 4 * cb]);
 #pragma unroll
-      for (int e = 0; e + 1 < B; ++e) x[q][e] = x[q][e + 1];
-      x[q][B - 1] = t;
-    }
+          for (int i = 0; i < 4; ++i) {
+            float4& y = t.y[i][c];
+            const float2 lo = __ffma2_rn(make_float2(l[k][i], l[k][i]), make_float2(u.x, u.y), make_float2(y.x, y.y));
+            const float2 hi = __ffma2_rn(make_float2(l[k][i], l[k][i]), make_float2(u.z, u.w), make_float2(y.z, y.w));
+            y = make_float4(lo.x, lo.y, hi.x, hi.y);
+          }
+        }
   }
 }
 
-// One group of columns; x[.][0..W) is the window that starts at the group's first column.  The
-// finished columns are kept in shared memory and the window slides on.
+// One group of columns; x[.][0..kCpGroup) are the rows tid and tid + kCpThreads, t what lies right of it.
 template <int W, int RPT>
-__device__ __forceinline__ void panel_group(const ClusterPanelArgs& a, ClusterShared<W, RPT>& sh, float (*x)[W], int* pos,
-                                            int row0, int g0, unsigned rank, unsigned C, bool& dead) {
+__device__ __forceinline__ void panel_group(const ClusterPanelArgs& a, ClusterShared<W, RPT>& sh, float (*x)[kCpGroup],
+                                            PanelTile<W>& t, int* pos, int g0, unsigned rank, unsigned C, bool& dead) {
   constexpr unsigned full = 0xffffffffu;
   constexpr int B = kCpGroup, R = W - B;
+  auto off = [&](const void* p) { return (unsigned)((const char*)p - (const char*)&sh); };
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int cg = a.c + g0, gp = (g0 / B) & 1;
   const int nb = min(B, a.w - g0);
+  const unsigned peer = cluster_map(&sh, (unsigned)(lane & 15) < C ? lane & 15 : 0);
   unsigned win = 0u;   // the winners' blocks, 4 bits each
   // one copy of the column's code (unrolled eight times, fetching it took longer than running
   // it): the current column is always x[.][0], and the group's window turns by one per column
@@ -571,55 +590,53 @@ __device__ __forceinline__ void panel_group(const ClusterPanelArgs& a, ClusterSh
   for (int jj = 0; jj < B; ++jj) {
     if (jj < nb) {
       const int cj = cg + jj, par = jj & 1;
-      // this thread's candidate, the warp's, the block's
+      // this thread's candidate, the warp's
       unsigned key = 0u, mp = full;
       int mq = 0;
 #pragma unroll
       for (int q = 0; q < RPT; ++q) {
-        const float v = fabsf(x[q][0]);
-        const unsigned kq = pos[q] >= cj && v >= 0.f ? __float_as_uint(v) + 1u : 0u;   // NaN: no candidate
-        if (kq > key || (kq == key && kq != 0u && (unsigned)pos[q] < mp)) { key = kq; mp = (unsigned)pos[q]; mq = q; }
+        const unsigned v = __float_as_uint(x[q][0]) & 0x7fffffffu;
+        const unsigned kq = (pos[q] >= cj) & (v <= 0x7f800000u) ? v + 1u : 0u;   // NaN: no candidate
+        const bool take = (kq > key) | ((kq == key) & ((unsigned)pos[q] < mp));
+        key = take ? kq : key;
+        mp = take ? (unsigned)pos[q] : mp;
+        mq = take ? q : mq;
       }
-      unsigned m = key, p = mp;
-      best_of(m, p);
-      // (wkey and wpos are double-buffered: a warp may be through this column's wait while
-      // another still reads them)
-      if (lane == 0) { sh.wkey[par][warp] = m; sh.wpos[par][warp] = p; }
-      const unsigned mw = m, pw_ = p;
-      __syncthreads();
-      m = lane < kCpWarps ? sh.wkey[par][lane] : 0u;
-      p = lane < kCpWarps ? sh.wpos[par][lane] : full;
-      best_of(m, p);
-      if (m != 0u ? (mw == m && pw_ == p) : warp == 0) {
-        // this warp holds the block's candidate: its window and head to every block
-        if (m != 0u && key == m && mp == p) {
+      unsigned m;
+      if (lane == best_lane(key, mp, m)) {
 #pragma unroll
-          for (int v = 0; v < B / 4; ++v) {
-            float4 r = make_float4(x[0][4 * v], x[0][4 * v + 1], x[0][4 * v + 2], x[0][4 * v + 3]);
+        for (int v = 0; v < B / 4; ++v) {
+          float4 r = make_float4(x[0][4 * v], x[0][4 * v + 1], x[0][4 * v + 2], x[0][4 * v + 3]);
 #pragma unroll
-            for (int q = 1; q < RPT; ++q)
-              if (mq == q) r = make_float4(x[q][4 * v], x[q][4 * v + 1], x[q][4 * v + 2], x[q][4 * v + 3]);
-            reinterpret_cast<float4*>(sh.cand[par])[v] = r;
-          }
+          for (int q = 1; q < RPT; ++q)
+            if (mq == q) r = make_float4(x[q][4 * v], x[q][4 * v + 1], x[q][4 * v + 2], x[q][4 * v + 3]);
+          reinterpret_cast<float4*>(sh.cand[warp])[v] = r;
         }
-        __syncwarp();
+        sh.whead[warp] = make_uint2(key, mp);
+      }
+      __syncwarp();
+      // warp 0 finds the block's and sends its window and head to every block
+      if (warp == 0) {
+        asm volatile("bar.sync 1, %0;" ::"n"(kCpThreads) : "memory");
+        const uint2 hw = lane < kCpWarps ? sh.whead[lane] : make_uint2(0u, full);
+        const int wi = best_lane(hw.x, hw.y, m);
+        const uint2 hs = make_uint2(m, __shfl_sync(full, hw.y, wi));
+        if (lane == 0) cluster_expect((unsigned)__cvta_generic_to_shared(&sh.bar[par]), C * (B * 4 + 8));
         const int to = lane & 15, h = lane >> 4;
         if (to < (int)C) {
-          const unsigned bar = cluster_map(&sh.bar[par], to);
-          cluster_send4(cluster_map(&sh.xch[gp][jj][rank][4 * h], to), reinterpret_cast<const float4*>(sh.cand[par])[h], bar);
-          if (h == 0) cluster_send(cluster_map(&sh.head[gp][jj][rank], to), m, p, bar);
+          const unsigned bar = peer + off(&sh.bar[par]);
+          cluster_send4(peer + off(&sh.xch[gp][jj][rank][4 * h]), reinterpret_cast<const float4*>(sh.cand[wi])[h], bar);
+          if (h == 0) cluster_send(peer + off(&sh.head[gp][jj][rank]), hs.x, hs.y, bar);
         }
+      } else {
+        asm volatile("bar.arrive 1, %0;" ::"n"(kCpThreads) : "memory");
       }
       const unsigned bar = (unsigned)__cvta_generic_to_shared(&sh.bar[par]);
-      if (tid == 0) cluster_expect(bar, C * (B * 4 + 8));
       if (!dead) dead = !cluster_wait(bar, (unsigned)((g0 + jj) >> 1) & 1u, a.err);
       // the cluster's pivot, found by every warp alike
       const uint2 hd = lane < (int)C ? sh.head[gp][jj][lane] : make_uint2(0u, full);
-      m = hd.x;
-      p = hd.y;
-      best_of(m, p);
-      const unsigned hit = __ballot_sync(full, m != 0u && hd.x == m && hd.y == p);
-      const unsigned wb = hit ? (unsigned)__ffs(hit) - 1u : 0u;
+      const unsigned wb = (unsigned)best_lane(hd.x, hd.y, m) % kCpMax;
+      const unsigned p = __shfl_sync(full, hd.y, wb);
       win |= wb << (4 * jj);
       const float* u = sh.xch[gp][jj][wb];
       // no finite candidate (or a wait that ran out): keep the row
@@ -631,8 +648,7 @@ __device__ __forceinline__ void panel_group(const ClusterPanelArgs& a, ClusterSh
       }
 #pragma unroll
       for (int q = 0; q < RPT; ++q) {
-        if (pos[q] == cj) pos[q] = pw;
-        else if (pos[q] == pw) pos[q] = cj;
+        pos[q] = pos[q] == cj ? pw : pos[q] == pw ? cj : pos[q];
       }
       if (pv != 0.f) {
         float ue[B];
@@ -648,22 +664,27 @@ __device__ __forceinline__ void panel_group(const ClusterPanelArgs& a, ClusterSh
         // x / pv by the reciprocal and one correction (the quotient to within an ulp) where nothing
         // overflows on the way; the division itself otherwise
         const float ap = fabsf(pv);
-        const bool mid = ap > 1e-30f && ap < 1e30f;
-        const float rp = mid ? __frcp_rn(pv) : 0.f;
+        float l[RPT];
+        if (ap > 1e-30f && ap < 1e30f) {
+          float rp;
+          asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rp) : "f"(pv));
 #pragma unroll
-        for (int q = 0; q < RPT; ++q)
-          if (pos[q] > cj) {
-            float l;
-            if (mid) {
-              l = x[q][0] * rp;
-              l = fmaf(fmaf(-l, pv, x[q][0]), rp, l);
-            } else {
-              l = x[q][0] / pv;
-            }
-            x[q][0] = l;
-#pragma unroll
-            for (int k = 1; k < B; ++k) x[q][k] = fmaf(-l, ue[k], x[q][k]);
+          for (int q = 0; q < RPT; ++q) {
+            l[q] = x[q][0] * rp;
+            l[q] = fmaf(fmaf(-l[q], pv, x[q][0]), rp, l[q]);
           }
+        } else {
+#pragma unroll
+          for (int q = 0; q < RPT; ++q) l[q] = x[q][0] / pv;
+        }
+#pragma unroll
+        for (int q = 0; q < RPT; ++q) {
+          const bool below = pos[q] > cj;
+          if (below) x[q][0] = l[q];
+#pragma unroll
+          for (int k = 1; k < B; ++k)
+            if (below) x[q][k] = fmaf(-l[q], ue[k], x[q][k]);
+        }
       }
     }
 #pragma unroll
@@ -674,53 +695,88 @@ __device__ __forceinline__ void panel_group(const ClusterPanelArgs& a, ClusterSh
       x[q][B - 1] = t;
     }
   }
-  if (g0 + B < a.w) {
-    // the group's pivot rows, right of it, to every block
+  const int g = g0 / B, rb = warp % 5, cb = warp / 5;
+  const bool more = g0 + B < a.w;
+  if (more) {
+    // which rows the pivots are
 #pragma unroll
     for (int q = 0; q < RPT; ++q) {
-      const int k = pos[q] - cg;
-      if (k >= 0 && k < B) {
-        sh.ownk[k] = g0 + 1;
-#pragma unroll
-        for (int v = 0; v < R / 4; ++v)
-          reinterpret_cast<float4*>(sh.own[k])[v] =
-              make_float4(x[q][B + 4 * v], x[q][B + 4 * v + 1], x[q][B + 4 * v + 2], x[q][B + 4 * v + 3]);
-      }
+      const int e = pos[q] - cg;
+      if ((unsigned)e < (unsigned)B) sh.prow[e] = (tid + q * kCpThreads) | (g0 << 16);
     }
+    if (tid == 0) cluster_expect((unsigned)__cvta_generic_to_shared(&sh.bar[2]), B * (R - g0) * 4);
     __syncthreads();
-    for (int e = warp; e < B * (int)C; e += kCpWarps) {   // a warp per row and destination
-      const int k = e % B, to = e / B;
-      if (sh.ownk[k] == g0 + 1 && lane < R / 4)
-        cluster_send4(cluster_map(&sh.rows[gp][k][4 * lane], to), reinterpret_cast<const float4*>(sh.own[k])[lane],
-                      cluster_map(&sh.bar[2], to));
-    }
-    const unsigned bar = (unsigned)__cvta_generic_to_shared(&sh.bar[2]);
-    if (tid == 0) cluster_expect(bar, B * R * 4);
-    if (!dead) dead = !cluster_wait(bar, (unsigned)gp, a.err);
-    // U12 = L11^-1 A12 of the group, a thread per column; L11 from the pivots' windows
-    if (tid < R) {
-      float uu[B];
+    // their columns right of the group to every block, by the warps that hold them
+    const unsigned barb = off(&sh.bar[2]);
+    const int mine = sh.prow[lane & 7];
+    unsigned todo = __ballot_sync(full, lane < B && (mine >> 16) == g0 && (mine & 0xffff) / 128 == rb);
+    while (todo) {
+      const int k = __ffs(todo) - 1;
+      todo &= todo - 1u;
+      const int r = __shfl_sync(full, mine, k) & 0xffff, ri = (r >> 5) & 3;
+      if (lane == (r & 31))
 #pragma unroll
-      for (int k = 0; k < B; ++k) {
-        // the k-th pivot's window starts at its own column: its multipliers e < k are at B - k + e
-        const float* lk = sh.xch[gp][k][(win >> (4 * k)) & 15u];
-        float v = sh.rows[gp][k][tid];
+        for (int i = 0; i < 4; ++i)
+          if (i == ri)
 #pragma unroll
-        for (int e = 0; e < k; ++e) v = fmaf(-lk[B - k + e], uu[e], v);
-        uu[k] = v;
-        sh.u12[gp][k][tid] = v;
+            for (int c = 0; c < PanelTile<W>::NCH; ++c) {
+              float* o = &sh.own[k][8 * c + 4 * cb];
+              asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"((unsigned)__cvta_generic_to_shared(o)),
+                           "f"(t.y[i][c].x), "f"(t.y[i][c].y), "f"(t.y[i][c].z), "f"(t.y[i][c].w) : "memory");
+            }
+      __syncwarp();
+      // 8 lanes per destination
+      const int c = lane & 7;
+      if (c >= g && c < PanelTile<W>::NCH) {
+        const float4 v = *reinterpret_cast<const float4*>(&sh.own[k][8 * c + 4 * cb]);
+        for (unsigned to = lane >> 3; to < C; to += 4) {
+          const unsigned dst = cluster_map(&sh, to);
+          cluster_send4(dst + off(&sh.rows[gp][k][8 * c + 4 * cb]), v, dst + barb);
+        }
       }
+      __syncwarp();
     }
-    __syncthreads();
-    if (g0 < W / 2) panel_update<W, W, RPT>(x, pos, cg, sh.u12[gp]);
-    else            panel_update<W / 2, W, RPT>(x, pos, cg, sh.u12[gp]);
+    // the rows' multipliers: a pivot row of this group takes only the earlier ones, a finished row none
+#pragma unroll
+    for (int q = 0; q < RPT; ++q)
+#pragma unroll
+      for (int k = 0; k < B; ++k) sh.l[k][tid + q * kCpThreads] = pos[q] - cg > k ? x[q][k] : 0.f;
   }
 #pragma unroll
+  for (int q = 0; q < RPT; ++q)
+#pragma unroll
+    for (int k = 0; k < B; ++k) sh.done[((g0 + k) * RPT + q) * kCpThreads + tid] = x[q][k];
+  if (!more) return;
+  const unsigned bar = (unsigned)__cvta_generic_to_shared(&sh.bar[2]);
+  if (!dead) dead = !cluster_wait(bar, (unsigned)gp, a.err);
+  // U12 = L11^-1 A12 of the group, a thread per column; L11 from the pivots' windows
+  if (tid >= g0 && tid < R) {
+    float uu[B];
+#pragma unroll
+    for (int k = 0; k < B; ++k) {
+      // the k-th pivot's window starts at its own column: its multipliers e < k are at B - k + e
+      const float* lk = sh.xch[gp][k][(win >> (4 * k)) & 15u];
+      float v = sh.rows[gp][k][tid];
+#pragma unroll
+      for (int e = 0; e < k; ++e) v = fmaf(-lk[B - k + e], uu[e], v);
+      uu[k] = v;
+      sh.u12[gp][k][tid] = v;
+    }
+  }
+  __syncthreads();
+  panel_update<W>(t, sh, g, gp, rb, cb);
+  // the next group's columns to the threads of their rows
+#pragma unroll
+  for (int c = 0; c < PanelTile<W>::NCH; ++c)
+    if (c == g)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) sh.turn[cb][128 * rb + lane + 32 * i] = t.y[i][c];
+  __syncthreads();
+#pragma unroll
   for (int q = 0; q < RPT; ++q) {
-#pragma unroll
-    for (int jj = 0; jj < B; ++jj) sh.done[((g0 + jj) * RPT + q) * kCpThreads + tid] = x[q][jj];
-#pragma unroll
-    for (int k = 0; k < W; ++k) x[q][k] = k + B < W ? x[q][k + B] : 0.f;
+    const float4 v0 = sh.turn[0][tid + q * kCpThreads], v1 = sh.turn[1][tid + q * kCpThreads];
+    x[q][0] = v0.x; x[q][1] = v0.y; x[q][2] = v0.z; x[q][3] = v0.w;
+    x[q][4] = v1.x; x[q][5] = v1.y; x[q][6] = v1.z; x[q][7] = v1.w;
   }
 }
 
@@ -731,7 +787,8 @@ __global__ void __launch_bounds__(kCpThreads, 1) k_panel_cluster(const ClusterPa
   using Sh = ClusterShared<W, RPT>;
   static_assert(offsetof(Sh, rows) % 16 == 0 && offsetof(Sh, u12) % 16 == 0 &&
                     offsetof(Sh, own) % 16 == 0 && offsetof(Sh, cand) % 16 == 0 && (W - kCpGroup) % 4 == 0 &&
-                    offsetof(Sh, xch) % 16 == 0 && offsetof(Sh, head) % 8 == 0 && offsetof(Sh, bar) % 8 == 0,
+                    offsetof(Sh, xch) % 16 == 0 && offsetof(Sh, turn) % 16 == 0 && offsetof(Sh, head) % 8 == 0 &&
+                    offsetof(Sh, whead) % 8 == 0 && offsetof(Sh, bar) % 8 == 0,
                 "vector accesses");
   static_assert(kCpMax <= 16 && kCpGroup == 8 && (W - kCpGroup) / 4 <= 32, "lanes per destination");
   static_assert(W - kCpGroup <= kCpThreads, "a thread per column of U12");
@@ -740,7 +797,9 @@ __global__ void __launch_bounds__(kCpThreads, 1) k_panel_cluster(const ClusterPa
   const unsigned rank = cluster_rank(), C = cluster_size();
   const int c = a.c, w = a.w, kp = a.c - a.k0;
   const int row0 = c + (int)rank * (kCpThreads * RPT) + tid;   // this thread's rows: row0 + q kCpThreads
-  float x[RPT][W];
+  static_assert(W == 64 && RPT == 2 && kCpThreads == 320, "tiles of 128 rows");
+  float x[RPT][kCpGroup];
+  PanelTile<W> t;
   int pos[RPT];
 #pragma unroll
   for (int q = 0; q < RPT; ++q) {
@@ -748,9 +807,22 @@ __global__ void __launch_bounds__(kCpThreads, 1) k_panel_cluster(const ClusterPa
     const bool in = r < a.n;
     pos[q] = in ? r : -1;
 #pragma unroll
-    for (int k = 0; k < W; ++k) x[q][k] = in && k < w ? a.A[(size_t)(c + k) * a.ld + r] : 0.f;
+    for (int k = 0; k < kCpGroup; ++k) x[q][k] = in && k < w ? a.A[(size_t)(c + k) * a.ld + r] : 0.f;
   }
-  if (tid < kCpGroup) sh.ownk[tid] = 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = c + (int)rank * (kCpThreads * RPT) + 128 * ((tid >> 5) % 5) + (tid & 31) + 32 * i;
+#pragma unroll
+    for (int e = 0; e < PanelTile<W>::NCH; ++e) {
+      const int k = 8 * (e + 1) + 4 * ((tid >> 5) / 5);
+      const float* g = a.A + (size_t)(c + k) * a.ld + r;
+      t.y[i][e].x = r < a.n && k < w ? g[0] : 0.f;
+      t.y[i][e].y = r < a.n && k + 1 < w ? g[a.ld] : 0.f;
+      t.y[i][e].z = r < a.n && k + 2 < w ? g[2 * a.ld] : 0.f;
+      t.y[i][e].w = r < a.n && k + 3 < w ? g[3 * a.ld] : 0.f;
+    }
+  }
+  if (tid < kCpGroup) sh.prow[tid] = -1;
   if (tid == 0) {
 #pragma unroll
     for (int b = 0; b < 3; ++b)
@@ -764,7 +836,7 @@ __global__ void __launch_bounds__(kCpThreads, 1) k_panel_cluster(const ClusterPa
   cluster_barrier();   // every block runs: its shared memory may be written
   bool dead = false;
 #pragma unroll 1
-  for (int g0 = 0; g0 < w; g0 += kCpGroup) panel_group<W, RPT>(a, sh, x, pos, row0, g0, rank, C, dead);
+  for (int g0 = 0; g0 < w; g0 += kCpGroup) panel_group<W, RPT>(a, sh, x, t, pos, g0, rank, C, dead);
   // every row to the place the interchanges gave it
 #pragma unroll 4
   for (int k = 0; k < w; ++k)
