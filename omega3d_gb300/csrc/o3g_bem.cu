@@ -110,19 +110,25 @@ inline cudaError_t zero_barrier(int* flags, cudaStream_t st) { return cudaMemset
 // loads in flight per thread before the stores (a plain load->store loop is latency-bound)
 __device__ __forceinline__ void stage_in(float* __restrict__ dst, int ldd, const float* __restrict__ src, long long ld,
                                          int rows, int cols) {
-  const int total = rows * cols;
-  for (int e0 = threadIdx.x; e0 < total; e0 += 8 * blockDim.x) {
+  const int nw = blockDim.x / 32, lane = threadIdx.x & 31;
+  const int nrb = (rows + 31) / 32, dcol = nw / nrb, drb = nw % nrb;
+  int col = (threadIdx.x >> 5) / nrb, rb = (threadIdx.x >> 5) % nrb;
+  while (col < cols) {
     float v[8];
+    int d[8];
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
-      const int e = e0 + q * blockDim.x;
-      v[q] = e < total ? __ldg(src + (size_t)(e / rows) * ld + (e % rows)) : 0.f;
+      const int r = 32 * rb + lane;
+      const bool in = col < cols && r < rows;
+      v[q] = in ? __ldg(src + (size_t)col * ld + r) : 0.f;
+      d[q] = in ? col * ldd + r : -1;
+      col += dcol;
+      rb += drb;
+      if (rb >= nrb) { rb -= nrb; ++col; }
     }
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int e = e0 + q * blockDim.x;
-      if (e < total) dst[(size_t)(e / rows) * ldd + (e % rows)] = v[q];
-    }
+    for (int q = 0; q < 8; ++q)
+      if (d[q] >= 0) dst[d[q]] = v[q];
   }
 }
 __device__ __forceinline__ void stage_out(float* __restrict__ dst, long long ld, const float* __restrict__ src, int lds,
@@ -433,7 +439,8 @@ __global__ void __launch_bounds__(kPanelThreads) k_panel_lu(PanelArgs a) {
 // memory costs as much as 32 different words (two full rows per thread: 58 reads for 112
 // products, and this update a fifth of the kernel).
 // Measured (one GB300), 64 columns: 112 -> 86 us (one warp's instructions in series are what
-// is left: 150 a column); factorisation at n = 10,240: 43.2 -> 29.3 ms.  Not kept: full
+// is left: 150 a column); factorisation at n = 10,240: 43.2 -> 29.3 ms (23.2 with the
+// kernels below).  Not kept: full
 // rows in every exchange with a rank-1 update of the whole width per column (2.3 us a column),
 // the column's code unrolled (by 8: 108 against 97 us; fetching it takes longer than running
 // it), a block barrier and a second search by every warp before the exchange (112 against
@@ -1005,64 +1012,69 @@ static int32_t launch_cluster_panel(const ClusterPlan& p, ClusterPanelArgs a, cu
   return O3G_OK;
 }
 
-// row interchanges p0..p1-1 (piv) applied to the columns [c0, c1) outside [s0, s1).  Each
-// block first composes the interchanges into one permutation of the rows they touch (the
-// np rows [p0, p1) and the distinct pivot rows below p1): slot s holds row rowof[s], and
-// after all interchanges the value of slot perm[s] ends up in slot s.  Then one warp per
-// column gathers the touched values and scatters them permuted: two parallel passes per
-// column instead of a chain of dependent loads.
-// dynamic shared memory for np interchanges: 8 warps' segments of 2 np floats, then pv,
-// slot_of (np ints each), rowof, perm (2 np ints each)
-inline size_t laswp_smem(int np_) { return (size_t)(8 * 2 * np_ + 6 * np_) * 4; }
-__global__ void __launch_bounds__(256) k_laswp(float* A, long long ld, int n, int p0, int p1, const int* piv, int c0,
-                                               int c1, int s0, int s1) {
+// Row interchanges p0..p1-1 (piv) as one gather: the rows they touch are [p0, p1) and the pivot
+// rows below, and a row's final value comes from where the interchanges, undone one by one from
+// the last to the first, lead back to.  Slot q of 2 np: row p0 + q, or the pivot row piv[p0 + q -
+// np] (-1 where that is not below p1; a row named twice is moved twice, to the same effect).
+// Every slot walks for itself: np steps of a few instructions on broadcast reads, where one thread
+// applying the interchanges in turn took most of 10 us for 64 and 40 us for 512 (k_laswp then:
+// 10.5 and 117 us at n = 10,240, now 5.4 and 9 + 13).
+__device__ __forceinline__ int2 row_slot(const int* pv, int p0, int np_, int n, int q) {
+  int row = q < np_ ? p0 + q : pv[q - np_];
+  if (q >= np_ && row < p0 + np_) row = -1;
+  int src = row;
+#pragma unroll 8
+  for (int e = np_ - 1; e >= 0; --e) {
+    const int a = p0 + e, b = pv[e];
+    src = src == a ? b : src == b ? a : src;
+  }
+  return make_int2(row, src);
+}
+// pv[e] = the pivot row of step e; one that is no interchange (or out of range) is the step's own row
+__device__ __forceinline__ void stage_pivots(int* pv, const int* piv, int p0, int np_, int n) {
+  for (int e = threadIdx.x; e < np_; e += blockDim.x) {
+    const int b = piv[p0 + e];
+    pv[e] = b < p0 + e || b >= n ? p0 + e : b;
+  }
+}
+// the slots of many interchanges, for k_laswp's blocks to share
+constexpr int kSwapInline = 128;   // up to this many, each block finds them itself
+__global__ void __launch_bounds__(128) k_row_map(const int* __restrict__ piv, int p0, int np_, int n, int2* map) {
+  extern __shared__ int rmsm[];
+  stage_pivots(rmsm, piv, p0, np_, n);
+  __syncthreads();
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q < 2 * np_) map[q] = row_slot(rmsm, p0, np_, n, q);
+}
+// The interchanges on the columns [c0, c1) outside [s0, s1): one warp per column gathers the rows
+// that change and scatters them, 8 loads in flight per lane.  Rows that stay are left alone.
+// dynamic shared memory for np interchanges: 8 warps' segments of 2 np floats, then the rows,
+// their sources (2 np ints each) and the pivots (np)
+inline size_t laswp_smem(int np_) { return (size_t)(8 * 2 * np_ + 5 * np_) * 4; }
+__global__ void __launch_bounds__(256) k_laswp(float* A, long long ld, int n, int p0, int p1, const int* piv,
+                                               const int2* map, int c0, int c1, int s0, int s1) {
   extern __shared__ float lsw[];
   const int np_ = p1 - p0;
   float* segs = lsw;                                         // [8][2 np]
-  int* pv = reinterpret_cast<int*>(segs + 8 * 2 * np_);      // [np]
-  int* slot_of = pv + np_;                                   // [np]: slot of pivot row pv[e]
-  int* rowof = slot_of + np_;                                // [2 np]
-  int* perm = rowof + 2 * np_;                               // [2 np]
+  int* rowof = reinterpret_cast<int*>(segs + 8 * 2 * np_);   // [2 np]
+  int* srcof = rowof + 2 * np_;                              // [2 np]
+  int* pv = srcof + 2 * np_;                                 // [np]
   __shared__ int nslots;
-  for (int e = threadIdx.x; e < np_; e += blockDim.x) pv[e] = piv[p0 + e];
+  if (threadIdx.x == 0) nslots = 0;
+  if (!map) stage_pivots(pv, piv, p0, np_, n);
   __syncthreads();
-  // the first interchange naming each pivot row below p1 (the same row can be named twice)
-  for (int e = threadIdx.x; e < np_; e += blockDim.x) {
-    const int p = pv[e];
-    int first = e;
-    if (p >= p1 && p < n)
-      for (int f = 0; f < e; ++f)
-        if (pv[f] == p) { first = f; break; }
-    slot_of[e] = first;   // provisional: the first occurrence's index
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int ns = np_;
-    for (int e = 0; e < np_; ++e) rowof[e] = p0 + e;
-    for (int e = 0; e < np_; ++e) {
-      const int p = pv[e];
-      if (p < p1 || p >= n) {
-        slot_of[e] = (p >= p0 && p < p1) ? p - p0 : -1;
-      } else if (slot_of[e] == e) {
-        rowof[ns] = p;
-        slot_of[e] = ns++;
-      } else {
-        slot_of[e] = slot_of[slot_of[e]];   // the earlier occurrence's slot (already final)
-      }
+  // (the slots' order does not matter)
+  for (int q = threadIdx.x; q < 2 * np_; q += blockDim.x) {
+    const int2 m = map ? map[q] : row_slot(pv, p0, np_, n, q);
+    if (m.x != m.y) {
+      const int at = atomicAdd(&nslots, 1);
+      rowof[at] = m.x;
+      srcof[at] = m.y;
     }
-    for (int q = 0; q < ns; ++q) perm[q] = q;
-    for (int e = 0; e < np_; ++e) {
-      const int p = pv[e];
-      if (p == p0 + e || p < p0 + e || p >= n) continue;
-      const int s2 = slot_of[e];
-      const int t = perm[e];
-      perm[e] = perm[s2];
-      perm[s2] = t;
-    }
-    nslots = ns;
   }
   __syncthreads();
   const int ns = nslots;
+  if (ns == 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int skip = (s1 > s0) ? (s1 - s0) : 0;
   const int ncol = c1 - c0 - skip;
@@ -1071,118 +1083,176 @@ __global__ void __launch_bounds__(256) k_laswp(float* A, long long ld, int n, in
     if (skip && col >= s0) col += skip;
     float* a = A + (size_t)col * ld;
     float* seg = segs + (size_t)warp * 2 * np_;
-    for (int q = lane; q < ns; q += 32) seg[q] = a[rowof[perm[q]]];
+    for (int q0 = lane; q0 < ns; q0 += 256) {
+      float v[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] = q0 + 32 * e < ns ? a[srcof[q0 + 32 * e]] : 0.f;
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        if (q0 + 32 * e < ns) seg[q0 + 32 * e] = v[e];
+    }
     __syncwarp();
     for (int q = lane; q < ns; q += 32) a[rowof[q]] = seg[q];
     __syncwarp();
   }
 }
 
-// B = L^-1 B for a unit lower jb x jb L (column-major at Lp, leading dimension ldl) and the
-// ncols columns of B (jb rows at Bp, leading dimension ldb): one warp per column of B, L in
-// shared memory
-__global__ void __launch_bounds__(256) k_trsm_unit_lower(const float* Lp, long long ldl, int jb, float* Bp,
-                                                         long long ldb, int ncols) {
-  extern __shared__ float L[];   // [jb][jb] column-major
-  stage_in(L, jb, Lp, ldl, jb, jb);
-  __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int cidx = blockIdx.x * (blockDim.x / 32) + warp; cidx < ncols; cidx += gridDim.x * (blockDim.x / 32)) {
-    float* col = Bp + (size_t)cidx * ldb;
-    float x[kNb / 32];
+// x <- L^-1 x for a unit lower L (columns of kNb floats in shared memory, zero below row jb; what lies
+// above its diagonal is not used), lane l holding rows l + 32 q: steps [32 b0, jb).  Both indices
+// into x are constants after unrolling.
+__device__ __forceinline__ void unit_lower_solve(float* x, const float* L, int jb, int b0) {
+  constexpr int NQ = kNb / 32;
+  const int lane = threadIdx.x & 31;
 #pragma unroll
-    for (int q = 0; q < kNb / 32; ++q) x[q] = (q * 32 + lane < jb) ? col[q * 32 + lane] : 0.f;
-    for (int i = 0; i < jb; ++i) {
-      const float xi = __shfl_sync(0xffffffffu, x[i >> 5], i & 31);
+  for (int b = 0; b < NQ; ++b) {
+    if (b < b0 || 32 * b >= jb) continue;
+#pragma unroll 8
+    for (int il = 0; il < 32; ++il) {
+      const float* col = L + (size_t)(32 * b + il) * kNb + lane;   // (a column beyond jb is zero)
+      const float xi = __shfl_sync(0xffffffffu, x[b], il);
+      x[b] = fmaf(lane > il ? -col[32 * b] : 0.f, xi, x[b]);
 #pragma unroll
-      for (int q = 0; q < kNb / 32; ++q) {
-        const int m = q * 32 + lane;
-        if (m > i && m < jb) x[q] = fmaf(-L[(size_t)i * jb + m], xi, x[q]);
-      }
+      for (int q = b + 1; q < NQ; ++q) x[q] = fmaf(-col[32 * q], xi, x[q]);
     }
+  }
+}
+// the jb x jb block at src into columns of kNb floats, zero beyond it
+__device__ __forceinline__ void stage_block(float* dst, const float* __restrict__ src, long long ld, int jb) {
+  if (jb < kNb) {
+    for (int e = threadIdx.x; e < kNb * kNb; e += blockDim.x)
+      if (e % kNb >= jb || e / kNb >= jb) dst[e] = 0.f;
+  }
+  stage_in(dst, kNb, src, ld, jb, jb);
+}
+constexpr size_t kBlockBytes = (size_t)kNb * kNb * sizeof(float);
+
+// B = L^-1 B for a unit lower jb x jb L (column-major at Lp, leading dimension ldl) and the
+// ncols columns of B (jb rows at Bp, leading dimension ldb), or, with identity set, B = L^-1: one
+// warp per column of B, L in shared memory.  Bound by its chain of jb shuffles and FMAs and by the
+// latency of fetching L: 14 us for 384 columns; 24 us with run-time indices into x and an
+// integer division per staged element.
+__global__ void __launch_bounds__(256) k_trsm_unit_lower(const float* Lp, long long ldl, int jb, float* Bp,
+                                                         long long ldb, int ncols, bool identity) {
+  extern __shared__ float L[];   // [jb][kNb]
+  constexpr int NQ = kNb / 32;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x / 32;
+  stage_block(L, Lp, ldl, jb);
+  __syncthreads();
+  for (int cidx = blockIdx.x * nw + warp; cidx < ncols; cidx += gridDim.x * nw) {
+    float* col = Bp + (size_t)cidx * ldb;
+    float x[NQ];
 #pragma unroll
-    for (int q = 0; q < kNb / 32; ++q)
+    for (int q = 0; q < NQ; ++q) {
+      const int m = q * 32 + lane;
+      x[q] = identity ? (m == cidx ? 1.f : 0.f) : m < jb ? col[m] : 0.f;
+    }
+    unit_lower_solve(x, L, jb, identity ? cidx / 32 : 0);
+#pragma unroll
+    for (int q = 0; q < NQ; ++q)
       if (q * 32 + lane < jb) col[q * 32 + lane] = x[q];
   }
 }
 
-// identity into a jb x jb column-major block
-__global__ void k_eye(float* E, int jb) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e < jb * jb) E[e] = (e % jb == e / jb) ? 1.f : 0.f;
+// FP32 products of a 128 x 128 block with 64 columns, 256 threads: thread (tr, tc) of 16 x 16
+// takes rows 4 tr .. + 3 and 64 + 4 tr .. + 3 and columns 4 tc .. + 3, summed in k order in packed
+// pairs of rows.  Every operand is loaded in one go, 24 16-byte loads in flight per thread: with 8
+// single words at a time the kernels spent their time on 12 rounds of memory latency (k_left_gemm
+// 26 us, now 10).
+static_assert(kNb == 128, "blocks of 128");
+constexpr int kProdCols = 64, kProdLd = kNb + 4;
+struct ProdShared {
+  alignas(16) float A[kNb][kNb];              // [k][row]
+  alignas(16) float B[kProdCols][kProdLd];    // [column][k]
+};
+// rows from rlim on and columns from clim on are zero; column k of the block at a + k lda
+__device__ __forceinline__ void prod_load_a(float4 (&v)[16], const float* __restrict__ a, long long lda, int rlim, int clim) {
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const int e = threadIdx.x + 256 * i, k = e >> 5, r = 4 * (e & 31);
+    v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (k < clim && r < rlim) v[i] = __ldcg(reinterpret_cast<const float4*>(a + (size_t)k * lda + r));
+    if (r + 1 >= rlim) v[i].y = 0.f;
+    if (r + 2 >= rlim) v[i].z = 0.f;
+    if (r + 3 >= rlim) v[i].w = 0.f;
+  }
 }
-
-// C[:, j] = L T[:, j] for j < ncols in FP32: L jb x jb (leading dimension jb, jb <= kNb), T
-// jb x ncols (leading dimension jb), C with leading dimension ldc.  L stays in shared memory;
-// T goes through it 64 columns at a time, transposed (k-major, rows padded to 68 floats so
-// the transposing stores spread over the banks).  Thread (tr, tc) of 16 x 16 owns rows
-// 8 tr .. 8 tr + 7 and columns 4 tc .. 4 tc + 3 of the 128 x 64 block: per k two 16-byte
-// loads of L and one of T feed 32 FMAs, summed in k order.
-constexpr int kLeftCols = 64;
-constexpr int kLeftLd = kLeftCols + 4;
-__global__ void __launch_bounds__(256) k_left_gemm(const float* __restrict__ L, int jb, const float* __restrict__ T,
-                                                   int ncols, float* __restrict__ C, long long ldc) {
-  extern __shared__ float4 lsm4[];
-  float* Ls = reinterpret_cast<float*>(lsm4);   // [k][kNb], zero beyond jb
-  float* Ts = Ls + (size_t)kNb * kNb;            // [k][kLeftLd]
-  // staging: 8 loads in flight per thread before their stores (a load -> store loop waits
-  // out the full memory latency at every element)
-  for (int e0 = threadIdx.x; e0 < kNb * kNb; e0 += 8 * blockDim.x) {
-    float v[8];
+__device__ __forceinline__ void prod_load_b(float4 (&v)[8], const float* __restrict__ b, long long ldb, int clim) {
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int e = e0 + q * blockDim.x, kk = e / kNb, r = e % kNb;
-      v[q] = (e < kNb * kNb && kk < jb && r < jb) ? __ldg(L + (size_t)kk * jb + r) : 0.f;
-    }
+  for (int i = 0; i < 8; ++i) {
+    const int e = threadIdx.x + 256 * i, c = e >> 5, k = 4 * (e & 31);
+    v[i] = c < clim ? __ldcg(reinterpret_cast<const float4*>(b + (size_t)c * ldb + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+}
+__device__ __forceinline__ void prod_store_a(ProdShared& sh, const float4 (&v)[16]) {
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int e = e0 + q * blockDim.x;
-      if (e < kNb * kNb) Ls[e] = v[q];
+  for (int i = 0; i < 16; ++i) {
+    const int e = threadIdx.x + 256 * i;
+    *reinterpret_cast<float4*>(&sh.A[e >> 5][4 * (e & 31)]) = v[i];
+  }
+}
+__device__ __forceinline__ void prod_store_b(ProdShared& sh, const float4 (&v)[8]) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int e = threadIdx.x + 256 * i;
+    *reinterpret_cast<float4*>(&sh.B[e >> 5][4 * (e & 31)]) = v[i];
+  }
+}
+// acc[c][2 h + p] += rows (64 h + 4 tr + 2 p, + 1) of column 4 tc + c
+__device__ __forceinline__ void prod_add(float2 (&acc)[4][4], const ProdShared& sh) {
+  const int tr = threadIdx.x & 15, tc = threadIdx.x >> 4;
+#pragma unroll 1
+  for (int k0 = 0; k0 < kNb; k0 += 4) {
+    float4 b[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) b[c] = *reinterpret_cast<const float4*>(&sh.B[4 * tc + c][k0]);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float4 a0 = *reinterpret_cast<const float4*>(&sh.A[k0 + k][4 * tr]);
+      const float4 a1 = *reinterpret_cast<const float4*>(&sh.A[k0 + k][64 + 4 * tr]);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const float bv = k == 0 ? b[c].x : k == 1 ? b[c].y : k == 2 ? b[c].z : b[c].w;
+        const float2 b2 = make_float2(bv, bv);
+        acc[c][0] = __ffma2_rn(make_float2(a0.x, a0.y), b2, acc[c][0]);
+        acc[c][1] = __ffma2_rn(make_float2(a0.z, a0.w), b2, acc[c][1]);
+        acc[c][2] = __ffma2_rn(make_float2(a1.x, a1.y), b2, acc[c][2]);
+        acc[c][3] = __ffma2_rn(make_float2(a1.z, a1.w), b2, acc[c][3]);
+      }
     }
   }
+}
+
+// B = L B in place for ncols columns of kNb rows (16-byte aligned): each block has read its 64
+// columns before it writes them
+__global__ void __launch_bounds__(256) k_left_gemm(const float* __restrict__ L, float* B, long long ldb, int ncols) {
+  extern __shared__ __align__(16) char lgsm[];
+  ProdShared& sh = *reinterpret_cast<ProdShared*>(lgsm);
   const int tr = threadIdx.x & 15, tc = threadIdx.x >> 4;
-  for (int c0 = blockIdx.x * kLeftCols; c0 < ncols; c0 += gridDim.x * kLeftCols) {
-    const int nc = min(kLeftCols, ncols - c0);
+  float4 va[16], vb[8];
+  prod_load_a(va, L, kNb, kNb, kNb);
+  int c0 = blockIdx.x * kProdCols;
+  prod_load_b(vb, B + (size_t)c0 * ldb, ldb, ncols - c0);
+  prod_store_a(sh, va);
+  for (; c0 < ncols; c0 += gridDim.x * kProdCols) {
+    prod_store_b(sh, vb);
     __syncthreads();
-    for (int e0 = threadIdx.x; e0 < kLeftCols * jb; e0 += 8 * blockDim.x) {
-      float v[8];
+    const int next = c0 + gridDim.x * kProdCols;
+    if (next < ncols) prod_load_b(vb, B + (size_t)next * ldb, ldb, ncols - next);
+    float2 acc[4][4];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int e = e0 + q * blockDim.x, c = e / jb, kk = e % jb;
-        v[q] = (e < kLeftCols * jb && c < nc) ? __ldg(T + (size_t)(c0 + c) * jb + kk) : 0.f;
-      }
+    for (int c = 0; c < 4; ++c)
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int e = e0 + q * blockDim.x, c = e / jb, kk = e % jb;
-        if (e < kLeftCols * jb) Ts[(size_t)kk * kLeftLd + c] = v[q];
-      }
-    }
-    __syncthreads();
-    float acc[8][4];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) acc[i][c] = 0.f;
-#pragma unroll 4
-    for (int kk = 0; kk < jb; ++kk) {
-      const float4 a0 = *reinterpret_cast<const float4*>(Ls + (size_t)kk * kNb + 8 * tr);
-      const float4 a1 = *reinterpret_cast<const float4*>(Ls + (size_t)kk * kNb + 8 * tr + 4);
-      const float4 b = *reinterpret_cast<const float4*>(Ts + (size_t)kk * kLeftLd + 4 * tc);
-      const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-      const float bv[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) acc[i][c] = fmaf(av[i], bv[c], acc[i][c]);
-    }
+      for (int r = 0; r < 4; ++r) acc[c][r] = make_float2(0.f, 0.f);
+    prod_add(acc, sh);
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-      const int col = 4 * tc + c;
-      if (col < nc)
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-          if (8 * tr + i < jb) C[(size_t)(c0 + col) * ldc + 8 * tr + i] = acc[i][c];
+      const int col = c0 + 4 * tc + c;
+      if (col >= ncols) break;
+      float* o = B + (size_t)col * ldb + 4 * tr;
+      *reinterpret_cast<float4*>(o) = make_float4(acc[c][0].x, acc[c][0].y, acc[c][1].x, acc[c][1].y);
+      *reinterpret_cast<float4*>(o + 64) = make_float4(acc[c][2].x, acc[c][2].y, acc[c][3].x, acc[c][3].y);
     }
+    __syncthreads();
   }
 }
 
@@ -1202,137 +1272,101 @@ __global__ void k_permute_to_float(const double* r, const int* perm, float* y, i
 constexpr int kDb = 512;
 constexpr int kDbSub = kDb / kNb;
 __host__ __device__ inline size_t dinv_floats(int n) { return (size_t)((n + kDb - 1) / kDb) * 2 * kDb * kDb; }
+// blockIdx.y: lower and upper; blockIdx.z: every kInvSplit-th column
+constexpr int kInvSplit = 4;
 __global__ void __launch_bounds__(256) k_diag_inverses(const float* __restrict__ LU, long long ld, int n,
                                                        float* __restrict__ dinv) {
-  extern __shared__ float D[];   // [jb][jb] diagonal block
+  extern __shared__ float D[];   // [jb][kNb] diagonal block
+  constexpr int NQ = kNb / 32;
   const int kb = blockIdx.x, k0 = kb * kNb, jb = min(kNb, n - k0);
-  stage_in(D, jb, LU + (size_t)k0 * ld + k0, ld, jb, jb);
+  const bool lower = blockIdx.y == 0;
+  stage_block(D, LU + (size_t)k0 * ld + k0, ld, jb);
   __syncthreads();
-  float* Li = dinv + (size_t)(kb / kDbSub) * 2 * kDb * kDb + (size_t)(kb % kDbSub) * kNb * (kDb + 1);
-  float* Ui = Li + (size_t)kDb * kDb;
+  float* X = dinv + (size_t)(kb / kDbSub) * 2 * kDb * kDb + (size_t)(kb % kDbSub) * kNb * (kDb + 1) +
+             (lower ? 0 : (size_t)kDb * kDb);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int c = warp; c < jb; c += blockDim.x / 32) {
-    float x[kNb / 32];
-    // L x = e_c
+  for (int c = warp * kInvSplit + blockIdx.z; c < jb; c += blockDim.x / 32 * kInvSplit) {
+    float x[NQ];
 #pragma unroll
-    for (int q = 0; q < kNb / 32; ++q) x[q] = (q * 32 + lane == c) ? 1.f : 0.f;
-    for (int i = c; i < jb; ++i) {
-      const float xi = __shfl_sync(0xffffffffu, x[i >> 5], i & 31);
+    for (int q = 0; q < NQ; ++q) x[q] = (q * 32 + lane == c) ? 1.f : 0.f;
+    if (lower) {
+      unit_lower_solve(x, D, jb, c / 32);
+    } else {
+      // U x = e_c, from row c up
 #pragma unroll
-      for (int q = 0; q < kNb / 32; ++q) {
-        const int m = q * 32 + lane;
-        if (m > i && m < jb) x[q] = fmaf(-D[(size_t)i * jb + m], xi, x[q]);
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < kNb / 32; ++q) {
-      const int m = q * 32 + lane;
-      if (m < kNb) Li[(size_t)c * kDb + m] = m < jb ? x[q] : 0.f;
-    }
-    // U x = e_c
-#pragma unroll
-    for (int q = 0; q < kNb / 32; ++q) x[q] = (q * 32 + lane == c) ? 1.f : 0.f;
-    for (int i = c; i >= 0; --i) {
-      if ((i & 31) == lane) x[i >> 5] = x[i >> 5] / D[(size_t)i * jb + i];
-      const float xi = __shfl_sync(0xffffffffu, x[i >> 5], i & 31);
-#pragma unroll
-      for (int q = 0; q < kNb / 32; ++q) {
-        const int m = q * 32 + lane;
-        if (m < i) x[q] = fmaf(-D[(size_t)i * jb + m], xi, x[q]);
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < kNb / 32; ++q) {
-      const int m = q * 32 + lane;
-      if (m < kNb) Ui[(size_t)c * kDb + m] = m < jb ? x[q] : 0.f;
-    }
-  }
-}
-
-// acc (8 x 8 of a 128 x 128 product per thread, 256 threads as 16 x 16) += A B over k < 128:
-// A(r, k) at a + k lda + r (rows < ar, columns < ac; zero beyond), B from b(k, c)
-template <class BLoad>
-__device__ __forceinline__ void merge_gemm(float (*acc)[8], const float* __restrict__ a, long long lda, int ar, int ac,
-                                           const BLoad& b, float (*As)[kNb + 4], float (*Bs)[kNb + 4]) {
-  const int tid = threadIdx.x, tr = tid & 15, tc = tid >> 4;
-  for (int k0 = 0; k0 < kNb; k0 += 16) {
-    float va[8], vb[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int e = tid + 256 * q;
-      const int r = e % kNb, ka = k0 + e / kNb;
-      va[q] = r < ar && ka < ac ? a[(size_t)ka * lda + r] : 0.f;
-      vb[q] = b(k0 + e % 16, e / 16);
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int e = tid + 256 * q;
-      As[e / kNb][e % kNb] = va[q];
-      Bs[e % 16][e / 16] = vb[q];
-    }
-    __syncthreads();
+      for (int b = NQ - 1; b >= 0; --b) {
+        if (b > c / 32) continue;
 #pragma unroll 4
-    for (int kk = 0; kk < 16; ++kk) {
-      float x[8], y[8];
+        for (int il = 31; il >= 0; --il) {
+          const int i = 32 * b + il;
+          if (i > c) continue;
+          const float* col = D + (size_t)i * kNb + lane;
+          if (il == lane) x[b] = x[b] / col[32 * b];
+          const float xi = __shfl_sync(0xffffffffu, x[b], il);
+          x[b] = fmaf(lane < il ? -col[32 * b] : 0.f, xi, x[b]);
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        x[q] = As[kk][tr + 16 * q];
-        y[q] = Bs[kk][tc + 16 * q];
+          for (int q = 0; q < b; ++q) x[q] = fmaf(-col[32 * q], xi, x[q]);
+        }
       }
+    }
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int q = 0; q < 8; ++q) acc[i][q] = fmaf(x[i], y[q], acc[i][q]);
+    for (int q = 0; q < NQ; ++q) {
+      const int m = q * 32 + lane;
+      X[(size_t)c * kDb + m] = m < jb ? x[q] : 0.f;
     }
   }
-  __syncthreads();
 }
 
 // The kNb x kNb blocks at distance d from the diagonal of every kDb block's inverses (d = 1, 2,
 // ... in turn): X_ij = -X_ii sum_{j <= k < i} L_ik X_kj, and for the upper factor
-// Y_ij = -Y_ii sum_{i < k <= j} U_ik Y_kj.  One block each; blockIdx.y: lower, upper.
-struct MergeShared {
-  float As[16][kNb + 4], Bs[16][kNb + 4];
-  float T[kNb][kNb + 1];   // [column][row]
-};
+// Y_ij = -Y_ii sum_{i < k <= j} U_ik Y_kj.  blockIdx.y: lower, upper; blockIdx.z: half of the columns.
 __global__ void __launch_bounds__(256) k_diag_merge(const float* __restrict__ LU, long long ld, int n, float* dinv,
                                                     int d) {
   extern __shared__ __align__(16) char mgsm[];
-  MergeShared& sh = *reinterpret_cast<MergeShared*>(mgsm);
+  ProdShared& sh = *reinterpret_cast<ProdShared*>(mgsm);
   const int per = kDbSub - d, b = blockIdx.x / per, t = blockIdx.x % per;
   const bool lower = blockIdx.y == 0;
   const int i = lower ? t + d : t, j = lower ? t : t + d;
   const int o = b * kDb;                                   // first row and column of the kDb block
   if (o + kNb * max(i, j) >= n) return;
   float* X = dinv + (size_t)b * 2 * kDb * kDb + (lower ? 0 : (size_t)kDb * kDb);
-  const int tid = threadIdx.x, tr = tid & 15, tc = tid >> 4;
-  float acc[8][8];
+  float* Xj = X + (size_t)(kNb * j + kProdCols * blockIdx.z) * kDb;   // this block's columns
+  const int tr = threadIdx.x & 15, tc = threadIdx.x >> 4;
+  float2 acc[4][4];
 #pragma unroll
-  for (int e = 0; e < 8; ++e)
+  for (int c = 0; c < 4; ++c)
 #pragma unroll
-    for (int q = 0; q < 8; ++q) acc[e][q] = 0.f;
-  const int ar = min(kNb, n - (o + kNb * i));
+    for (int r = 0; r < 4; ++r) acc[c][r] = make_float2(0.f, 0.f);
+  float4 va[16], vb[8];
   for (int k = lower ? j : i + 1; k <= (lower ? i - 1 : j); ++k) {
-    const float* xb = X + (size_t)kNb * j * kDb + kNb * k;
-    merge_gemm(acc, LU + (size_t)(o + kNb * k) * ld + o + kNb * i, ld, ar, min(kNb, n - (o + kNb * k)),
-               [&](int kk, int c) { return xb[(size_t)c * kDb + kk]; }, sh.As, sh.Bs);
+    prod_load_a(va, LU + (size_t)(o + kNb * k) * ld + o + kNb * i, ld, n - (o + kNb * i), n - (o + kNb * k));
+    prod_load_b(vb, Xj + kNb * k, kDb, kProdCols);
+    __syncthreads();
+    prod_store_a(sh, va);
+    prod_store_b(sh, vb);
+    __syncthreads();
+    prod_add(acc, sh);
   }
+  // (columns of X_ii beyond the matrix hold nothing)
+  prod_load_a(va, X + (size_t)kNb * i * (kDb + 1), kDb, kNb, n - (o + kNb * i));
+  __syncthreads();
+  prod_store_a(sh, va);
 #pragma unroll
-  for (int e = 0; e < 8; ++e)
+  for (int c = 0; c < 4; ++c)
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      sh.T[tc + 16 * q][tr + 16 * e] = acc[e][q];
-      acc[e][q] = 0.f;
+    for (int h = 0; h < 2; ++h) {
+      *reinterpret_cast<float4*>(&sh.B[4 * tc + c][64 * h + 4 * tr]) =
+          make_float4(acc[c][2 * h].x, acc[c][2 * h].y, acc[c][2 * h + 1].x, acc[c][2 * h + 1].y);
+      acc[c][2 * h] = acc[c][2 * h + 1] = make_float2(0.f, 0.f);
     }
   __syncthreads();
-  merge_gemm(acc, X + (size_t)kNb * i * (kDb + 1), kDb, kNb, kNb, [&](int kk, int c) { return sh.T[c][kk]; }, sh.As,
-             sh.Bs);
-  float* out = X + (size_t)kNb * j * kDb + kNb * i;
+  prod_add(acc, sh);
 #pragma unroll
-  for (int e = 0; e < 8; ++e)
+  for (int c = 0; c < 4; ++c)
 #pragma unroll
-    for (int q = 0; q < 8; ++q) out[(size_t)(tc + 16 * q) * kDb + tr + 16 * e] = -acc[e][q];
+    for (int h = 0; h < 2; ++h)
+      *reinterpret_cast<float4*>(Xj + (size_t)(4 * tc + c) * kDb + kNb * i + 64 * h + 4 * tr) =
+          make_float4(-acc[c][2 * h].x, -acc[c][2 * h].y, -acc[c][2 * h + 1].x, -acc[c][2 * h + 1].y);
 }
 
 struct TrsvArgs {
@@ -1784,7 +1818,7 @@ extern "C" int32_t o3g_bem_factor(o3g_bem_t* h, void* stream) {
     return O3G_ERR_INVALID_ARG;
   }
   const size_t cand = align_up((2 * (size_t)G + 2 * (size_t)G * kNb + 2 * (size_t)kNb) * sizeof(unsigned long long));
-  O3G_TRY(bem_scratch(h, cand + align_up((size_t)kNb * kNb * 4) + align_up((size_t)kNb * n * 4) + (1 << 20)));
+  O3G_TRY(bem_scratch(h, cand + align_up((size_t)kNb * kNb * 4) + align_up(2 * (size_t)kNbOuter * 8) + (1 << 20)));
   Carve cv(h->scratch);
   // keys and tagged rows back to back, zeroed together once per factorisation
   const size_t xwords = 2 * (size_t)G + 2 * (size_t)G * kNb + 2 * (size_t)kNb;
@@ -1797,8 +1831,7 @@ extern "C" int32_t o3g_bem_factor(o3g_bem_t* h, void* stream) {
                                  cudaMemcpyDeviceToDevice, st));
   KernelTimer& tm = thread_timer();
   tm.begin(st);
-  const size_t tsm = (size_t)kNb * kNb * sizeof(float);
-  O3G_CUDA_TRY(cudaFuncSetAttribute(k_trsm_unit_lower, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm));
+  O3G_CUDA_TRY(cudaFuncSetAttribute(k_trsm_unit_lower, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBlockBytes));
   O3G_CUDA_TRY(cudaFuncSetAttribute(k_laswp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)laswp_smem(kNbOuter)));
   // C = C - A B on the tensor cores (o3g_tcgemm.cu: tcgen05, TF32 products, FP32 sums; all
   // operands column-major in LU); the error word of its pipeline waits is flags[4]
@@ -1818,35 +1851,32 @@ extern "C" int32_t o3g_bem_factor(o3g_bem_t* h, void* stream) {
     if (ncols <= 0) return;
     int tb = (ncols + 7) / 8;
     if (tb > 4 * df.num_sms) tb = 4 * df.num_sms;
-    k_trsm_unit_lower<<<tb, 256, (size_t)jb * jb * sizeof(float), st>>>(h->LU + (size_t)k0 * ld + k0, ld, jb,
-                                                                         h->LU + (size_t)c0 * ld + k0, ld, ncols);
+    k_trsm_unit_lower<<<tb, 256, kBlockBytes, st>>>(h->LU + (size_t)k0 * ld + k0, ld, jb, h->LU + (size_t)c0 * ld + k0,
+                                                    ld, ncols, false);
     note_launch();
   };
-  // the same solve for a wide right-hand side: Linv = L11^-1 once (TRSM on the identity),
-  // then B <- Linv B as an FP32 product (k_left_gemm) through a scratch copy
+  // the same solve for a wide right-hand side (whole blocks): Linv = L11^-1 once, then B <- Linv B
+  // as an FP32 product
   float* linv = cv.take<float>((size_t)kNb * kNb);
-  const size_t lsm_bytes = ((size_t)kNb * kNb + (size_t)kNb * kLeftLd) * sizeof(float);
-  O3G_CUDA_TRY(cudaFuncSetAttribute(k_left_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lsm_bytes));
-  float* tmp = cv.take<float>((size_t)kNb * n);
-  auto trsm_wide = [&](int k0, int jb, int c0, int ncols) -> int32_t {
-    if (ncols <= 0) return O3G_OK;
-    k_eye<<<(jb * jb + 255) / 256, 256, 0, st>>>(linv, jb);
-    k_trsm_unit_lower<<<(jb + 7) / 8, 256, (size_t)jb * jb * sizeof(float), st>>>(h->LU + (size_t)k0 * ld + k0, ld,
-                                                                                 jb, linv, jb, jb);
+  O3G_CUDA_TRY(cudaFuncSetAttribute(k_left_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ProdShared)));
+  auto trsm_wide = [&](int k0, int c0, int ncols) {
+    k_trsm_unit_lower<<<kNb / 8, 256, kBlockBytes, st>>>(h->LU + (size_t)k0 * ld + k0, ld, kNb, linv, kNb, kNb, true);
+    const int lb = std::min((ncols + kProdCols - 1) / kProdCols, 2 * df.num_sms);
+    k_left_gemm<<<lb, 256, sizeof(ProdShared), st>>>(linv, h->LU + (size_t)c0 * ld + k0, ld, ncols);
     note_launch(2);
-    float* B = h->LU + (size_t)c0 * ld + k0;
-    O3G_CUDA_TRY(cudaMemcpy2DAsync(tmp, (size_t)jb * sizeof(float), B, ld * sizeof(float), (size_t)jb * sizeof(float),
-                                   ncols, cudaMemcpyDeviceToDevice, st));
-    const int lb = std::min((ncols + kLeftCols - 1) / kLeftCols, 2 * df.num_sms);
-    k_left_gemm<<<lb, 256, lsm_bytes, st>>>(linv, jb, tmp, ncols, B, ld);
-    note_launch();
-    return O3G_OK;
   };
+  int2* rowmap = cv.take<int2>(2 * (size_t)kNbOuter);
   auto laswp = [&](int p0, int p1, int c0, int c1, int s0, int s1) {
     const int cnt = (c1 - c0) - (s1 > s0 ? s1 - s0 : 0);
     if (cnt <= 0) return;
     const int lb = std::min((cnt + 7) / 8, 8 * df.num_sms);
-    k_laswp<<<lb, 256, laswp_smem(p1 - p0), st>>>(h->LU, ld, n, p0, p1, h->piv, c0, c1, s0, s1);
+    const bool shared_map = p1 - p0 > kSwapInline;
+    if (shared_map) {
+      k_row_map<<<(2 * (p1 - p0) + 127) / 128, 128, (size_t)(p1 - p0) * sizeof(int), st>>>(h->piv, p0, p1 - p0, n, rowmap);
+      note_launch();
+    }
+    k_laswp<<<lb, 256, laswp_smem(p1 - p0), st>>>(h->LU, ld, n, p0, p1, h->piv, shared_map ? rowmap : nullptr, c0, c1, s0,
+                                                  s1);
     note_launch();
   };
   auto at = [&](int r, int c) { return h->LU + (size_t)c * ld + r; };
@@ -1907,21 +1937,19 @@ extern "C" int32_t o3g_bem_factor(o3g_bem_t* h, void* stream) {
     if (K1 < n) {
       // U12 = L11^-1 A12 for the KB x KB unit lower L11, block by block
       for (int k0 = K0; k0 < K1; k0 += kNb) {
-        const int jb = std::min(kNb, K1 - k0);
-        O3G_TRY(trsm_wide(k0, jb, K1, n - K1));
-        if (k0 + jb < K1) O3G_TRY(gemm(K1 - k0 - jb, n - K1, jb, at(k0 + jb, k0), at(k0, K1), at(k0 + jb, K1)));
+        trsm_wide(k0, K1, n - K1);   // (K1 < n: the outer panel is whole blocks)
+        if (k0 + kNb < K1) O3G_TRY(gemm(K1 - k0 - kNb, n - K1, kNb, at(k0 + kNb, k0), at(k0, K1), at(k0 + kNb, K1)));
       }
       O3G_TRY(gemm(n - K1, n - K1, KB, at(K1, K0), at(K0, K1), at(K1, K1)));
     }
   }
   {
-    const size_t dsm = (size_t)kNb * kNb * sizeof(float);
-    O3G_CUDA_TRY(cudaFuncSetAttribute(k_diag_inverses, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsm));
-    k_diag_inverses<<<(n + kNb - 1) / kNb, 256, dsm, st>>>(h->LU, ld, n, h->dinv);
-    O3G_CUDA_TRY(cudaFuncSetAttribute(k_diag_merge, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MergeShared)));
+    O3G_CUDA_TRY(cudaFuncSetAttribute(k_diag_inverses, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBlockBytes));
+    k_diag_inverses<<<dim3((n + kNb - 1) / kNb, 2, kInvSplit), 256, kBlockBytes, st>>>(h->LU, ld, n, h->dinv);
+    O3G_CUDA_TRY(cudaFuncSetAttribute(k_diag_merge, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ProdShared)));
     const int nbig = (n + kDb - 1) / kDb;
     for (int d = 1; d < kDbSub && n > d * kNb; ++d)
-      k_diag_merge<<<dim3(nbig * (kDbSub - d), 2), 256, sizeof(MergeShared), st>>>(h->LU, ld, n, h->dinv, d);
+      k_diag_merge<<<dim3(nbig * (kDbSub - d), 2, kNb / kProdCols), 256, sizeof(ProdShared), st>>>(h->LU, ld, n, h->dinv, d);
     note_launch(kDbSub);
   }
   tm.end(st);
