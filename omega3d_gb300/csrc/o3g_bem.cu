@@ -1386,7 +1386,7 @@ struct TrsvArgs {
 // depend on.  kDb 512: 128 columns a step, every block applying the whole 128 x 128 inverse for
 // itself, took 8-10 us a step; 1024 would double the memory of the inverses (n kDb 8 bytes) to
 // save a few barriers.  A whole solve with 3 refinements, before and after: n = 640 0.44 -> 0.36
-// ms, 2,560 0.99 -> 0.56, 10,240 5.41 -> 1.59, 15,360 8.12 -> 2.56; the inverses cost 0.1 ms per factorisation.
+// ms, 2,560 0.99 -> 0.56, 10,240 5.41 -> 1.59, 15,360 8.12 -> 2.56; the inverses cost 0.2 ms per factorisation.
 constexpr int kTrRows = 64, kTrChunks = kSolveThreads / kTrRows, kTrCols = kDb / kTrChunks;
 constexpr size_t trsv_smem(int K) { return (size_t)K * (kDb + kSolveThreads) * sizeof(float); }
 template <int K, bool LOWER>

@@ -287,153 +287,183 @@ __global__ void __launch_bounds__(kCB) k_coeff(const SrcRec* __restrict__ srec, 
   }
 }
 
-// One warp per listed pair (maxlev <= 3): the subdivision tree is expanded level by level.
-// Level 1 has 16 child pairs (source child a outer, target child b inner, one lane each);
-// every child pair that is neither well separated nor at maxlev contributes 16 pairs to the
-// next level, kept in a per-warp list in shared memory in enumeration order.  Leaves are
-// summed per lane and reduced across the warp in a fixed order.
-//
-// A pair at level L needs only the centroids of one level-L sub-triangle of each panel,
-// and every pair of a level shares them: the warp builds the 4^L sub-triangles of both
-// panels once per level (each from its stored parent by child(), the same operations as a
-// descent from the root) and keeps their centroids in shared memory, indexed by the
-// path (2 bits per level, level 1 in the low bits).  A pair then costs six shared loads,
-// the distance test and the leaf.
+// The listed pairs (maxlev <= 3).  A node is a pair of sub-triangles of one level that is split: its 16
+// child pairs (4 x 4 centroids of the next level) are either leaves or nodes themselves.  Every
+// leaf of a pair has the same strengths up to 1 / 16 per level, so u_k = s_k x w (and q w for the
+// source) with one vector sum w = sum f r3 d over all leaves: a leaf costs 12 operations, half
+// as many issue slots in packed FP32, instead of the 30 that form the cross products of each.
+// One lane takes a whole node: 8 centroids from k_pack_centroids' table, 16 pairs.  A warp takes 32
+// listed pairs: first every lane its own pair's level 1; then pair by pair those with close children
+// (a third), their nodes spread over the lanes; w is reduced per pair in a fixed order and
+// each lane projects and writes its own pair.  Measured (one GB300), 20,480 panels, 4.0 million
+// pairs, 317 leaves or nodes each: 6.41 -> 2.03 ms (54 % of the issue slots); it was one warp per pair from the start, with both
+// panels' sub-triangles built for each.
 constexpr int kNearWarps = 4;
-struct NearShared {
-  float tri[2][20][9];   // [source, target][level 1: 0..3, level 2: 4..19] sub-triangles
-  float cen[2][84][3];   // [source, target][level 1: 0..3, level 2: 4..19, level 3: 20..83]
-};
+constexpr int kCenRow = 84;   // centroids per panel: 4 of level 1, 16 of level 2, 64 of level 3, children together
+struct NearSum { float x, y, z; };
 
-__device__ __forceinline__ void store_tri(float* d, const TriG& t) {
-  d[0] = t.x0; d[1] = t.y0; d[2] = t.z0; d[3] = t.x1; d[4] = t.y1; d[5] = t.z1; d[6] = t.x2; d[7] = t.y2; d[8] = t.z2;
-}
-__device__ __forceinline__ TriG load_tri(const float* d) {
-  return TriG{d[0], d[1], d[2], d[3], d[4], d[5], d[6], d[7], d[8]};
-}
-__device__ __forceinline__ void store_cen(float* d, const TriG& t) {
-  float cx, cy, cz;
-  cen(t, cx, cy, cz);
-  d[0] = cx; d[1] = cy; d[2] = cz;
-}
-
-// the level-lev sub-triangles of both panels (and their centroids) into sh; lev 1..3
-__device__ __forceinline__ void build_level(NearShared& sh, const TriG& S0, const TriG& T0, int lev, int lane) {
-  if (lev == 1) {
-    if (lane < 8) {
-      const int side = lane >> 2, c = lane & 3;
-      const TriG t = child(side ? T0 : S0, c);
-      store_tri(sh.tri[side][c], t);
-      store_cen(sh.cen[side][c], t);
-    }
-  } else if (lev == 2) {
-    // path p = (level-2 child << 2) | level-1 child
-    const int side = lane >> 4, p = lane & 15;
-    const TriG t = child(load_tri(sh.tri[side][p & 3]), p >> 2);
-    store_tri(sh.tri[side][4 + p], t);
-    store_cen(sh.cen[side][4 + p], t);
-  } else {
-#pragma unroll 1
-    for (int e = lane; e < 128; e += 32) {
-      const int side = e >> 6, p = e & 63;
-      store_cen(sh.cen[side][20 + p], child(load_tri(sh.tri[side][4 + (p & 15)]), p >> 4));
-    }
+// Adds f times the leaves' r3 d of the node with source centroids s[0..3] and target centroids t[0..3]
+// to w.  TEST: returns the pairs (bit 4 a + b) that are not well separated, which are left out;
+// otherwise every pair is a leaf.
+template <bool TEST>
+__device__ __forceinline__ unsigned near_node(const float4* __restrict__ s, const float4* __restrict__ t, float thr, float f,
+                                              NearSum& w) {
+  float2 tx[2], ty[2], tz[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const float4 p = __ldg(t + 2 * h), q = __ldg(t + 2 * h + 1);
+    tx[h] = make_float2(p.x, q.x);
+    ty[h] = make_float2(p.y, q.y);
+    tz[h] = make_float2(p.z, q.z);
   }
-  __syncwarp();
+  float4 sc[4];
+#pragma unroll
+  for (int a = 0; a < 4; ++a) sc[a] = __ldg(s + a);
+  // as farther_rn
+  const float thr2 = __fmul_rn(thr, thr);
+  const float above = __fmul_rn(thr2, 1.00000095367431640625f), below = __fmul_rn(thr2, 0.99999904632568359375f);
+  auto is_near = [&](float d2) {
+    if (d2 > above) return false;
+    if (d2 < below) return true;
+    return !(__fsqrt_rn(d2) > thr);
+  };
+  float2 wx = make_float2(0.f, 0.f), wy = wx, wz = wx;
+  unsigned mask = 0u;
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const float2 dx = __fadd2_rn(tx[h], make_float2(-sc[a].x, -sc[a].x));
+      const float2 dy = __fadd2_rn(ty[h], make_float2(-sc[a].y, -sc[a].y));
+      const float2 dz = __fadd2_rn(tz[h], make_float2(-sc[a].z, -sc[a].z));
+      const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
+      const float2 rs = make_float2(rsq_hw(r2.x), rsq_hw(r2.y));
+      float2 r3 = __fmul2_rn(__fmul2_rn(rs, rs), rs);
+      if (TEST) {
+        const float2 d2 = __fadd2_rn(__fadd2_rn(__fmul2_rn(dx, dx), __fmul2_rn(dy, dy)), __fmul2_rn(dz, dz));
+        const bool n0 = is_near(d2.x), n1 = is_near(d2.y);
+        if (n0) { r3.x = 0.f; mask |= 1u << (4 * a + 2 * h); }
+        if (n1) { r3.y = 0.f; mask |= 1u << (4 * a + 2 * h + 1); }
+      }
+      wx = __ffma2_rn(r3, dx, wx);
+      wy = __ffma2_rn(r3, dy, wy);
+      wz = __ffma2_rn(r3, dz, wz);
+    }
+  w.x = fmaf(f, wx.x + wx.y, w.x);
+  w.y = fmaf(f, wy.x + wy.y, w.y);
+  w.z = fmaf(f, wz.x + wz.y, w.z);
+  return mask;
 }
 
 template <int NUNK>
-__global__ void __launch_bounds__(32 * kNearWarps) k_coeff_near(const SrcRec* __restrict__ srec,
-                                                               const TriG* __restrict__ stri,
-                                                               const TriG* __restrict__ ttri,
-                                                               const float* __restrict__ tarea,
-                                                               const float* __restrict__ t1x,
-                                                               const float* __restrict__ t1y,
-                                                               const float* __restrict__ t1z,
-                                                               const float* __restrict__ t2x,
-                                                               const float* __restrict__ t2y,
-                                                               const float* __restrict__ t2z,
-                                                               const float* __restrict__ tnx,
-                                                               const float* __restrict__ tny,
-                                                               const float* __restrict__ tnz, int maxlev,
-                                                               float* __restrict__ coeff, long long ld, NearList nl) {
-  __shared__ unsigned lst[kNearWarps][2][256];
-  __shared__ NearShared shw[kNearWarps];
+__global__ void __launch_bounds__(32 * kNearWarps) k_coeff_near(
+    const SrcRec* __restrict__ srec, const float4* __restrict__ scen, const float4* __restrict__ tcen,
+    const float* __restrict__ tarea, const float* __restrict__ t1x, const float* __restrict__ t1y,
+    const float* __restrict__ t1z, const float* __restrict__ t2x, const float* __restrict__ t2y,
+    const float* __restrict__ t2z, const float* __restrict__ tnx, const float* __restrict__ tny,
+    const float* __restrict__ tnz, int maxlev, float* __restrict__ coeff, long long ld, NearList nl) {
+  constexpr unsigned full = 0xffffffffu;
+  // nodes of levels 1 and 2: (source sub-triangle, target sub-triangle << 8)
+  __shared__ unsigned short lst1[kNearWarps][16], lst2[kNearWarps][256];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  NearShared& sh = shw[warp];
   const unsigned total = min(*nl.count, nl.cap);
   const float fac = (float)(1.0 / (4.0 * 3.14159265358979323846));
-  for (unsigned p = blockIdx.x * kNearWarps + warp; p < total; p += gridDim.x * kNearWarps) {
-    const uint2 ij = nl.pairs[p];
+  for (unsigned p0 = (blockIdx.x * kNearWarps + warp) * 32u; p0 < total; p0 += gridDim.x * kNearWarps * 32u) {
+    const bool act = p0 + lane < total;
+    const uint2 ij = nl.pairs[act ? p0 + lane : p0];
     const int i = (int)ij.x, j = (int)ij.y;
-    const SrcRec s = srec[j];
-    const TriG S0 = stri[j], T0 = ttri[i];
-    const float sa = s.s1.w, ta = tarea[i];
     // the level-lev threshold is thr0 0.5^lev exactly (as in pair_subdivide)
-    const float thr0 = __fmul_rn(__fadd_rn(__fsqrt_rn(sa), __fsqrt_rn(ta)), 4.0f);
-    float u[3][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
-    // level L items: (parent index in the level L-1 list, child 0..15); codes keep the
-    // source path in bits 0..7 and the target path in bits 8..15 (2 bits per level)
-    int nparent = 1;
-    for (int lev = 1; lev <= maxlev; ++lev) {
-      build_level(sh, S0, T0, lev, lane);
-      const int nitems = nparent * 16;
-      const int cur = lev & 1, prev = cur ^ 1;
-      int nnext = 0;
-      const float f4 = __int_as_float((127 - 2 * lev) << 23);
-      const float f = f4 * f4;   // 0.0625^lev (Kernels.h:1275-1278)
-      const float thr = __fmul_rn(thr0, __int_as_float((127 - lev) << 23));
-      const float thr2 = __fmul_rn(thr, thr);
-      const int off = lev == 1 ? 0 : (lev == 2 ? 4 : 20);   // first centroid of the level
-      for (int base = 0; base < nitems; base += 32) {
-        const int k = base + lane;
-        bool expand = false;
-        unsigned code = 0;
-        if (k < nitems) {
-          const unsigned pc = lev == 1 ? 0u : lst[warp][prev][k >> 4];
-          const unsigned a = (unsigned)((k & 15) >> 2), b = (unsigned)(k & 3);
-          const unsigned sp = (pc & 0xffu) | (a << (2 * (lev - 1)));
-          const unsigned tp = ((pc >> 8) & 0xffu) | (b << (2 * (lev - 1)));
-          code = sp | (tp << 8);
-          const float* sc = sh.cen[0][off + sp];
-          const float* tc = sh.cen[1][off + tp];
-          const float scx = sc[0], scy = sc[1], scz = sc[2];
-          const float tcx = tc[0], tcy = tc[1], tcz = tc[2];
-          if (lev >= maxlev || farther_rn(tcx, tcy, tcz, scx, scy, scz, thr, thr2)) {
-            leaf3<NUNK>(tcx, tcy, tcz, scx, scy, scz, s.s1.x * f, s.s1.y * f, s.s1.z * f, s.s2.x * f, s.s2.y * f,
-                        s.s2.z * f, s.s1.w * f, u);
-          } else {
-            expand = true;
-          }
-        }
-        const unsigned m = __ballot_sync(0xffffffffu, expand);
-        if (expand) lst[warp][cur][nnext + __popc(m & ((1u << lane) - 1u))] = code;
-        nnext += __popc(m);
+    const float thr0 = __fmul_rn(__fadd_rn(__fsqrt_rn(srec[j].s1.w), __fsqrt_rn(tarea[i])), 4.0f);
+    NearSum w{0.f, 0.f, 0.f};
+    const float4* S = scen + (size_t)j * kCenRow;
+    const float4* T = tcen + (size_t)i * kCenRow;
+    // leaves of level lev carry 0.0625^lev of the strengths (Kernels.h:1275-1278)
+    unsigned mask = 0u;
+    if (maxlev > 1) mask = near_node<true>(S, T, 0.5f * thr0, 0.0625f, w);
+    else            near_node<false>(S, T, 0.f, 0.0625f, w);
+    for (unsigned todo = __ballot_sync(full, act && mask != 0u); todo; todo &= todo - 1u) {
+      const int o = __ffs(todo) - 1;
+      const unsigned om = __shfl_sync(full, mask, o);
+      const float othr = __shfl_sync(full, thr0, o);
+      const float4* OS = scen + (size_t)__shfl_sync(full, j, o) * kCenRow;
+      const float4* OT = tcen + (size_t)__shfl_sync(full, i, o) * kCenRow;
+      if (lane < 16 && (om >> lane) & 1u)
+        lst1[warp][__popc(om & ((1u << lane) - 1u))] = (unsigned short)((lane >> 2) | ((lane & 3) << 8));
+      __syncwarp();
+      const int n1 = __popc(om);
+      NearSum v{0.f, 0.f, 0.f};
+      unsigned m = 0u, sid = 0u, tid = 0u;
+      if (lane < n1) {
+        const unsigned c = lst1[warp][lane];
+        sid = c & 0xffu;
+        tid = c >> 8;
+        if (maxlev > 2) m = near_node<true>(OS + 4 + 4 * sid, OT + 4 + 4 * tid, 0.25f * othr, 0.00390625f, v);
+        else            near_node<false>(OS + 4 + 4 * sid, OT + 4 + 4 * tid, 0.f, 0.00390625f, v);
+      }
+      // the close pairs of level 2 in order
+      int at = __popc(m);
+#pragma unroll
+      for (int d = 1; d < 16; d <<= 1) {
+        const int up = __shfl_up_sync(full, at, d);
+        if (lane >= d) at += up;
+      }
+      const int n2 = __shfl_sync(full, at, 15);
+      at -= __popc(m);
+      for (; m; m &= m - 1u) {
+        const unsigned k = (unsigned)__ffs(m) - 1u;
+        lst2[warp][at++] = (unsigned short)((4u * sid + (k >> 2)) | ((4u * tid + (k & 3u)) << 8));
       }
       __syncwarp();
-      nparent = nnext;
-      if (nparent == 0) break;
+      for (int e = lane; e < n2; e += 32) {
+        const unsigned c = lst2[warp][e];
+        near_node<false>(OS + 20 + 4 * (c & 0xffu), OT + 20 + 4 * (c >> 8), 0.f, 0.000244140625f, v);
+      }
+#pragma unroll
+      for (int d = 16; d > 0; d >>= 1) {
+        v.x += __shfl_xor_sync(full, v.x, d);
+        v.y += __shfl_xor_sync(full, v.y, d);
+        v.z += __shfl_xor_sync(full, v.z, d);
+      }
+      if (lane == o) {
+        w.x += v.x;
+        w.y += v.y;
+        w.z += v.z;
+      }
+      __syncwarp();
     }
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) u[k][c] += __shfl_xor_sync(0xffffffffu, u[k][c], o);
-    if (lane < NUNK * NUNK) {
-      const int k = lane / NUNK, l = lane % NUNK;
-      float bx, by, bz;
-      if (l == 0) { bx = t1x[i]; by = t1y[i]; bz = t1z[i]; }
-      else if (l == 1) { bx = t2x[i]; by = t2y[i]; bz = t2z[i]; }
-      else { bx = tnx[i]; by = tny[i]; bz = tnz[i]; }
-      const float ux = k == 0 ? u[0][0] : (k == 1 ? u[1][0] : u[2][0]);
-      const float uy = k == 0 ? u[0][1] : (k == 1 ? u[1][1] : u[2][1]);
-      const float uz = k == 0 ? u[0][2] : (k == 1 ? u[1][2] : u[2][2]);
+    if (act) {
+      const float4 s1 = srec[j].s1, s2 = srec[j].s2;
+      const float b[3][3] = {{t1x[i], t1y[i], t1z[i]}, {t2x[i], t2y[i], t2z[i]},
+                             {NUNK == 3 ? tnx[i] : 0.f, NUNK == 3 ? tny[i] : 0.f, NUNK == 3 ? tnz[i] : 0.f}};
+      const float u[3][3] = {{w.z * s1.y - w.y * s1.z, w.x * s1.z - w.z * s1.x, w.y * s1.x - w.x * s1.y},
+                             {w.z * s2.y - w.y * s2.z, w.x * s2.z - w.z * s2.x, w.y * s2.x - w.x * s2.y},
+                             {s1.w * w.x, s1.w * w.y, s1.w * w.z}};
       float* col = coeff + (size_t)j * NUNK * (size_t)ld + (size_t)i * NUNK;
-      col[(size_t)k * ld + l] = (ux * bx + uy * by + uz * bz) * fac;
+#pragma unroll
+      for (int k = 0; k < NUNK; ++k)
+#pragma unroll
+        for (int l = 0; l < NUNK; ++l)
+          col[(size_t)k * ld + l] = (u[k][0] * b[l][0] + u[k][1] * b[l][1] + u[k][2] * b[l][2]) * fac;
     }
-    __syncwarp();
   }
+}
+
+// the centroids of a panel's sub-triangles, 16 threads per panel (one per level-2 sub-triangle)
+__global__ void k_pack_centroids(int np, const TriG* __restrict__ tri, float4* cen_out) {
+  const int g = blockIdx.x * blockDim.x + threadIdx.x, j = g >> 4, p = g & 15;
+  if (j >= np) return;
+  float4* o = cen_out + (size_t)j * kCenRow;
+  auto put = [&](int at, const TriG& t) {
+    float cx, cy, cz;
+    cen(t, cx, cy, cz);
+    o[at] = make_float4(cx, cy, cz, 0.f);
+  };
+  const TriG t1 = child(tri[j], p >> 2);
+  if ((p & 3) == 0) put(p >> 2, t1);
+  const TriG t2 = child(t1, p & 3);
+  put(4 + p, t2);
+#pragma unroll
+  for (int c = 0; c < 4; ++c) put(20 + 4 * p + c, child(t2, c));
 }
 
 __global__ void k_pack_tri(int np, const float* __restrict__ x, const float* __restrict__ y,
@@ -483,6 +513,7 @@ extern "C" int32_t o3g_panels_on_panels_coeff(int32_t maxlev, int32_t nunk, int3
                                    : 0u;
   size_t bytes = align_up((size_t)snp_pad * sizeof(SrcRec)) + align_up((size_t)snp_pad * sizeof(TriG)) +
                  align_up((size_t)tnp * sizeof(TriG)) + align_up(sizeof(unsigned)) + align_up((size_t)cap * 8);
+  if (cap > 0) bytes += align_up((size_t)snp * kCenRow * 16) + align_up((size_t)tnp * kCenRow * 16);
   Workspace* ws = nullptr;
   O3G_TRY(workspace_get(st, bytes, &ws));
   Carve cv(ws->base);
@@ -493,12 +524,19 @@ extern "C" int32_t o3g_panels_on_panels_coeff(int32_t maxlev, int32_t nunk, int3
   nl.count = cv.take<unsigned>(1);
   nl.pairs = cv.take<uint2>(cap > 0 ? cap : 1);
   nl.cap = cap;
+  float4* scen = cap > 0 ? cv.take<float4>((size_t)snp * kCenRow) : nullptr;
+  float4* tcen = cap > 0 ? cv.take<float4>((size_t)tnp * kCenRow) : nullptr;
   O3G_CUDA_TRY(cudaMemsetAsync(nl.count, 0, sizeof(unsigned), st));
   k_pack_src_panels<<<(snp_pad + 255) / 256, 256, 0, st>>>(snp, src->x, src->y, src->z, src->idx, src->area, src->x1x,
                                                           src->x1y, src->x1z, src->x2x, src->x2y, src->x2z, snp_pad,
                                                           srec, stri);
   k_pack_tri<<<(tnp + 255) / 256, 256, 0, st>>>(tnp, targ->x, targ->y, targ->z, targ->idx, ttri);
   note_launch(2);
+  if (cap > 0 && maxlev > 0) {
+    k_pack_centroids<<<(unsigned)((16LL * snp + 255) / 256), 256, 0, st>>>(snp, stri, scen);
+    k_pack_centroids<<<(unsigned)((16LL * tnp + 255) / 256), 256, 0, st>>>(tnp, ttri, tcen);
+    note_launch(2);
+  }
   dim3 grid((tnp + kCB - 1) / kCB, sblocks);
   KernelTimer& tm = thread_timer();
   tm.begin(st);
@@ -510,7 +548,7 @@ extern "C" int32_t o3g_panels_on_panels_coeff(int32_t maxlev, int32_t nunk, int3
                                      targ->x2y, targ->x2z, nullptr, nullptr, nullptr, tnp, is_self, maxlev, coeffs, ld,
                                      vec2, nl);
     if (cap > 0)
-      k_coeff_near<2><<<nearblocks, 32 * kNearWarps, 0, st>>>(srec, stri, ttri, targ->area, targ->x1x, targ->x1y,
+      k_coeff_near<2><<<nearblocks, 32 * kNearWarps, 0, st>>>(srec, scen, tcen, targ->area, targ->x1x, targ->x1y,
                                                               targ->x1z, targ->x2x, targ->x2y, targ->x2z, nullptr,
                                                               nullptr, nullptr, maxlev, coeffs, ld, nl);
   } else {
@@ -518,7 +556,7 @@ extern "C" int32_t o3g_panels_on_panels_coeff(int32_t maxlev, int32_t nunk, int3
                                      targ->x2y, targ->x2z, targ->nx, targ->ny, targ->nz, tnp, is_self, maxlev, coeffs,
                                      ld, 0, nl);
     if (cap > 0)
-      k_coeff_near<3><<<nearblocks, 32 * kNearWarps, 0, st>>>(srec, stri, ttri, targ->area, targ->x1x, targ->x1y,
+      k_coeff_near<3><<<nearblocks, 32 * kNearWarps, 0, st>>>(srec, scen, tcen, targ->area, targ->x1x, targ->x1y,
                                                               targ->x1z, targ->x2x, targ->x2y, targ->x2z, targ->nx,
                                                               targ->ny, targ->nz, maxlev, coeffs, ld, nl);
   }
