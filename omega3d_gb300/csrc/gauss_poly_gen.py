@@ -216,7 +216,8 @@ def write_ds(table, worst, path):
 // D(q) = -(2/3) G'(q), degree {DEG_DS} in t = q s + o (s, o the float
 // values below).  Coefficients of degree >= {NDS} are floats (Horner in float); degrees
 // {NDS - 1}..0 are (hi, lo) float pairs (Horner in double-single).  Evaluated that way from an
-// exact q the result stays within {worst:.2e} relative of the double-precision functions.
+// exact q the result stays within {worst:.2e} relative of the double-precision functions
+// (D, which is rounded to float, needs the pairs of degrees 1 and 0 only).
 #pragma once
 
 namespace o3g {{

@@ -128,10 +128,9 @@ __device__ __forceinline__ void pair_g_ds(const V4<float>& t, const V4<float>& s
   const dsf dx = ds_two_sum(t.x, -s.x);
   const dsf dy = ds_two_sum(t.y, -s.y);
   const dsf dz = ds_two_sum(t.z, -s.z);
-  const dsf d2 = ds_add(ds_add(ds_sq(dx), ds_sq(dy)), ds_sq(dz));
   dsf r3;
   float b3;
-  core_ds<C, true>(d2, w.w, HAVE_TR ? t.w : 0.f, r3, b3);
+  core_ds<C, true>(dx, dy, dz, w.w, HAVE_TR ? t.w : 0.f, r3, b3);
   const dsf cx = ds_cross(dz, w.y, dy, w.z);
   const dsf cy = ds_cross(dx, w.z, dz, w.x);
   const dsf cz = ds_cross(dy, w.x, dx, w.y);
@@ -161,10 +160,9 @@ __device__ __forceinline__ void pair_v_ds(const V4<float>& t, const V4<float>& s
   const dsf dx = ds_two_sum(t.x, -s.x);
   const dsf dy = ds_two_sum(t.y, -s.y);
   const dsf dz = ds_two_sum(t.z, -s.z);
-  const dsf d2 = ds_add(ds_add(ds_sq(dx), ds_sq(dy)), ds_sq(dz));
   dsf r3;
   float b3;
-  core_ds<C, false>(d2, w.w, HAVE_TR ? t.w : 0.f, r3, b3);
+  core_ds<C, false>(dx, dy, dz, w.w, HAVE_TR ? t.w : 0.f, r3, b3);
   ds_accum(a[0], a[3], r3, ds_cross(dz, w.y, dy, w.z));
   ds_accum(a[1], a[4], r3, ds_cross(dx, w.z, dz, w.x));
   ds_accum(a[2], a[5], r3, ds_cross(dy, w.x, dx, w.y));
@@ -196,9 +194,11 @@ __device__ __forceinline__ void sweep_tile(const V4<T>* sp, const V4<T>* sw, con
                                            float (*hi)[NH], float (*lo)[NH]) {
   constexpr bool SUMC = SumComp<MODE>::value;
   constexpr int FOLD = SUMC ? 16 : NS;
+  // the accurate pair is 170 (RM) to 250 operations long: four of them overflow the instruction cache
+  constexpr int UN = MODE == MODE_DS ? 2 : 4;
 #pragma unroll 1
   for (int j0 = 0; j0 < NS; j0 += FOLD) {
-#pragma unroll 4
+#pragma unroll UN
     for (int j = j0; j < j0 + FOLD; ++j) {
       const V4<T> s = sp[j];
       const V4<T> w = sw[j];
