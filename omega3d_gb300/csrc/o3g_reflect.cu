@@ -11,6 +11,15 @@
 // minimum (a new minimum restarts the sums).  All float arithmetic uses the _rn
 // intrinsics in the reference's operation order (no contraction) and its 1/x in double,
 // so the pushed positions are bit-identical to the reference's.
+//
+// A panel whose distance is sure to be at least the running minimum plus 10 epsilon changes
+// nothing, so each point skips the panels whose bounding spheres are out of its reach: 12
+// operations instead of 130.  The sphere bounds the corners and edges; it bounds the interior
+// test, whose distance is the product with the panel's normal, for normals that are unit and
+// perpendicular to within 1e-3, and other panels are never skipped.  The points of a warp lie
+// anywhere, so each lane marks its own panels of every 32 and takes them one by one, whichever
+// the others take: skipping only what the whole warp can skip left half of the panels.  Measured
+// (one GB300), 65,536 points, 1,280 panels: 690 -> 430 us (559 by warps).
 #include "o3g_common.cuh"
 
 #include <cfloat>
@@ -31,6 +40,22 @@ struct PanelTri {
   float4 g;   // e20 (x0 - x2), inv20
 };
 
+// a sphere around the panel: centroid, 1.03 times its radius; infinite where the panel may not be skipped
+__device__ __forceinline__ float4 bound_of(const PanelTri& t) {
+  const float cx = (t.a.x + t.a.w + t.b.z) * (1.f / 3.f), cy = (t.a.y + t.b.x + t.b.w) * (1.f / 3.f),
+              cz = (t.a.z + t.b.y + t.c.x) * (1.f / 3.f);
+  auto d2 = [&](float x, float y, float z) { return (x - cx) * (x - cx) + (y - cy) * (y - cy) + (z - cz) * (z - cz); };
+  const float r2 = fmaxf(fmaxf(d2(t.a.x, t.a.y, t.a.z), d2(t.a.w, t.b.x, t.b.y)), d2(t.b.z, t.b.w, t.c.x));
+  const float nx = t.c.y, ny = t.c.z, nz = t.c.w;
+  auto flat = [&](const float4& e) {
+    const float p = nx * e.x + ny * e.y + nz * e.z;
+    return p * p <= 1e-6f * (e.x * e.x + e.y * e.y + e.z * e.z);
+  };
+  const float nn = nx * nx + ny * ny + nz * nz;
+  const bool good = nn >= 0.999f && nn <= 1.001f && flat(t.e) && flat(t.f) && flat(t.g) && r2 < 1e30f;
+  return make_float4(cx, cy, cz, good ? 1.03f * sqrtf(r2) : __int_as_float(0x7f800000));
+}
+
 __device__ __forceinline__ float dot_rn(float a0, float a1, float a2, float b0, float b1, float b2) {
   return __fadd_rn(__fadd_rn(__fmul_rn(a0, b0), __fmul_rn(a1, b1)), __fmul_rn(a2, b2));
 }
@@ -42,7 +67,7 @@ __device__ __forceinline__ float4 edge_rec(float ax, float ay, float az, float b
 
 __global__ void k_pack_tri(int np, const float* __restrict__ x, const float* __restrict__ y,
                            const float* __restrict__ z, const uint32_t* __restrict__ idx, const float* __restrict__ nx,
-                           const float* __restrict__ ny, const float* __restrict__ nz, PanelTri* out) {
+                           const float* __restrict__ ny, const float* __restrict__ nz, PanelTri* out, float4* bound) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= np) return;
   const uint32_t p0 = idx[3 * (size_t)j], p1 = idx[3 * (size_t)j + 1], p2 = idx[3 * (size_t)j + 2];
@@ -54,6 +79,7 @@ __global__ void k_pack_tri(int np, const float* __restrict__ x, const float* __r
   t.f = edge_rec(x[p1], y[p1], z[p1], x[p2], y[p2], z[p2]);
   t.g = edge_rec(x[p2], y[p2], z[p2], x[p0], y[p0], z[p0]);
   out[j] = t;
+  bound[j] = bound_of(t);
 }
 
 // squared distance |e x d|^2 / |e|^2 to the edge's line, kept when the foot lies on the edge
@@ -117,9 +143,11 @@ __device__ __forceinline__ void closest_rn(const PanelTri& p, float tx, float ty
 }
 
 __global__ void __launch_bounds__(kRB) k_clear_inner(int n, float* x, float* y, float* z,
-                                                     const PanelTri* __restrict__ tri, int np, float cut,
+                                                     const PanelTri* __restrict__ tri,
+                                                     const float4* __restrict__ bound, int np, float cut,
                                                      int* pushed) {
-  __shared__ PanelTri st[kRB];
+  __shared__ float4 st[6][kRB];   // a..g of the panels
+  __shared__ float4 sb[kRB];
   const int i = blockIdx.x * kRB + threadIdx.x;
   const bool live = i < n;
   const float tx = live ? x[i] : 0.f, ty = live ? y[i] : 0.f, tz = live ? z[i] : 0.f;
@@ -127,24 +155,46 @@ __global__ void __launch_bounds__(kRB) k_clear_inner(int n, float* x, float* y, 
   float mind = FLT_MAX;
   float mn0 = 0.f, mn1 = 0.f, mn2 = 0.f, mc0 = 0.f, mc1 = 0.f, mc2 = 0.f;
   int nh = 0;
+  // 1.02 sqrt(mind + eps); infinite until the minimum is well below closest_rn's own start of 9.9e9 (a panel
+  // farther than that has that distance)
+  float reach = __int_as_float(0x7f800000);
   for (int j0 = 0; j0 < np; j0 += kRB) {
     __syncthreads();
-    if (j0 + (int)threadIdx.x < np) st[threadIdx.x] = tri[j0 + threadIdx.x];
+    const bool has = j0 + (int)threadIdx.x < np;
+    if (has) {
+      const PanelTri p = tri[j0 + threadIdx.x];
+      st[0][threadIdx.x] = p.a; st[1][threadIdx.x] = p.b; st[2][threadIdx.x] = p.c;
+      st[3][threadIdx.x] = p.e; st[4][threadIdx.x] = p.f; st[5][threadIdx.x] = p.g;
+    }
+    if (has) sb[threadIdx.x] = bound[j0 + threadIdx.x];
     __syncthreads();
     const int m = min(kRB, np - j0);
-    for (int jj = 0; jj < m; ++jj) {
-      const PanelTri p = st[jj];
-      float d2, cx, cy, cz;
-      closest_rn(p, tx, ty, tz, d2, cx, cy, cz);
-      if (d2 < __fsub_rn(mind, eps)) {
-        mind = d2;
-        mn0 = __fadd_rn(0.f, p.c.y); mn1 = __fadd_rn(0.f, p.c.z); mn2 = __fadd_rn(0.f, p.c.w);
-        mc0 = __fadd_rn(0.f, cx); mc1 = __fadd_rn(0.f, cy); mc2 = __fadd_rn(0.f, cz);
-        nh = 1;
-      } else if (d2 < __fadd_rn(mind, eps)) {
-        mn0 = __fadd_rn(mn0, p.c.y); mn1 = __fadd_rn(mn1, p.c.z); mn2 = __fadd_rn(mn2, p.c.w);
-        mc0 = __fadd_rn(mc0, cx); mc1 = __fadd_rn(mc1, cy); mc2 = __fadd_rn(mc2, cz);
-        ++nh;
+    for (int jb = 0; jb < m; jb += 32) {
+      unsigned todo = 0u;
+#pragma unroll 8
+      for (int k = 0; k < 32; ++k) {
+        const float4 b = sb[jb + k];
+        const float dx = tx - b.x, dy = ty - b.y, dz = tz - b.z, rr = reach + b.w;
+        if (!(dx * dx + dy * dy + dz * dz > rr * rr)) todo |= 1u << k;
+      }
+      if (m - jb < 32) todo &= (1u << (m - jb)) - 1u;
+      if (!live) todo = 0u;
+      for (; todo; todo &= todo - 1u) {
+        const int jj = jb + __ffs(todo) - 1;
+        const PanelTri p{st[0][jj], st[1][jj], st[2][jj], st[3][jj], st[4][jj], st[5][jj]};
+        float d2, cx, cy, cz;
+        closest_rn(p, tx, ty, tz, d2, cx, cy, cz);
+        if (d2 < __fsub_rn(mind, eps)) {
+          mind = d2;
+          reach = mind < 9.4e9f ? 1.02f * sqrtf(mind + eps) : reach;
+          mn0 = __fadd_rn(0.f, p.c.y); mn1 = __fadd_rn(0.f, p.c.z); mn2 = __fadd_rn(0.f, p.c.w);
+          mc0 = __fadd_rn(0.f, cx); mc1 = __fadd_rn(0.f, cy); mc2 = __fadd_rn(0.f, cz);
+          nh = 1;
+        } else if (d2 < __fadd_rn(mind, eps)) {
+          mn0 = __fadd_rn(mn0, p.c.y); mn1 = __fadd_rn(mn1, p.c.z); mn2 = __fadd_rn(mn2, p.c.w);
+          mc0 = __fadd_rn(mc0, cx); mc1 = __fadd_rn(mc1, cy); mc2 = __fadd_rn(mc2, cz);
+          ++nh;
+        }
       }
     }
   }
@@ -169,11 +219,14 @@ int32_t clear_inner_layer_dev(int n, float* x, float* y, float* z, const o3g_sur
                               int* dev_count, cudaStream_t st) {
   const int np = surf.np;
   Workspace* ws = nullptr;
-  O3G_TRY(workspace_get(st, align_up((size_t)np * sizeof(PanelTri)), &ws));
-  PanelTri* tri = (PanelTri*)ws->base;
+  O3G_TRY(workspace_get(st, align_up((size_t)np * sizeof(PanelTri)) + align_up((size_t)np * sizeof(float4)), &ws));
+  Carve cv(ws->base);
+  PanelTri* tri = cv.take<PanelTri>(np);
+  float4* bound = cv.take<float4>(np);
   if (n == 0) return O3G_OK;
-  k_pack_tri<<<(np + 255) / 256, 256, 0, st>>>(np, surf.x, surf.y, surf.z, surf.idx, surf.nx, surf.ny, surf.nz, tri);
-  k_clear_inner<<<(n + kRB - 1) / kRB, kRB, 0, st>>>(n, x, y, z, tri, np, cut, dev_count);
+  k_pack_tri<<<(np + 255) / 256, 256, 0, st>>>(np, surf.x, surf.y, surf.z, surf.idx, surf.nx, surf.ny, surf.nz, tri,
+                                               bound);
+  k_clear_inner<<<(n + kRB - 1) / kRB, kRB, 0, st>>>(n, x, y, z, tri, bound, np, cut, dev_count);
   note_launch(2);
   O3G_CUDA_TRY(cudaGetLastError());
   return O3G_OK;
