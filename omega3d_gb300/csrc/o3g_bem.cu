@@ -422,9 +422,11 @@ __global__ void __launch_bounds__(kPanelThreads) k_panel_lu(PanelArgs a) {
 // What bounds a panel is latency: one pivot exchange per column.  Through global memory
 // (k_panel_lu, 152 blocks) it costs 3.1 us a column; among the 16 blocks of one cluster the
 // candidates travel through distributed shared memory behind the hardware's cluster barrier.
-// The rows then have to fit 16 SMs: 640 rows of W = 64 columns in a block's registers, so up to
+// The rows then have to fit 16 SMs: up to 640 rows of W = 64 columns in a block's registers, so
 // 10,240 rows fit; a kNb-column panel is factored W columns at a time (k_panel_next brings the
-// second half up to date).  More rows than that go to k_panel_lu.
+// second half up to date).  More rows than that go to k_panel_lu.  A column's steps are a chain that
+// every warp runs for itself, so the fewer warps share a scheduler the faster: 64 columns take 86 us
+// with 10 warps a block (10,240 rows), 73 with 8 (8,192), 65 with 4 (4,096), whatever the cluster's size.
 //
 // Rows do not move while the sub-panel is factored: each thread tracks the position its rows have
 // after the interchanges so far (LAPACK's order); the sub-panel's rows are stored there at
@@ -438,19 +440,18 @@ __global__ void __launch_bounds__(kPanelThreads) k_panel_lu(PanelArgs a) {
 // tile reads 4 multipliers and 4 elements of U for 16 products, and a broadcast read of shared
 // memory costs as much as 32 different words (two full rows per thread: 58 reads for 112
 // products, and this update a fifth of the kernel).
-// Measured (one GB300), 64 columns: 112 -> 86 us (one warp's instructions in series are what
-// is left: 150 a column); factorisation at n = 10,240: 43.2 -> 29.3 ms (23.2 with the
-// kernels below).  Not kept: full
+// Measured (one GB300), 64 columns with 10 warps: 112 -> 86 us (one warp's instructions in series
+// are what is left: 150 a column); factorisation at n = 10,240: 43.2 -> 21.6 ms with the kernels below.  Not kept: full
 // rows in every exchange with a rank-1 update of the whole width per column (2.3 us a column),
 // the column's code unrolled (by 8: 108 against 97 us; fetching it takes longer than running
 // it), a block barrier and a second search by every warp before the exchange (112 against
 // 97 us), a cluster barrier instead of mbarriers (its release waits for the finished columns'
 // global stores).
-constexpr int kCpThreads = 320;
-constexpr int kCpWarps = kCpThreads / 32;
 constexpr int kCpMax = 16;                  // blocks per cluster
 constexpr int kCpGroup = 8;                 // columns between two updates of the rest
 constexpr int kCpW = 64, kCpRows = 2;       // columns of a sub-panel, rows per thread
+// threads per block, the fewest that hold a panel: 4,096 rows, 8,192, 10,240 in 16 blocks
+constexpr int kCpThreads[] = {128, 256, 320};
 
 struct ClusterPanelArgs {
   float* A;
@@ -461,21 +462,22 @@ struct ClusterPanelArgs {
   int* err;               // set when a wait runs out
   const float* u;         // the rows of U above the sub-panel, (c - k0) x w column-major (k_panel_next)
 };
-template <int W, int RPT> struct ClusterShared {
+template <int W, int NT> struct ClusterShared {
+  static constexpr int RPT = kCpRows, warps = NT / 32;
   static constexpr int R = W - kCpGroup;          // columns right of the first group
-  static constexpr int rows_n = RPT * kCpThreads; // rows of a block
+  static constexpr int rows_n = RPT * NT;         // rows of a block
   float xch[2][kCpGroup][kCpMax][kCpGroup];       // the blocks' candidate windows, by group parity and column
   float rows[2][kCpGroup][R];                     // the pivot rows' later columns, by group parity
   float u12[2][kCpGroup][R];                      // the same after the solve
   float own[kCpGroup][R];                         // those that this block sends
-  float cand[kCpWarps][kCpGroup];                 // the warps' candidate windows
+  float cand[warps][kCpGroup];                    // the warps' candidate windows
   float l[kCpGroup][rows_n];                      // the group's multipliers, 0 where a row takes no update
   float4 turn[2][rows_n];                         // the next group's columns, from tiles to rows
   uint2 head[2][kCpGroup][kCpMax];                // candidates' |value| bits + 1 (0: none) and positions
-  uint2 whead[kCpWarps];                          // the warps'
+  uint2 whead[warps];                             // the warps'
   unsigned long long bar[3];                      // mbarriers: a column's candidates (by parity), a group's rows
   int prow[kCpGroup];                             // the group's k-th pivot row, if it is one of this block's (-1)
-  float done[W * RPT * kCpThreads];               // the finished columns
+  float done[W * RPT * NT];                       // the finished columns
 };
 __device__ __forceinline__ unsigned cluster_rank() {
   unsigned r;
@@ -544,29 +546,30 @@ __device__ __forceinline__ bool cluster_wait(unsigned bar, unsigned parity, int*
   return false;
 }
 
-// A block's rows right of the group: warp w holds the rows 128 (w % 5) + lane + 32 i, i < 4, and of
-// every group's 8 columns the half w / 5 (chunk c: columns 8 (c + 1) + 4 (w / 5) .. + 3).
+// A block's rows right of the group, NRB = NT / 64 row blocks of 128: warp w holds the rows 128 (w % NRB) +
+// lane + 32 i, i < 4, and of every group's 8 columns the half w / NRB (chunk c: columns 8 (c + 1) +
+// 4 (w / NRB) .. + 3).
 template <int W> struct PanelTile {
   static constexpr int NCH = W / kCpGroup - 1;
   float4 y[4][NCH];
 };
 // their rank-kCpGroup update after group g: y -= l u
-template <int W, class Shared>
-__device__ __forceinline__ void panel_update(PanelTile<W>& t, const Shared& sh, int g, int gp, int rb, int cb) {
-  constexpr int kHalfK = kCpGroup / 2;   // multipliers in registers at a time
+template <int W, int NT>
+__device__ __forceinline__ void panel_update(PanelTile<W>& t, const ClusterShared<W, NT>& sh, int g, int gp, int rb, int cb) {
+  constexpr int KS = NT > 256 ? kCpGroup / 2 : kCpGroup;   // multipliers in registers at a time
   const int lane = threadIdx.x & 31;
 #pragma unroll 1
-  for (int k0 = 0; k0 < kCpGroup; k0 += kHalfK) {
-    float l[kHalfK][4];
+  for (int k0 = 0; k0 < kCpGroup; k0 += KS) {
+    float l[KS][4];
 #pragma unroll
-    for (int k = 0; k < kHalfK; ++k)
+    for (int k = 0; k < KS; ++k)
 #pragma unroll
       for (int i = 0; i < 4; ++i) l[k][i] = -sh.l[k0 + k][128 * rb + lane + 32 * i];
 #pragma unroll
     for (int c = 0; c < PanelTile<W>::NCH; ++c)
       if (c >= g)
 #pragma unroll
-        for (int k = 0; k < kHalfK; ++k) {
+        for (int k = 0; k < KS; ++k) {
           const float4 u = *reinterpret_cast<const float4*>(&sh.u12[gp][k0 + k][8 * c + 4 * cb]);
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
@@ -579,12 +582,12 @@ __device__ __forceinline__ void panel_update(PanelTile<W>& t, const Shared& sh, 
   }
 }
 
-// One group of columns; x[.][0..kCpGroup) are the rows tid and tid + kCpThreads, t what lies right of it.
-template <int W, int RPT>
-__device__ __forceinline__ void panel_group(const ClusterPanelArgs& a, ClusterShared<W, RPT>& sh, float (*x)[kCpGroup],
+// One group of columns; x[.][0..kCpGroup) are the rows tid and tid + NT, t what lies right of it.
+template <int W, int NT>
+__device__ __forceinline__ void panel_group(const ClusterPanelArgs& a, ClusterShared<W, NT>& sh, float (*x)[kCpGroup],
                                             PanelTile<W>& t, int* pos, int g0, unsigned rank, unsigned C, bool& dead) {
   constexpr unsigned full = 0xffffffffu;
-  constexpr int B = kCpGroup, R = W - B;
+  constexpr int B = kCpGroup, R = W - B, RPT = kCpRows, NRB = NT / 64;
   auto off = [&](const void* p) { return (unsigned)((const char*)p - (const char*)&sh); };
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int cg = a.c + g0, gp = (g0 / B) & 1;
@@ -624,8 +627,8 @@ __device__ __forceinline__ void panel_group(const ClusterPanelArgs& a, ClusterSh
       __syncwarp();
       // warp 0 finds the block's and sends its window and head to every block
       if (warp == 0) {
-        asm volatile("bar.sync 1, %0;" ::"n"(kCpThreads) : "memory");
-        const uint2 hw = lane < kCpWarps ? sh.whead[lane] : make_uint2(0u, full);
+        asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory");
+        const uint2 hw = lane < NT / 32 ? sh.whead[lane] : make_uint2(0u, full);
         const int wi = best_lane(hw.x, hw.y, m);
         const uint2 hs = make_uint2(m, __shfl_sync(full, hw.y, wi));
         if (lane == 0) cluster_expect((unsigned)__cvta_generic_to_shared(&sh.bar[par]), C * (B * 4 + 8));
@@ -636,7 +639,7 @@ __device__ __forceinline__ void panel_group(const ClusterPanelArgs& a, ClusterSh
           if (h == 0) cluster_send(peer + off(&sh.head[gp][jj][rank]), hs.x, hs.y, bar);
         }
       } else {
-        asm volatile("bar.arrive 1, %0;" ::"n"(kCpThreads) : "memory");
+        asm volatile("bar.arrive 1, %0;" ::"n"(NT) : "memory");
       }
       const unsigned bar = (unsigned)__cvta_generic_to_shared(&sh.bar[par]);
       if (!dead) dead = !cluster_wait(bar, (unsigned)((g0 + jj) >> 1) & 1u, a.err);
@@ -702,14 +705,14 @@ __device__ __forceinline__ void panel_group(const ClusterPanelArgs& a, ClusterSh
       x[q][B - 1] = t;
     }
   }
-  const int g = g0 / B, rb = warp % 5, cb = warp / 5;
+  const int g = g0 / B, rb = warp % NRB, cb = warp / NRB;
   const bool more = g0 + B < a.w;
   if (more) {
     // which rows the pivots are
 #pragma unroll
     for (int q = 0; q < RPT; ++q) {
       const int e = pos[q] - cg;
-      if ((unsigned)e < (unsigned)B) sh.prow[e] = (tid + q * kCpThreads) | (g0 << 16);
+      if ((unsigned)e < (unsigned)B) sh.prow[e] = (tid + q * NT) | (g0 << 16);
     }
     if (tid == 0) cluster_expect((unsigned)__cvta_generic_to_shared(&sh.bar[2]), B * (R - g0) * 4);
     __syncthreads();
@@ -747,12 +750,12 @@ __device__ __forceinline__ void panel_group(const ClusterPanelArgs& a, ClusterSh
 #pragma unroll
     for (int q = 0; q < RPT; ++q)
 #pragma unroll
-      for (int k = 0; k < B; ++k) sh.l[k][tid + q * kCpThreads] = pos[q] - cg > k ? x[q][k] : 0.f;
+      for (int k = 0; k < B; ++k) sh.l[k][tid + q * NT] = pos[q] - cg > k ? x[q][k] : 0.f;
   }
 #pragma unroll
   for (int q = 0; q < RPT; ++q)
 #pragma unroll
-    for (int k = 0; k < B; ++k) sh.done[((g0 + k) * RPT + q) * kCpThreads + tid] = x[q][k];
+    for (int k = 0; k < B; ++k) sh.done[((g0 + k) * RPT + q) * NT + tid] = x[q][k];
   if (!more) return;
   const unsigned bar = (unsigned)__cvta_generic_to_shared(&sh.bar[2]);
   if (!dead) dead = !cluster_wait(bar, (unsigned)gp, a.err);
@@ -771,7 +774,7 @@ __device__ __forceinline__ void panel_group(const ClusterPanelArgs& a, ClusterSh
     }
   }
   __syncthreads();
-  panel_update<W>(t, sh, g, gp, rb, cb);
+  panel_update<W, NT>(t, sh, g, gp, rb, cb);
   // the next group's columns to the threads of their rows
 #pragma unroll
   for (int c = 0; c < PanelTile<W>::NCH; ++c)
@@ -781,36 +784,37 @@ __device__ __forceinline__ void panel_group(const ClusterPanelArgs& a, ClusterSh
   __syncthreads();
 #pragma unroll
   for (int q = 0; q < RPT; ++q) {
-    const float4 v0 = sh.turn[0][tid + q * kCpThreads], v1 = sh.turn[1][tid + q * kCpThreads];
+    const float4 v0 = sh.turn[0][tid + q * NT], v1 = sh.turn[1][tid + q * NT];
     x[q][0] = v0.x; x[q][1] = v0.y; x[q][2] = v0.z; x[q][3] = v0.w;
     x[q][4] = v1.x; x[q][5] = v1.y; x[q][6] = v1.z; x[q][7] = v1.w;
   }
 }
 
-template <int W, int RPT>
-__global__ void __launch_bounds__(kCpThreads, 1) k_panel_cluster(const ClusterPanelArgs a) {
+template <int W, int NT>
+__global__ void __launch_bounds__(NT, 1) k_panel_cluster(const ClusterPanelArgs a) {
+  constexpr int RPT = kCpRows, NRB = NT / 64;
   extern __shared__ __align__(16) char cpsm[];
   static_assert(kNb % W == 0 && W % 16 == 0, "whole sub-panels and groups");
-  using Sh = ClusterShared<W, RPT>;
+  using Sh = ClusterShared<W, NT>;
   static_assert(offsetof(Sh, rows) % 16 == 0 && offsetof(Sh, u12) % 16 == 0 &&
                     offsetof(Sh, own) % 16 == 0 && offsetof(Sh, cand) % 16 == 0 && (W - kCpGroup) % 4 == 0 &&
                     offsetof(Sh, xch) % 16 == 0 && offsetof(Sh, turn) % 16 == 0 && offsetof(Sh, head) % 8 == 0 &&
                     offsetof(Sh, whead) % 8 == 0 && offsetof(Sh, bar) % 8 == 0,
                 "vector accesses");
   static_assert(kCpMax <= 16 && kCpGroup == 8 && (W - kCpGroup) / 4 <= 32, "lanes per destination");
-  static_assert(W - kCpGroup <= kCpThreads, "a thread per column of U12");
-  ClusterShared<W, RPT>& sh = *reinterpret_cast<ClusterShared<W, RPT>*>(cpsm);
+  static_assert(W - kCpGroup <= NT, "a thread per column of U12");
+  ClusterShared<W, NT>& sh = *reinterpret_cast<ClusterShared<W, NT>*>(cpsm);
   const int tid = threadIdx.x;
   const unsigned rank = cluster_rank(), C = cluster_size();
   const int c = a.c, w = a.w, kp = a.c - a.k0;
-  const int row0 = c + (int)rank * (kCpThreads * RPT) + tid;   // this thread's rows: row0 + q kCpThreads
-  static_assert(W == 64 && RPT == 2 && kCpThreads == 320, "tiles of 128 rows");
+  const int row0 = c + (int)rank * (NT * RPT) + tid;   // this thread's rows: row0 + q NT
+  static_assert(W == 64 && RPT == 2 && NT % 64 == 0 && sizeof(Sh) <= 227 * 1024, "tiles of 128 rows, two column halves");
   float x[RPT][kCpGroup];
   PanelTile<W> t;
   int pos[RPT];
 #pragma unroll
   for (int q = 0; q < RPT; ++q) {
-    const int r = row0 + q * kCpThreads;
+    const int r = row0 + q * NT;
     const bool in = r < a.n;
     pos[q] = in ? r : -1;
 #pragma unroll
@@ -818,10 +822,10 @@ __global__ void __launch_bounds__(kCpThreads, 1) k_panel_cluster(const ClusterPa
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int r = c + (int)rank * (kCpThreads * RPT) + 128 * ((tid >> 5) % 5) + (tid & 31) + 32 * i;
+    const int r = c + (int)rank * (NT * RPT) + 128 * ((tid >> 5) % NRB) + (tid & 31) + 32 * i;
 #pragma unroll
     for (int e = 0; e < PanelTile<W>::NCH; ++e) {
-      const int k = 8 * (e + 1) + 4 * ((tid >> 5) / 5);
+      const int k = 8 * (e + 1) + 4 * ((tid >> 5) / NRB);
       const float* g = a.A + (size_t)(c + k) * a.ld + r;
       t.y[i][e].x = r < a.n && k < w ? g[0] : 0.f;
       t.y[i][e].y = r < a.n && k + 1 < w ? g[a.ld] : 0.f;
@@ -838,18 +842,18 @@ __global__ void __launch_bounds__(kCpThreads, 1) k_panel_cluster(const ClusterPa
   }
   // the rows of U above this sub-panel (k_panel_next)
   if (rank == 0)
-    for (int e = tid; e < kp * w; e += kCpThreads)
+    for (int e = tid; e < kp * w; e += NT)
       a.A[(size_t)(c + e / kp) * a.ld + a.k0 + e % kp] = a.u[e];
   cluster_barrier();   // every block runs: its shared memory may be written
   bool dead = false;
 #pragma unroll 1
-  for (int g0 = 0; g0 < w; g0 += kCpGroup) panel_group<W, RPT>(a, sh, x, t, pos, g0, rank, C, dead);
+  for (int g0 = 0; g0 < w; g0 += kCpGroup) panel_group<W, NT>(a, sh, x, t, pos, g0, rank, C, dead);
   // every row to the place the interchanges gave it
 #pragma unroll 4
   for (int k = 0; k < w; ++k)
 #pragma unroll
     for (int q = 0; q < RPT; ++q)
-      if (pos[q] >= 0) a.A[(size_t)(c + k) * a.ld + pos[q]] = sh.done[(k * RPT + q) * kCpThreads + tid];
+      if (pos[q] >= 0) a.A[(size_t)(c + k) * a.ld + pos[q]] = sh.done[(k * RPT + q) * NT + tid];
   cluster_barrier();   // no block leaves while another may still write to its shared memory
 }
 
@@ -953,25 +957,26 @@ __global__ void __launch_bounds__(256) k_panel_next(float* A, long long ld, int 
     }
 }
 
-// The cluster kernel for m rows, or nothing when they do not fit: sub-panel width, blocks
+// The cluster kernels by the rows that they take: block size, shared memory and the largest cluster
+// that can be resident on this device (0: none)
 struct ClusterPlan {
   const void* kernel = nullptr;
-  int width = 0, blocks = 0;
+  int threads = 0, blocks = 0;
   size_t smem = 0;
 };
-// the largest cluster of the variant that can be resident on this device (0: none); sets the
-// kernel's attributes, once per factorisation
-template <int W, int RPT> static int32_t cluster_setup_of(int* largest) {
-  const void* k = (const void*)&k_panel_cluster<W, RPT>;
-  const size_t smem = sizeof(ClusterShared<W, RPT>);
-  O3G_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  O3G_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-  *largest = 0;
-  for (int c = kCpMax; c >= 1 && *largest == 0; c /= 2) {
+// sets the kernel's attributes, once per factorisation that may use it
+template <int NT> static int32_t cluster_setup_of(ClusterPlan* p) {
+  p->kernel = (const void*)&k_panel_cluster<kCpW, NT>;
+  p->threads = NT;
+  p->smem = sizeof(ClusterShared<kCpW, NT>);
+  p->blocks = 0;
+  O3G_CUDA_TRY(cudaFuncSetAttribute(p->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p->smem));
+  O3G_CUDA_TRY(cudaFuncSetAttribute(p->kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  for (int c = kCpMax; c >= 1 && p->blocks == 0; c /= 2) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(c);
-    cfg.blockDim = dim3(kCpThreads);
-    cfg.dynamicSmemBytes = smem;
+    cfg.blockDim = dim3(NT);
+    cfg.dynamicSmemBytes = p->smem;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = c;
@@ -979,25 +984,35 @@ template <int W, int RPT> static int32_t cluster_setup_of(int* largest) {
     cfg.attrs = at;
     cfg.numAttrs = 1;
     int nc = 0;
-    if (cudaOccupancyMaxActiveClusters(&nc, k, &cfg) == cudaSuccess && nc > 0) *largest = c;
+    if (cudaOccupancyMaxActiveClusters(&nc, p->kernel, &cfg) == cudaSuccess && nc > 0) p->blocks = c;
     else (void)cudaGetLastError();
   }
   return O3G_OK;
 }
-template <int W, int RPT> static bool cluster_fits(int m, int cmax, ClusterPlan* p) {
-  int c = 1;
-  while (c < cmax && c * kCpThreads * RPT < m) c *= 2;
-  if (cmax == 0 || c * kCpThreads * RPT < m) return false;
-  p->kernel = (const void*)&k_panel_cluster<W, RPT>;
-  p->width = W;
-  p->blocks = c;
-  p->smem = sizeof(ClusterShared<W, RPT>);
-  return true;
+// those that a matrix of n rows can use (the first that holds a panel is taken)
+static int32_t cluster_setup(int n, ClusterPlan (&p)[3]) {
+  static_assert(sizeof(kCpThreads) / sizeof(int) == 3, "one setup each");
+  O3G_TRY(cluster_setup_of<kCpThreads[0]>(&p[0]));
+  if (n > p[0].blocks * kCpThreads[0] * kCpRows) O3G_TRY(cluster_setup_of<kCpThreads[1]>(&p[1]));
+  if (n > p[1].blocks * kCpThreads[1] * kCpRows && p[1].kernel) O3G_TRY(cluster_setup_of<kCpThreads[2]>(&p[2]));
+  return O3G_OK;
+}
+// the plan for a panel of m rows, or nothing when it fits none
+static ClusterPlan cluster_for(int m, const ClusterPlan (&p)[3]) {
+  for (const ClusterPlan& v : p) {
+    const int rows = v.threads * kCpRows;
+    if (v.kernel == nullptr || v.blocks * rows < m) continue;
+    ClusterPlan r = v;
+    r.blocks = 1;
+    while (r.blocks * rows < m) r.blocks *= 2;
+    return r;
+  }
+  return ClusterPlan();
 }
 static int32_t launch_cluster_panel(const ClusterPlan& p, ClusterPanelArgs a, cudaStream_t st) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(p.blocks);
-  cfg.blockDim = dim3(kCpThreads);
+  cfg.blockDim = dim3(p.threads);
   cfg.dynamicSmemBytes = p.smem;
   cfg.stream = st;
   cudaLaunchAttribute at[1];
@@ -1804,7 +1819,7 @@ extern "C" int32_t o3g_bem_factor(o3g_bem_t* h, void* stream) {
   O3G_CUDA_TRY(cudaFuncGetAttributes(&fa, k_panel_lu));
   const size_t max_smem = (size_t)optin - fa.sharedSizeBytes;
   O3G_CUDA_TRY(cudaFuncSetAttribute(k_panel_lu, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem));
-  // panels of up to 40,960 rows run in one cluster (k_panel_cluster); this sizes k_panel_lu
+  // panels of up to 10,240 rows run in one cluster (k_panel_cluster); this sizes k_panel_lu
   int G = std::min(df.num_sms, 32 * kMaxKeysPerLane);
   int R = (n + G - 1) / G;
   size_t smem = ((size_t)kNb * R + 2 * kNb + 32) * sizeof(float);
@@ -1880,8 +1895,8 @@ extern "C" int32_t o3g_bem_factor(o3g_bem_t* h, void* stream) {
     note_launch();
   };
   auto at = [&](int r, int c) { return h->LU + (size_t)c * ld + r; };
-  int cmax = 0;
-  O3G_TRY((cluster_setup_of<kCpW, kCpRows>(&cmax)));
+  ClusterPlan plans[3];
+  O3G_TRY(cluster_setup(n, plans));
   O3G_CUDA_TRY(cudaFuncSetAttribute(k_panel_next, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PanelNextShared)));
   static_assert(kNb == 2 * kCpW && kCpW <= kNextMax, "at most one earlier sub-panel");
   // two-level right-looking LU: kNb-column panels inside kNbOuter-column outer panels; the
@@ -1893,11 +1908,11 @@ extern "C" int32_t o3g_bem_factor(o3g_bem_t* h, void* stream) {
       const int m = n - k0;
       // the debug wait test (o3g_debug_wait_test) needs a kernel that polls
       ClusterPlan cp;
-      if (!wait_test_on()) (void)cluster_fits<kCpW, kCpRows>(m, cmax, &cp);
+      if (!wait_test_on()) cp = cluster_for(m, plans);
       if (cp.kernel) {
-        for (int c = k0; c < k0 + jb; c += cp.width) {
+        for (int c = k0; c < k0 + jb; c += kCpW) {
           ClusterPanelArgs ca;
-          ca.A = h->LU; ca.ld = ld; ca.n = n; ca.k0 = k0; ca.c = c; ca.w = std::min(cp.width, k0 + jb - c);
+          ca.A = h->LU; ca.ld = ld; ca.n = n; ca.k0 = k0; ca.c = c; ca.w = std::min(kCpW, k0 + jb - c);
           ca.piv = h->piv; ca.singular = h->flags + 1; ca.err = h->flags;
           ca.u = linv;
           if (c > k0) {
