@@ -399,8 +399,9 @@ __device__ __forceinline__ void pair2(const float2* tt, const float4& q0, const 
   // which operands carry the signs decides the register assignment: at 65,536 particles (RM) the
   // compensated kernel takes 49.7 cycles per pair with the strengths negated and 53.3 with the
   // separations, the plain one 42.4 and 41.2 (51.5 and 41.3 with five staged rows)
-  const float2 ndx = ACC ? dx : neg2(dx), ndy = ACC ? dy : neg2(dy), ndz = ACC ? dz : neg2(dz);
-  const float2 nwx = ACC ? neg2(wx) : wx, nwy = ACC ? neg2(wy) : wy, nwz = ACC ? neg2(wz) : wz;
+  constexpr bool NEGW = ACC || C == CORE_EXP;
+  const float2 ndx = NEGW ? dx : neg2(dx), ndy = NEGW ? dy : neg2(dy), ndz = NEGW ? dz : neg2(dz);
+  const float2 nwx = NEGW ? neg2(wx) : wx, nwy = NEGW ? neg2(wy) : wy, nwz = NEGW ? neg2(wz) : wz;
   float2 cx = __fmul2_rn(ndy, nwz), cy = __fmul2_rn(dx, wz), cz = __fmul2_rn(ndx, nwy);
   cx = __ffma2_rn(dz, wy, cx);     // dz wy - dy wz
   cy = __ffma2_rn(ndz, nwx, cy);   // dx wz - dz wx
@@ -925,7 +926,11 @@ struct PairKernel {
 // 110.2 ms, while the per-split partial sums the reduction reads grow with the split
 // count (29 splits, 730 MB, at 96 waves).  The allocating entry points use kPairWaves.
 constexpr int kPairWaves = 48;
-inline void plan_pair(int ns, int nt, int tpt, int slots, PairPlan* p, int waves = 6) {
+// A split has two tiles at least, or one (`fine`) where that makes no more than 1.5 waves of blocks: a
+// few blocks wait on their own latency (700 particles, RM plain with gradients 25 -> 17 us,
+// exponential core 168 -> 101; 1,000 sources on 50,000 targets, where single tiles make 1.7 waves:
+// 310 us with two, 322 with one).
+inline void plan_pair(int ns, int nt, int tpt, int slots, PairPlan* p, int waves = 6, bool fine = false) {
   p->tpt = tpt;
   p->ntiles = (ns + kBlock - 1) / kBlock;
   p->ns_pad = p->ntiles * kBlock;
@@ -934,7 +939,8 @@ inline void plan_pair(int ns, int nt, int tpt, int slots, PairPlan* p, int waves
   p->nt_pad = p->tblocks * tchunk;
   const long want = (long)waves * (slots > 0 ? slots : 1);
   long nsplit = (want + p->tblocks - 1) / p->tblocks;
-  const long max_split = p->ntiles >= 2 ? p->ntiles / 2 : 1;
+  long max_split = p->ntiles >= 2 ? p->ntiles / 2 : 1;
+  if (fine && 2L * p->ntiles * p->tblocks <= 3L * slots) max_split = p->ntiles;
   if (nsplit > max_split) nsplit = max_split;
   if (nsplit < 1) nsplit = 1;
   p->tiles_per_split = (int)((p->ntiles + nsplit - 1) / nsplit);
@@ -959,7 +965,7 @@ int32_t run_points_points(int ns, const I* sx, const I* sy, const I* sz, const I
   int nb = 0;
   O3G_TRY(occupancy_blocks(PairKernel<C, MODE, GRADS, HAVE_TR, TPT, T, O>::ptr(), kBlock, &nb));
   PairPlan pl;
-  plan_pair(ns, nt, TPT, nb * df.num_sms, &pl, kPairWaves);
+  plan_pair(ns, nt, TPT, nb * df.num_sms, &pl, kPairWaves, true);
   const int nsp = same ? (pl.ns_pad > pl.nt_pad ? pl.ns_pad : pl.nt_pad) : pl.ns_pad;
   size_t bytes = 2 * align_up((size_t)nsp * sizeof(V4<T>));
   if (!same) bytes += align_up((size_t)pl.nt_pad * sizeof(V4<T>));
