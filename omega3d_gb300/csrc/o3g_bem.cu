@@ -5,7 +5,9 @@
 // is solved by
 //   * an FP32 LU factorisation with partial pivoting (row-by-row the same pivot choice
 //     as LAPACK's getrf: largest magnitude, first index on ties), panels of kNb columns:
-//       - k_panel_lu: one cooperative kernel factors the whole kNb-column panel; each
+//       - k_panel_cluster: panels of up to 10,240 rows, 64 columns at a time, in one thread-block
+//         cluster: rows in registers, pivot candidates through distributed shared memory;
+//       - k_panel_lu: taller ones; one cooperative kernel factors the whole kNb-column panel; each
 //         block keeps its slab of rows in shared memory; per column every block publishes
 //         its pivot candidate (the whole row, and the diagonal row if it holds it) and then
 //         a tagged 64-bit key with release semantics; every block polls all keys (relaxed
@@ -14,13 +16,14 @@
 //         Each block updates the next column first, publishes its next candidate, and runs
 //         the rest of the rank-1 update while the other blocks publish;
 //       - k_laswp: the panel's row interchanges applied to the other columns;
-//       - k_trsm_unit_lower: U12 = L11^-1 A12, one warp per column, L11 in shared memory;
+//       - k_trsm_unit_lower, k_left_gemm: U12 = L11^-1 A12, one warp per column, or by the explicit
+//         inverse for the columns beyond the outer panel;
 //       - trailing update A22 -= L21 U12 on the tensor cores (o3g_tcgemm.cu: tcgen05, TF32
 //         products, FP32 sums), two-level blocking so the big updates have k = 512;
 //   * iterative refinement: residuals r = b - A x formed FP64-accurately (double-single
 //     FP32 arithmetic, k_matvec_ds) from the unfactored FP32 matrix and the FP64 iterate,
-//     corrections from the FP32 factors (forward/back substitution in one cooperative kernel
-//     each), until ||r||/||b|| <= tol;
+//     corrections from the FP32 factors (k_trsv: forward/back substitution in one cooperative
+//     kernel each, 512 columns a step by explicit inverses of the diagonal blocks), until ||r||/||b|| <= tol;
 //   * or, without any factorisation, restarted GMRES -- the reference's own solver
 //     (BEM.h:182-202) -- with FP64 Krylov vectors, classical Gram-Schmidt with one
 //     reorthogonalisation, and the same FP64-accurate products (o3g_bem_solve_gmres).
@@ -28,7 +31,6 @@
 // flag that all blocks check, so a fault in the barrier logic ends the kernel instead of
 // hanging.
 #include "o3g_common.cuh"
-
 
 #include <algorithm>
 #include <cmath>
@@ -437,9 +439,8 @@ __global__ void __launch_bounds__(kPanelThreads) k_panel_lu(PanelArgs a) {
 // same winner found by every warp, the rank-1 update of the window.  Per group the pivot rows'
 // later columns are sent to every block, solved against the group's L (U12), and the columns right
 // of the group, held as tiles of 4 rows x 4 columns per thread and chunk, take the rank-8 update: a
-// tile reads 4 multipliers and 4 elements of U for 16 products, and a broadcast read of shared
-// memory costs as much as 32 different words (two full rows per thread: 58 reads for 112
-// products, and this update a fifth of the kernel).
+// tile reads 4 multipliers and 4 elements of U for 16 products (two full rows per thread: 58 reads
+// for 112 products, and this update a fifth of the kernel).
 // Measured (one GB300), 64 columns with 10 warps: 112 -> 86 us (one warp's instructions in series
 // are what is left: 150 a column); factorisation at n = 10,240: 43.2 -> 21.6 ms with the kernels below.  Not kept: full
 // rows in every exchange with a rank-1 update of the whole width per column (2.3 us a column),

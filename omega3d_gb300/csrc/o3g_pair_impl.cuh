@@ -252,9 +252,9 @@ __device__ __forceinline__ void sweep_tile(const V4<T>* sp, const V4<T>* sw, con
 //   Q[0][p] = (-x0, -x1, -y0, -y1)    Q[1][p] = (-z0, -z1, c0, c1)     (c: core parameter)
 //   Q[2][p] = (wx0, wx1, wy0, wy1)    Q[3][p] = (wz0, wz1)             (8 of its 16 bytes)
 // (negated positions turn the separations into adds; the cross products' differences negate
-// a register operand, which costs nothing).  Rows are worth saving: a broadcast read still returns
-// 16 bytes to each of 32 lanes, four cycles of the SM's 128 bytes a cycle, so five rows with one
-// target per thread took 80 of the 104 cycles that four schedulers' pairs take.
+// a register operand, which costs nothing).  A fifth row with the negated strengths costs a load, its
+// registers and with them a resident block: RM compensated takes 80 registers (6 blocks per SM) and
+// 49.7 cycles per pair without it, 90 (5) and 51.5 with it; Gaussian 62.5 and 64.0.
 __device__ __forceinline__ void stage_pair(const V4<float>& s, const V4<float>& w, float4 (*Q)[kBlock / 2], int j) {
   const int p = j >> 1, h = j & 1;
   float* q0 = reinterpret_cast<float*>(&Q[0][p]);
