@@ -1729,7 +1729,6 @@ extern "C" int32_t o3g_bem_create(int64_t n, o3g_bem_t** out) {
   if (e == cudaSuccess) e = o3g::dev_alloc((void**)&h->piv, n * sizeof(int));
   if (e == cudaSuccess) e = o3g::dev_alloc((void**)&h->perm, n * sizeof(int));
   if (e == cudaSuccess) e = o3g::dev_alloc((void**)&h->flags, 64 * sizeof(int));
-  if (e == cudaSuccess) e = o3g::dev_alloc((void**)&h->dinv, dinv_floats((int)n) * sizeof(float));
   if (e != cudaSuccess) {
     (void)cudaGetLastError();
     set_error_cuda("o3g_bem_create: cudaMalloc", e);
@@ -1857,6 +1856,16 @@ extern "C" int32_t o3g_bem_factor(o3g_bem_t* h, void* stream) {
       (void)cudaGetLastError();
       h->tcw = nullptr;
       set_error_cuda("o3g_bem_factor: tensor-core scratch", e);
+      return O3G_ERR_ALLOC;
+    }
+  }
+  // the inverses of the diagonal blocks, 4 KB per row: what is only solved by GMRES has no use for them
+  if (!h->dinv) {
+    const cudaError_t e = o3g::dev_alloc((void**)&h->dinv, dinv_floats(n) * sizeof(float));
+    if (e != cudaSuccess) {
+      (void)cudaGetLastError();
+      h->dinv = nullptr;
+      set_error_cuda("o3g_bem_factor: diagonal inverses", e);
       return O3G_ERR_ALLOC;
     }
   }
