@@ -28,6 +28,8 @@
 #include "o3g_common.cuh"
 #include "o3g_sort.cuh"
 
+#include <cfloat>
+
 namespace o3g {
 
 constexpr int kBlock = 128;  // threads per block == sources per shared tile
@@ -368,14 +370,19 @@ __device__ __forceinline__ void core2(const float2& dx, const float2& dy, const 
       if (GRADS) b3 = __ffma2_rn(__fmul2_rn(r3, f2(-5.f)), s2, __fmul2_rn(dn5, f2(2.f)));
     } else if constexpr (C == CORE_V2) {
       // CoreFunc.h:318-330: rs = (d^4 + c)^(-1/2), r3 = rs sqrt(rs).  d^4 may be subnormal where
-      // r3 is still finite, so rs comes from rsqrtf(); sqrt(rs) = rs rs^(-1/2) with one
-      // Newton step
+      // r3 is still finite, so rs comes from rsqrtf(); sqrt(rs) by one Newton step on z = rs rs^(-1/2)
+      // with the residual rs - z^2, exact in one fma (Heron's step; rms error as sqrtf's).
       const float2 den = __ffma2_rn(r2, r2, cst);
-      const float2 rs = make_float2(rsq<ACC>(den.x), rsq<ACC>(den.y));
-      const float2 y = make_float2(rsq_hw(rs.x), rsq_hw(rs.y));
+      float2 rs = make_float2(rsq<ACC>(den.x), rsq<ACC>(den.y));
+      // Where d^4 overflows (d > 4.3e9: a parked particle, the padding against a far target) rs and r3
+      // are 0, so y stays finite; the corrected rs would be 0 inf there.  Where it underflows with no
+      // core, rs and r3 are infinite, so z stays finite.  (A NaN passes both.)
+      if (ACC) rs = make_float2(den.x > FLT_MAX ? 0.f : rs.x, den.y > FLT_MAX ? 0.f : rs.y);
+      else     rs = make_float2(rs.x > FLT_MAX ? FLT_MAX : rs.x, rs.y > FLT_MAX ? FLT_MAX : rs.y);
+      const float2 y = make_float2(rsq_hw(fmaxf(rs.x, 1e-30f)), rsq_hw(fmaxf(rs.y, 1e-30f)));
       const float2 z = __fmul2_rn(rs, y);
-      const float2 e = __ffma2_rn(make_float2(-z.x, -z.y), y, f2(1.f));
-      r3 = __fmul2_rn(rs, __ffma2_rn(__fmul2_rn(z, f2(0.5f)), e, z));
+      const float2 e = __ffma2_rn(neg2(z), z, rs);
+      r3 = __fmul2_rn(rs, __ffma2_rn(__fmul2_rn(y, f2(0.5f)), e, z));
       if (GRADS) b3 = __fmul2_rn(r3, rs);
     } else {
       static_assert(C == CORE_GAUSS, "");
