@@ -172,12 +172,11 @@ __device__ __forceinline__ void pair_v_ds(const V4<float>& t, const V4<float>& s
 
 // The gradient sums from their parts: a[3..11] by the factor that b3 leaves out, and
 // a[12..14] into the antisymmetric terms: tvx += sz r3, twx -= sy r3, tuy -= sz r3,
-// twy += sx r3, tuz += sy r3, tvz -= sx r3 (Kernels.h:185-191).  NO_ZZ: a[11] was not summed;
-// d . (s x d) = 0, so the sums of b3 d (x) (s x d) have no trace.
-template <int C, bool NO_ZZ = false, class T>
+// twy += sx r3, tuz += sy r3, tvz -= sx r3 (Kernels.h:185-191).  (The sums of b3 d (x) (s x d) have
+// no trace, but zz = -(xx + yy) would carry the rounding of xx and yy, where zz may be small or 0.)
+template <int C, class T>
 __device__ __forceinline__ void fold_grads(T* a) {
   constexpr T k = T(GradScale<C>::value);
-  if (NO_ZZ) a[11] = -(a[3] + a[7]);
   a[3] *= k;
   a[4] = fma(k, a[4], a[14]);
   a[5] = fma(k, a[5], -a[13]);
@@ -255,8 +254,7 @@ __device__ __forceinline__ void sweep_tile(const V4<T>* sp, const V4<T>* sw, con
 //   Q[2][p] = (wx0, wx1, wy0, wy1)    Q[3][p] = (wz0, wz1)             (8 of its 16 bytes)
 // (negated positions turn the separations into adds; the cross products' differences negate
 // a register operand, which costs nothing).  A fifth row with the negated strengths costs a load, its
-// registers and with them a resident block: RM compensated takes 80 registers (6 blocks per SM) and
-// 49.7 cycles per pair without it, 90 (5) and 51.5 with it; Gaussian 62.5 and 64.0.
+// registers and, where they decide it, a resident block.
 __device__ __forceinline__ void stage_pair(const V4<float>& s, const V4<float>& w, float4 (*Q)[kBlock / 2], int j) {
   const int p = j >> 1, h = j & 1;
   float* q0 = reinterpret_cast<float*>(&Q[0][p]);
@@ -392,8 +390,8 @@ __device__ __forceinline__ void core2(const float2& dx, const float2& dy, const 
 }
 
 // one target (tt = (x,x), (y,y), (z,z), (c,c)) against the source pair of q0..q2, wz; a[] as in
-// pair_g / pair_v, one float2 lane per source.  NO_ZZ: a[11] is left out (fold_grads).
-template <int C, bool ACC, bool HAVE_TR, bool GRADS, bool NO_ZZ>
+// pair_g / pair_v, one float2 lane per source.
+template <int C, bool ACC, bool HAVE_TR, bool GRADS>
 __device__ __forceinline__ void pair2(const float2* tt, const float4& q0, const float4& q1, const float4& q2,
                                       const float2& wz, float2* a, const float* gtab) {
   const float2 dx = __fadd2_rn(tt[0], f2lo(q0));
@@ -431,7 +429,7 @@ __device__ __forceinline__ void pair2(const float2* tt, const float4& q0, const 
     a[6] = __ffma2_rn(dy, cx, a[6]);
     a[9] = __ffma2_rn(dz, cx, a[9]);
     a[10] = __ffma2_rn(dz, cy, a[10]);
-    if (!NO_ZZ) a[11] = __ffma2_rn(dz, cz, a[11]);
+    a[11] = __ffma2_rn(dz, cz, a[11]);
   }
 }
 
@@ -443,7 +441,7 @@ __device__ __forceinline__ void sweep_pairs(const float4 (*Q)[kBlock / 2], int p
                                             float2 (*acc)[NA], float (*hi)[NH], float (*lo)[NH], const float* gtab) {
   constexpr bool ACC = (MODE == MODE_COMP);
   constexpr int FOLD = ACC ? 8 : NP;
-  // the compensated loop holds 90 to 96 registers (5 blocks per SM) when it is not unrolled;
+  // the compensated loop with gradients holds 86 to 96 registers (5 blocks per SM) when it is not unrolled;
   // the plain one gains 1 % from two pairs per turn
   constexpr int UN = ACC ? 1 : 2;
 #pragma unroll 1
@@ -454,8 +452,7 @@ __device__ __forceinline__ void sweep_pairs(const float4 (*Q)[kBlock / 2], int p
       const float4 q0 = Q[0][p], q1 = Q[1][p], q2 = Q[2][p];
       const float2 wz = *reinterpret_cast<const float2*>(&Q[3][p]);
 #pragma unroll
-      for (int k = 0; k < TPT; ++k)
-        pair2<C, ACC, HAVE_TR, GRADS, ACC>(tt[k], q0, q1, q2, wz, acc[k], gtab);
+      for (int k = 0; k < TPT; ++k) pair2<C, ACC, HAVE_TR, GRADS>(tt[k], q0, q1, q2, wz, acc[k], gtab);
     }
     if (ACC) {
 #pragma unroll
@@ -463,7 +460,7 @@ __device__ __forceinline__ void sweep_pairs(const float4 (*Q)[kBlock / 2], int p
         float a1[NA];
 #pragma unroll
         for (int c = 0; c < NA; ++c) a1[c] = acc[k][c].x + acc[k][c].y;
-        if (GRADS) fold_grads<C, ACC>(a1);
+        if (GRADS) fold_grads<C>(a1);
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
           const float s = hi[k][c] + a1[c];

@@ -162,7 +162,7 @@ __device__ __forceinline__ void far_pair(const float2* tt, const float4& q0, con
     a[6] = __ffma2_rn(dy, cx, a[6]);
     a[9] = __ffma2_rn(dz, cx, a[9]);
     a[10] = __ffma2_rn(dz, cy, a[10]);
-    if (SRC || !ACC) a[11] = __ffma2_rn(dz, cz, a[11]);   // fold_grads' NO_ZZ otherwise
+    a[11] = __ffma2_rn(dz, cz, a[11]);
   }
 }
 
@@ -196,10 +196,10 @@ __device__ __forceinline__ void leaf(float dx, float dy, float dz, float sx, flo
 }
 
 // the 3 or 12 results from a thread's sums
-template <bool GRADS, bool SRC, bool NO_ZZ = false>
+template <bool GRADS, bool SRC>
 __device__ __forceinline__ void panel_fold(float* a) {
   if (!GRADS) return;
-  fold_grads<CORE_SING, NO_ZZ>(a);
+  fold_grads<CORE_SING>(a);
   if (SRC) {
     a[3] += a[15];
     a[7] += a[15];
@@ -385,7 +385,7 @@ __device__ __forceinline__ void sweep_panels(const float4* __restrict__ tiles, i
           v[c] = a[k][c].x + a[k][c].y;
           a[k][c] = f2(0.f);
         }
-        panel_fold<GRADS, SRC, !SRC>(v);
+        panel_fold<GRADS, SRC>(v);
         fold_tile<NC>(v, hi[k], lo[k]);
       }
     }
