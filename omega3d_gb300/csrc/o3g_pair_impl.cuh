@@ -762,7 +762,8 @@ __global__ void __launch_bounds__(kBlock, PairMinBlocks<C, MODE, GRADS, TPT>::va
 // target's splits (each a contiguous run, then the runs in order: a fixed order, whatever the
 // scheduling), so that few targets with many splits still fill the GPU.  Compensated: (hi, lo)
 // pairs are added in double-single (two-sum), as exact as the double sums it replaces and on
-// FP32 instructions: GB300's FP64 adds made this kernel 389 us at 65,536 targets x 57 splits.
+// FP32 instructions: GB300's FP64 adds made this kernel 389 us at 65,536 targets x 57 splits.  Only a
+// sum that passes FLT_MAX on the way, which two floats cannot come back from, is added in FP64.
 template <int NC, bool ACC, class T, class O>
 __global__ void k_reduce(const T* __restrict__ partial, int nsplit, int nt, int nt_pad, OutPtrs<O> out,
                          const uint32_t* __restrict__ tperm) {
@@ -802,8 +803,20 @@ __global__ void k_reduce(const T* __restrict__ partial, int nsplit, int nt, int 
     }
   }
   O* p = out.p[c] + (tperm ? (int)tperm[idx] : idx);
-  if (ACC) *p = (O)((double)*p + ((double)s + (double)l));
-  else     *p = (O)((T)*p + s);
+  if constexpr (ACC) {
+    double d = (double)s + (double)l;
+    if (!(fabsf(s) <= FLT_MAX && fabsf(l) <= FLT_MAX)) {
+      d = 0.0;
+      for (int k = 0; k < nsplit; ++k) {
+        const T* q = partial + ((size_t)k * 2 * NC + c) * nt_pad + idx;
+        d += (double)q[0];
+        d += (double)q[(size_t)NC * nt_pad];
+      }
+    }
+    *p = (O)((double)*p + d);
+  } else {
+    *p = (O)((T)*p + s);
+  }
 }
 template <int NC, bool ACC, class T, class O>
 void launch_reduce(const T* partial, int nsplit, int nt, int nt_pad, const OutPtrs<O>& out, const uint32_t* tperm,
