@@ -65,9 +65,9 @@ __device__ __forceinline__ dsf ds_mul(dsf x, dsf y) {
   return {p, __fmaf_rn(x.l, y.h, __fmaf_rn(x.h, y.l, __fmaf_rn(x.h, y.h, -p)))};
 }
 // Powers of x^(-1/2) from the hardware estimate y and its residual r = 1 - x y^2 (from exact
-// products; below 2^-21, so the neglected 15/8 r^2 is below 2^-41): x^(-3/2) = y^3 (1 + 3/2 r) and x^(-1)
-// = y^2 (1 + r), unnormalised.  Renormalising the root, its square and its cube took twice the
-// operations.
+// products; below 2^-21): x^(-3/2) = y^3 (1 + 3/2 r + 15/8 r^2) and x^(-1) = y^2 (1 + r + r^2),
+// unnormalised, the next terms below 2^-62.  Renormalising the root, its square and its cube took
+// twice the operations.
 struct dsrs {
   dsf r3, r2;
 };
@@ -78,9 +78,10 @@ __device__ __forceinline__ dsrs ds_rsqrt32(dsf x) {
   r = __fmaf_rn(-x.h, y2.l, r);
   r = __fmaf_rn(-x.l, y2.h, r);
   dsrs o;
-  o.r2 = {y2.h, __fmaf_rn(y2.h, r, y2.l)};
+  o.r2 = {y2.h, __fmaf_rn(y2.h, __fmaf_rn(r, r, r), y2.l)};
   const float c = __fmul_rn(y2.h, y);
-  o.r3 = {c, __fmaf_rn(c, __fmul_rn(1.5f, r), __fmaf_rn(y2.l, y, __fmaf_rn(y2.h, y, -c)))};
+  const float q = __fmul_rn(r, __fmaf_rn(1.875f, r, 1.5f));
+  o.r3 = {c, __fmaf_rn(c, q, __fmaf_rn(y2.l, y, __fmaf_rn(y2.h, y, -c)))};
   return o;
 }
 // p u - q v (p, q double-single, u, v float), unnormalised: the sum hi + lo is the value
