@@ -295,7 +295,9 @@ int32_t o3g_bem_set_block(o3g_bem_t* h, int64_t rstart, int64_t nrows, int64_t c
 int32_t o3g_bem_factor(o3g_bem_t* h, void* stream);
 /* solve A x = b (BEM.h:202): b, x (float) and x64 (double, nullable) in `mem` memory;
  * returns the refinement count and the final FP64 relative residual; O3G_ERR_NOT_CONVERGED
- * when tol is not reached within max_iter refinements (x still holds the best iterate) */
+ * when tol is not reached within max_iter refinements (x still holds the best iterate).  A system that
+ * does not get there with the inverses of the factors' 512-column diagonal blocks is refined once more from
+ * the start with those of the 128-column ones, up to max_iter again; iters counts the last of the two */
 int32_t o3g_bem_solve(o3g_bem_t* h, const float* b, float* x, double* x64, int32_t mem, double tol,
                       int32_t max_iter, int32_t* iters, double* relres, void* stream);
 /* solve A x = b without factorising: restarted GMRES(restart), the reference's own method

@@ -1395,27 +1395,31 @@ struct TrsvArgs {
   Barrier bar;
 };
 
-// L w = y (LOWER) or U x = w for K right-hand sides, kDb columns at a time.  What bounds it is
+// L w = y (LOWER) or U x = w for K right-hand sides, STEP columns at a time.  What bounds it is
 // latency: per step the segment is multiplied by its block's inverse (a few rows per CUDA block),
 // a grid barrier, the other rows take the segment's columns of the factor (each block its share
 // of rows), a grid barrier.  The factor's elements are loaded before the barriers they do not
-// depend on.  kDb 512: 128 columns a step, every block applying the whole 128 x 128 inverse for
+// depend on.  STEP is kDb: 128 columns a step, every block applying the whole 128 x 128 inverse for
 // itself, took 8-10 us a step; 1024 would double the memory of the inverses (n kDb 8 bytes) to
-// save a few barriers.  A whole solve with 3 refinements, before and after: n = 640 0.44 -> 0.36
+// save a few barriers.  STEP kNb uses the kNb x kNb inverses alone, for systems that the bigger ones
+// are too inaccurate for (refine_passes).  A whole solve with 3 refinements, before and after: n = 640 0.44 -> 0.36
 // ms, 2,560 0.99 -> 0.56, 10,240 5.41 -> 1.59, 15,360 8.12 -> 2.56; the inverses cost 0.2 ms per factorisation.
-constexpr int kTrRows = 64, kTrChunks = kSolveThreads / kTrRows, kTrCols = kDb / kTrChunks;
-constexpr size_t trsv_smem(int K) { return (size_t)K * (kDb + kSolveThreads) * sizeof(float); }
-template <int K, bool LOWER>
+constexpr int kTrRows = 64, kTrChunks = kSolveThreads / kTrRows;
+constexpr size_t trsv_smem(int K, int step) { return (size_t)K * (step + kSolveThreads) * sizeof(float); }
+template <int K, bool LOWER, int STEP>
 __global__ void __launch_bounds__(kSolveThreads) k_trsv(TrsvArgs a) {
+  static_assert(kDb % STEP == 0 && STEP % kNb == 0, "whole inverses");
+  constexpr int kTrCols = STEP / kTrChunks, kColThreads = kSolveThreads / 4;
   extern __shared__ float trsm[];
-  float* yd = trsm;               // [K][kDb]
-  float* part = trsm + K * kDb;   // [K][kTrChunks][kTrRows]
+  float* yd = trsm;                // [K][STEP]
+  float* part = trsm + K * STEP;   // [K][kTrChunks][kTrRows]
   const int G = gridDim.x, tid = threadIdx.x, n = a.n;
-  const int nblk = (n + kDb - 1) / kDb;
+  const int nblk = (n + STEP - 1) / STEP;
   for (int s = 0; s < nblk; ++s) {
     const int b = LOWER ? s : nblk - 1 - s;
-    const int k0 = b * kDb, jb = min(kDb, n - k0);
-    const float* D = a.dinv + (size_t)b * 2 * kDb * kDb + (LOWER ? 0 : (size_t)kDb * kDb);
+    const int k0 = b * STEP, jb = min(STEP, n - k0);
+    const float* D = a.dinv + (size_t)(k0 / kDb) * 2 * kDb * kDb + (size_t)(k0 % kDb) * (kDb + 1) +
+                     (LOWER ? 0 : (size_t)kDb * kDb);
     // this block's rows of the update, and their elements for the first kTrRows of them
     const int lo = LOWER ? k0 + jb : 0, hi = LOWER ? n : k0;
     const int share = (hi - lo + G - 1) / G;
@@ -1440,8 +1444,8 @@ __global__ void __launch_bounds__(kSolveThreads) k_trsv(TrsvArgs a) {
 #pragma unroll
       for (int c = 0; c < K; ++c) v[c] = 0.f;
 #pragma unroll
-      for (int h = 0; h < kDb / (kSolveThreads / 4); ++h) {
-        const int col = (tid >> 2) + h * (kSolveThreads / 4);
+      for (int h = 0; h < (STEP + kColThreads - 1) / kColThreads; ++h) {
+        const int col = (tid >> 2) + h * kColThreads;
         const bool in = row < d1 && col < jb && (LOWER ? col <= row : col >= row);
         const float dv = in ? __ldg(D + (size_t)col * kDb + row) : 0.f;
         if (in)
@@ -1468,7 +1472,7 @@ __global__ void __launch_bounds__(kSolveThreads) k_trsv(TrsvArgs a) {
     if (!grid_sync(a.bar)) return;
     for (int e = tid; e < K * jb; e += kSolveThreads) {
       const int c = e / jb, k = e - c * jb;
-      yd[c * kDb + k] = __ldcg(a.out + (size_t)c * n + k0 + k);
+      yd[c * STEP + k] = __ldcg(a.out + (size_t)c * n + k0 + k);
     }
     for (int r0 = i0; r0 < i1; r0 += kTrRows) {
       if (r0 > i0) load(r0 + r);
@@ -1479,7 +1483,7 @@ __global__ void __launch_bounds__(kSolveThreads) k_trsv(TrsvArgs a) {
 #pragma unroll
       for (int t = 0; t < kTrCols; ++t)
 #pragma unroll
-        for (int c = 0; c < K; ++c) v[c] = fmaf(m[t], q * kTrCols + t < jb ? yd[c * kDb + q * kTrCols + t] : 0.f, v[c]);
+        for (int c = 0; c < K; ++c) v[c] = fmaf(m[t], q * kTrCols + t < jb ? yd[c * STEP + q * kTrCols + t] : 0.f, v[c]);
 #pragma unroll
       for (int c = 0; c < K; ++c) part[(c * kTrChunks + q) * kTrRows + r] = v[c];
       __syncthreads();
@@ -1498,32 +1502,44 @@ __global__ void __launch_bounds__(kSolveThreads) k_trsv(TrsvArgs a) {
   }
 }
 
-// both solves for K right-hand sides: lower.y -> lower.out = upper.y -> upper.out
-template <int K>
+// both solves for K right-hand sides, `step` (kDb or kNb) columns at a time: lower.y -> lower.out =
+// upper.y -> upper.out
+template <int K, int STEP>
 static int32_t launch_trsv(const TrsvArgs& lower, const TrsvArgs& upper, int G, cudaStream_t st) {
-  const void* ks[2] = {(const void*)&k_trsv<K, true>, (const void*)&k_trsv<K, false>};
+  const void* ks[2] = {(const void*)&k_trsv<K, true, STEP>, (const void*)&k_trsv<K, false, STEP>};
   TrsvArgs args[2] = {lower, upper};
+  const size_t smem = trsv_smem(K, STEP);
   for (int e = 0; e < 2; ++e) {
     void* av[] = {&args[e]};
-    O3G_CUDA_TRY(cudaFuncSetAttribute(ks[e], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trsv_smem(K)));
+    O3G_CUDA_TRY(cudaFuncSetAttribute(ks[e], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     O3G_CUDA_TRY(zero_barrier(lower.bar.err, st));
-    O3G_CUDA_TRY(cudaLaunchCooperativeKernel(ks[e], dim3(G), dim3(kSolveThreads), av, trsv_smem(K), st));
+    O3G_CUDA_TRY(cudaLaunchCooperativeKernel(ks[e], dim3(G), dim3(kSolveThreads), av, smem, st));
   }
   note_launch(2);
   return O3G_OK;
 }
-static int32_t trsv(int K, const TrsvArgs& lower, const TrsvArgs& upper, int G, cudaStream_t st) {
+template <int K>
+static int32_t launch_trsv(int step, const TrsvArgs& lower, const TrsvArgs& upper, int G, cudaStream_t st) {
+  return step == kDb ? launch_trsv<K, kDb>(lower, upper, G, st) : launch_trsv<K, kNb>(lower, upper, G, st);
+}
+static int32_t trsv(int K, int step, const TrsvArgs& lower, const TrsvArgs& upper, int G, cudaStream_t st) {
   switch (K) {
-    case 1: return launch_trsv<1>(lower, upper, G, st);
-    case 2: return launch_trsv<2>(lower, upper, G, st);
-    case 3: return launch_trsv<3>(lower, upper, G, st);
-    case 4: return launch_trsv<4>(lower, upper, G, st);
-    case 5: return launch_trsv<5>(lower, upper, G, st);
-    case 6: return launch_trsv<6>(lower, upper, G, st);
-    case 7: return launch_trsv<7>(lower, upper, G, st);
-    default: return launch_trsv<8>(lower, upper, G, st);
+    case 1: return launch_trsv<1>(step, lower, upper, G, st);
+    case 2: return launch_trsv<2>(step, lower, upper, G, st);
+    case 3: return launch_trsv<3>(step, lower, upper, G, st);
+    case 4: return launch_trsv<4>(step, lower, upper, G, st);
+    case 5: return launch_trsv<5>(step, lower, upper, G, st);
+    case 6: return launch_trsv<6>(step, lower, upper, G, st);
+    case 7: return launch_trsv<7>(step, lower, upper, G, st);
+    default: return launch_trsv<8>(step, lower, upper, G, st);
   }
 }
+// The refinement's passes: with the kDb solves, and, for a system that does not reach its tolerance with
+// them, once more from the start with the kNb solves (the same solves when n <= kNb).  An explicit
+// inverse's error grows with its block's condition: unit lower triangles whose inverses grow to 1e4 over 512
+// columns take up to 3 times the refinements or none are enough, where kNb columns converge.
+static int refine_passes(int n) { return n > kNb ? 2 : 1; }
+static int refine_step(int pass) { return pass == 0 ? kDb : kNb; }
 // one block per SM (1024 threads and at most 48 KB each: always resident together)
 static int trsv_grid(int num_sms) { return num_sms; }
 
@@ -2065,26 +2081,30 @@ extern "C" int32_t o3g_bem_solve(o3g_bem_t* h, const float* b, float* x, double*
   int it = 0;
   KernelTimer& tm = thread_timer();
   tm.begin(st);
-  for (it = 0; it <= max_iter; ++it) {
-    // r = b - A x in FP64-accurate double-single arithmetic (r = b at x = 0)
-    if (it > 0) {
-      k_split_f64<<<nrb, 256, 0, st>>>(xd, xh, xl, n);
-      k_matvec_ds<<<dim3(nrb, ncb), 256, 0, st>>>(h->A, ld, n, xh, xl, part);
+  for (int pass = 0; pass < refine_passes(n); ++pass) {
+    if (pass > 0) O3G_CUDA_TRY(cudaMemsetAsync(xd, 0, (size_t)n * 8, st));
+    for (it = 0; it <= max_iter; ++it) {
+      // r = b - A x in FP64-accurate double-single arithmetic (r = b at x = 0)
+      if (it > 0) {
+        k_split_f64<<<nrb, 256, 0, st>>>(xd, xh, xl, n);
+        k_matvec_ds<<<dim3(nrb, ncb), 256, 0, st>>>(h->A, ld, n, xh, xl, part);
+        note_launch(2);
+      }
+      k_matvec_finish<<<nrb, 256, 0, st>>>(part, it > 0 ? ncb : 0, n, bd, rd, nrm);
+      note_launch();
+      O3G_CUDA_TRY(cudaMemcpyAsync(hn.data(), nrm, (size_t)nrb * 8, cudaMemcpyDeviceToHost, st));
+      O3G_CUDA_TRY(cudaStreamSynchronize(st));
+      double rr = 0.0;
+      for (int k = 0; k < nrb; ++k) rr += hn[k];
+      if (it == 0) bnorm = std::sqrt(rr);
+      rel = bnorm > 0.0 ? std::sqrt(rr) / bnorm : std::sqrt(rr);
+      if (rel <= tol || it == max_iter || (!std::isfinite(rel) && pass + 1 < refine_passes(n))) break;
+      k_permute_to_float<<<nrb, 256, 0, st>>>(rd, h->perm, y, n);
+      O3G_TRY(trsv(1, refine_step(pass), ta, tb, G, st));
+      k_axpy_f2d<<<nrb, 256, 0, st>>>(xd, y, n);
       note_launch(2);
     }
-    k_matvec_finish<<<nrb, 256, 0, st>>>(part, it > 0 ? ncb : 0, n, bd, rd, nrm);
-    note_launch();
-    O3G_CUDA_TRY(cudaMemcpyAsync(hn.data(), nrm, (size_t)nrb * 8, cudaMemcpyDeviceToHost, st));
-    O3G_CUDA_TRY(cudaStreamSynchronize(st));
-    double rr = 0.0;
-    for (int k = 0; k < nrb; ++k) rr += hn[k];
-    if (it == 0) bnorm = std::sqrt(rr);
-    rel = bnorm > 0.0 ? std::sqrt(rr) / bnorm : std::sqrt(rr);
-    if (rel <= tol || it == max_iter) break;
-    k_permute_to_float<<<nrb, 256, 0, st>>>(rd, h->perm, y, n);
-    O3G_TRY(trsv(1, ta, tb, G, st));
-    k_axpy_f2d<<<nrb, 256, 0, st>>>(xd, y, n);
-    note_launch(2);
+    if (rel <= tol) break;
   }
   tm.end(st);
   int fl = 0;
@@ -2690,25 +2710,37 @@ extern "C" int32_t o3g_bem_solve_many(o3g_bem_t* h, int32_t nrhs, const float* B
     up = lo;
     up.y = w; up.out = y;
     std::vector<double> rr, bnorm(K, 0.0), rel(K, 1.0);
-    unsigned active = (1u << K) - 1u;
+    unsigned todo = (1u << K) - 1u;   // the columns of this pass
     std::vector<int> it_of(K, max_iter);
-    for (int it = 0; it <= max_iter; ++it) {
-      O3G_TRY(matvec_multi(h, K, it > 0 ? xin : none, bin, rout, xh, xl, part, nrm, &rr, st));
-      for (int c = 0; c < K; ++c) {
-        if (it == 0) bnorm[c] = std::sqrt(rr[c]);
-        if (!((active >> c) & 1u)) continue;
-        rel[c] = bnorm[c] > 0.0 ? std::sqrt(rr[c]) / bnorm[c] : std::sqrt(rr[c]);
-        if (rel[c] <= tol || it == max_iter) {
-          active &= ~(1u << c);
-          it_of[c] = it;
+    for (int pass = 0; pass < refine_passes(n) && todo; ++pass) {
+      unsigned active = todo;
+      const bool last = pass + 1 == refine_passes(n);
+      bool finite = true;
+      for (int c = 0; c < K && pass > 0; ++c)
+        if ((todo >> c) & 1u) O3G_CUDA_TRY(cudaMemsetAsync(xd + (size_t)c * n, 0, (size_t)n * 8, st));
+      for (int it = 0; it <= max_iter; ++it) {
+        O3G_TRY(matvec_multi(h, K, it > 0 || pass > 0 ? xin : none, bin, rout, xh, xl, part, nrm, &rr, st));
+        for (int c = 0; c < K; ++c) {
+          if (it == 0 && pass == 0) bnorm[c] = std::sqrt(rr[c]);
+          if (!((active >> c) & 1u)) continue;
+          rel[c] = bnorm[c] > 0.0 ? std::sqrt(rr[c]) / bnorm[c] : std::sqrt(rr[c]);
+          if (!std::isfinite(rel[c])) finite = false;
+          if (rel[c] <= tol || it == max_iter || (!std::isfinite(rel[c]) && !last)) {
+            active &= ~(1u << c);
+            it_of[c] = it;
+          }
         }
+        if (!active) break;
+        k_permute_to_float_multi<<<dim3(nrb, K), 256, 0, st>>>(rd, h->perm, y, n, active);
+        note_launch();
+        O3G_TRY(trsv(K, refine_step(pass), lo, up, G, st));
+        k_axpy_f2d<<<(unsigned)((knn + 255) / 256), 256, 0, st>>>(xd, y, (int)knn);
+        note_launch();
       }
-      if (!active) break;
-      k_permute_to_float_multi<<<dim3(nrb, K), 256, 0, st>>>(rd, h->perm, y, n, active);
-      note_launch();
-      O3G_TRY(trsv(K, lo, up, G, st));
-      k_axpy_f2d<<<(unsigned)((knn + 255) / 256), 256, 0, st>>>(xd, y, (int)knn);
-      note_launch();
+      // (an infinite inverse spoils the finished columns too: 0 inf)
+      if (finite)
+        for (int c = 0; c < K; ++c)
+          if (rel[c] <= tol) todo &= ~(1u << c);
     }
     int fl = 0;
     O3G_CUDA_TRY(cudaMemcpyAsync(&fl, h->flags, sizeof(int), cudaMemcpyDeviceToHost, st));
