@@ -91,13 +91,15 @@ int32_t o3g_launch_count(uint64_t* n);
 int32_t o3g_alloc_count(uint64_t* n);
 
 /* Wait test.  Some kernels wait on the device for one another's progress, each wait
- * bounded: the grid barriers of the BEM panel factorisation and triangular solves, and the
- * dependency waits of the particle split.  A wait that runs out sets an error word, every
+ * bounded: the grid barriers of the BEM panel factorisation and triangular solves, the exchanges
+ * of its panels in one thread-block cluster, and the dependency waits of the particle split.  A wait that runs out sets an error word, every
  * other wait then returns at once, the kernels end, and the call returns O3G_ERR_TIMEOUT
  * with the device still usable.  With enable != 0 (process-wide, until called with 0)
  * those waits are given a condition that nothing fulfils (a barrier count one above the
  * number of blocks, a flag nothing sets) and a limit of about a millisecond, so that tests
- * can see them run out.  A split that runs out leaves the particles unchanged. */
+ * can see them run out.  With 1 the panels take the kernel with grid barriers, with 2 the
+ * one with exchanges in a cluster where they fit it.  A split that runs out leaves the
+ * particles unchanged. */
 int32_t o3g_debug_wait_test(int32_t enable);
 
 /* Measures the FP32 FMA throughput of the current device (TFLOP/s, counting an FMA as

@@ -462,6 +462,7 @@ struct ClusterPanelArgs {
   int* singular;
   int* err;               // set when a wait runs out
   const float* u;         // the rows of U above the sub-panel, (c - k0) x w column-major (k_panel_next)
+  int test;               // the wait test: every wait runs out
 };
 template <int W, int NT> struct ClusterShared {
   static constexpr int RPT = kCpRows, warps = NT / 32;
@@ -476,7 +477,7 @@ template <int W, int NT> struct ClusterShared {
   float4 turn[2][rows_n];                         // the next group's columns, from tiles to rows
   uint2 head[2][kCpGroup][kCpMax];                // candidates' |value| bits + 1 (0: none) and positions
   uint2 whead[warps];                             // the warps'
-  unsigned long long bar[3];                      // mbarriers: a column's candidates (by parity), a group's rows
+  unsigned long long bar[4];                      // mbarriers: a column's candidates (by parity), a group's rows, none (wait test)
   int prow[kCpGroup];                             // the group's k-th pivot row, if it is one of this block's (-1)
   float done[W * RPT * NT];                       // the finished columns
 };
@@ -526,24 +527,38 @@ __device__ __forceinline__ int best_lane(unsigned key, unsigned pos, unsigned& m
   }
   return __ffs(eq) - 1;
 }
-// waits (bounded) for the mbarrier's phase; every thread for itself.  All blocks of a cluster are
-// resident, so it can only run out if one of them faults.
-__device__ __forceinline__ bool cluster_wait(unsigned bar, unsigned parity, int* err) {
+__device__ __forceinline__ unsigned cluster_test(unsigned bar, unsigned parity) {
+  unsigned done;
+  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+               : "=r"(done)
+               : "r"(bar), "r"(parity)
+               : "memory");
+  return done;
+}
+// suspends for up to 1 us
+__device__ __forceinline__ unsigned cluster_try(unsigned bar, unsigned parity) {
+  unsigned done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 1000;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(done)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return done;
+}
+// A warp's wait (bounded) for the phase of mbarrier `bar`.  All blocks of a cluster are resident, so it can
+// only run out if one of them faults, or in the wait test, where it polls `never` (parity 0: a phase that
+// nothing completes) for a short time.  A wait that runs out sets the error word, gives the copies in flight to
+// this block time to land (in the wait test they all do) and returns false in the whole warp.
+constexpr unsigned kClusterTries = 1u << 21, kClusterTestTries = 1u << 6, kClusterDrain = 1u << 16;
+__device__ __forceinline__ bool cluster_wait(unsigned bar, unsigned parity, int* err, unsigned never) {
+  const unsigned wb = never ? never : bar, limit = never ? kClusterTestTries : kClusterTries;
   unsigned done = 0u;
-  // polled first (a suspended wait wakes up later), then with suspensions of up to 1 us
-  for (int it = 0; it < 4096 && !done; ++it)
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(done)
-                 : "r"(bar), "r"(parity)
-                 : "memory");
-  for (unsigned it = 0; it < (1u << 21) && !done; ++it)
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 1000;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(bar), "r"(parity)
-        : "memory");
-  if (done) return true;
+  for (int it = 0; it < 4096 && !done; ++it) done = cluster_test(wb, parity);   // (a suspended wait wakes up later)
+  for (unsigned it = 0; it < limit && !done; ++it) done = cluster_try(wb, parity);
+  if (__all_sync(0xffffffffu, done != 0u)) return true;
   atomicExch(err, 1);
+  for (unsigned it = 0; it < kClusterDrain && !cluster_try(bar, parity); ++it) {}
+  __syncwarp();
   return false;
 }
 
@@ -594,6 +609,7 @@ __device__ __forceinline__ void panel_group(const ClusterPanelArgs& a, ClusterSh
   const int cg = a.c + g0, gp = (g0 / B) & 1;
   const int nb = min(B, a.w - g0);
   const unsigned peer = cluster_map(&sh, (unsigned)(lane & 15) < C ? lane & 15 : 0);
+  const unsigned never = a.test ? (unsigned)__cvta_generic_to_shared(&sh.bar[3]) : 0u;
   unsigned win = 0u;   // the winners' blocks, 4 bits each
   // one copy of the column's code (unrolled eight times, fetching it took longer than running
   // it): the current column is always x[.][0], and the group's window turns by one per column
@@ -632,18 +648,22 @@ __device__ __forceinline__ void panel_group(const ClusterPanelArgs& a, ClusterSh
         const uint2 hw = lane < NT / 32 ? sh.whead[lane] : make_uint2(0u, full);
         const int wi = best_lane(hw.x, hw.y, m);
         const uint2 hs = make_uint2(m, __shfl_sync(full, hw.y, wi));
-        if (lane == 0) cluster_expect((unsigned)__cvta_generic_to_shared(&sh.bar[par]), C * (B * 4 + 8));
+        // (after a wait that ran out nothing is sent or armed any more: the phases before may be open)
+        if (lane == 0 && !dead) cluster_expect((unsigned)__cvta_generic_to_shared(&sh.bar[par]), C * (B * 4 + 8));
         const int to = lane & 15, h = lane >> 4;
-        if (to < (int)C) {
+        if (to < (int)C && !dead) {
           const unsigned bar = peer + off(&sh.bar[par]);
           cluster_send4(peer + off(&sh.xch[gp][jj][rank][4 * h]), reinterpret_cast<const float4*>(sh.cand[wi])[h], bar);
           if (h == 0) cluster_send(peer + off(&sh.head[gp][jj][rank]), hs.x, hs.y, bar);
         }
-      } else {
+      } else if (!dead) {
         asm volatile("bar.arrive 1, %0;" ::"n"(NT) : "memory");
+      } else {
+        // no exchange holds this warp back: it waits here, or it would arrive twice in one turn
+        asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory");
       }
       const unsigned bar = (unsigned)__cvta_generic_to_shared(&sh.bar[par]);
-      if (!dead) dead = !cluster_wait(bar, (unsigned)((g0 + jj) >> 1) & 1u, a.err);
+      if (!dead) dead = !cluster_wait(bar, (unsigned)((g0 + jj) >> 1) & 1u, a.err, never);
       // the cluster's pivot, found by every warp alike
       const uint2 hd = lane < (int)C ? sh.head[gp][jj][lane] : make_uint2(0u, full);
       const unsigned wb = (unsigned)best_lane(hd.x, hd.y, m) % kCpMax;
@@ -716,7 +736,7 @@ __device__ __forceinline__ void panel_group(const ClusterPanelArgs& a, ClusterSh
       const int e = pos[q] - cg;
       if ((unsigned)e < (unsigned)B) sh.prow[e] = (tid + q * NT) | (g0 << 16);
     }
-    if (tid == 0) cluster_expect((unsigned)__cvta_generic_to_shared(&sh.bar[2]), B * (R - g0) * 4);
+    if (tid == 0 && !dead) cluster_expect((unsigned)__cvta_generic_to_shared(&sh.bar[2]), B * (R - g0) * 4);
     __syncthreads();
     // their columns right of the group to every block, by the warps that hold them
     const unsigned barb = off(&sh.bar[2]);
@@ -739,7 +759,7 @@ __device__ __forceinline__ void panel_group(const ClusterPanelArgs& a, ClusterSh
       __syncwarp();
       // 8 lanes per destination
       const int c = lane & 7;
-      if (c >= g && c < PanelTile<W>::NCH) {
+      if (!dead && c >= g && c < PanelTile<W>::NCH) {
         const float4 v = *reinterpret_cast<const float4*>(&sh.own[k][8 * c + 4 * cb]);
         for (unsigned to = lane >> 3; to < C; to += 4) {
           const unsigned dst = cluster_map(&sh, to);
@@ -760,7 +780,7 @@ __device__ __forceinline__ void panel_group(const ClusterPanelArgs& a, ClusterSh
     for (int k = 0; k < B; ++k) sh.done[((g0 + k) * RPT + q) * NT + tid] = x[q][k];
   if (!more) return;
   const unsigned bar = (unsigned)__cvta_generic_to_shared(&sh.bar[2]);
-  if (!dead) dead = !cluster_wait(bar, (unsigned)gp, a.err);
+  if (!dead) dead = !cluster_wait(bar, (unsigned)gp, a.err, never);
   // U12 = L11^-1 A12 of the group, a thread per column; L11 from the pivots' windows
   if (tid >= g0 && tid < R) {
     float uu[B];
@@ -838,7 +858,7 @@ __global__ void __launch_bounds__(NT, 1) k_panel_cluster(const ClusterPanelArgs 
   if (tid < kCpGroup) sh.prow[tid] = -1;
   if (tid == 0) {
 #pragma unroll
-    for (int b = 0; b < 3; ++b)
+    for (int b = 0; b < 4; ++b)
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((unsigned)__cvta_generic_to_shared(&sh.bar[b])) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -1933,15 +1953,16 @@ extern "C" int32_t o3g_bem_factor(o3g_bem_t* h, void* stream) {
     for (int k0 = K0; k0 < K1; k0 += kNb) {
       const int jb = std::min(kNb, K1 - k0);
       const int m = n - k0;
-      // the debug wait test (o3g_debug_wait_test) needs a kernel that polls
+      // (the wait test of the grid barriers, o3g_debug_wait_test(1), takes the kernel that polls them)
       ClusterPlan cp;
-      if (!wait_test_on()) cp = cluster_for(m, plans);
+      if (!wait_test_on() || wait_test_clusters()) cp = cluster_for(m, plans);
       if (cp.kernel) {
         for (int c = k0; c < k0 + jb; c += kCpW) {
           ClusterPanelArgs ca;
           ca.A = h->LU; ca.ld = ld; ca.n = n; ca.k0 = k0; ca.c = c; ca.w = std::min(kCpW, k0 + jb - c);
           ca.piv = h->piv; ca.singular = h->flags + 1; ca.err = h->flags;
           ca.u = linv;
+          ca.test = wait_test_clusters() ? 1 : 0;
           if (c > k0) {
             k_panel_next<<<(n - c + kNextRows - 1) / kNextRows, 256, sizeof(PanelNextShared), st>>>(h->LU, ld, n, k0, c - k0,
                                                                                                ca.w, linv);
@@ -2002,7 +2023,7 @@ extern "C" int32_t o3g_bem_factor(o3g_bem_t* h, void* stream) {
   O3G_CUDA_TRY(cudaMemcpyAsync(piv.data(), h->piv, n * sizeof(int), cudaMemcpyDeviceToHost, st));
   O3G_CUDA_TRY(cudaStreamSynchronize(st));
   if (fl[0]) {
-    set_error("o3g_bem_factor: a grid barrier timed out");
+    set_error("o3g_bem_factor: a grid barrier or a panel's exchange timed out");
     return O3G_ERR_TIMEOUT;
   }
   if (fl[4]) {

@@ -95,8 +95,10 @@ int32_t tc_gemm_sub(int m, int n, int k, const float* A, long long lda, const fl
 
 // wait test (o3g_debug_wait_test): when on, the bounded device-side waits of the BEM
 // factorisation and solves and of the particle split wait for a condition nothing fulfils,
-// with a short limit, so that they run out and the call returns O3G_ERR_TIMEOUT
+// with a short limit, so that they run out and the call returns O3G_ERR_TIMEOUT; the panels'
+// grid barriers, or (wait_test_clusters) their exchanges in a cluster
 bool wait_test_on();
+bool wait_test_clusters();
 
 // ------------------------------------------------------------------------------
 // vector types

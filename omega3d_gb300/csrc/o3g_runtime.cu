@@ -115,6 +115,7 @@ void note_launch(int n) { g_launches += (unsigned long long)n; }
 
 static std::atomic<int> g_wait_test{0};
 bool wait_test_on() { return g_wait_test.load() != 0; }
+bool wait_test_clusters() { return g_wait_test.load() == 2; }
 
 static std::atomic<unsigned long long> g_allocs{0};
 // The pool behind dev_alloc_async, one per device.  The device's default pool returns its memory to
@@ -236,7 +237,7 @@ int32_t o3g_flops_per_pair(int32_t core, int32_t grads, int32_t have_tr) {
 }
 
 int32_t o3g_debug_wait_test(int32_t enable) {
-  o3g::g_wait_test.store(enable != 0 ? 1 : 0);
+  o3g::g_wait_test.store(enable == 2 ? 2 : enable != 0 ? 1 : 0);
   return O3G_OK;
 }
 
