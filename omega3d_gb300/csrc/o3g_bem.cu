@@ -2011,9 +2011,11 @@ extern "C" int32_t o3g_bem_factor(o3g_bem_t* h, void* stream) {
     k_diag_inverses<<<dim3((n + kNb - 1) / kNb, 2, kInvSplit), 256, kBlockBytes, st>>>(h->LU, ld, n, h->dinv);
     O3G_CUDA_TRY(cudaFuncSetAttribute(k_diag_merge, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ProdShared)));
     const int nbig = (n + kDb - 1) / kDb;
-    for (int d = 1; d < kDbSub && n > d * kNb; ++d)
+    note_launch();
+    for (int d = 1; d < kDbSub && n > d * kNb; ++d) {
       k_diag_merge<<<dim3(nbig * (kDbSub - d), 2, kNb / kProdCols), 256, sizeof(ProdShared), st>>>(h->LU, ld, n, h->dinv, d);
-    note_launch(kDbSub);
+      note_launch();
+    }
   }
   tm.end(st);
   O3G_CUDA_TRY(cudaGetLastError());
