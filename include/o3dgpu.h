@@ -90,6 +90,12 @@ int32_t o3g_launch_count(uint64_t* n);
  * handles, and the scratch of split, merge, reflection and shedding. */
 int32_t o3g_alloc_count(uint64_t* n);
 
+/* Split, merge, shedding and clear_inner_layer keep up to 1 GiB of their scratch per device
+ * between calls.  This gives what is not in use on the current device back to the system, for
+ * a caller whose own allocator runs short (an allocation of this library that fails does so by
+ * itself).  Waits for the device's work; may be called at any time, from any thread. */
+int32_t o3g_release_scratch(void);
+
 /* Wait test.  Some kernels wait on the device for one another's progress, each wait
  * bounded: the grid barriers of the BEM panel factorisation and triangular solves, the exchanges
  * of its panels in one thread-block cluster, and the dependency waits of the particle split.  A wait that runs out sets an error word, every

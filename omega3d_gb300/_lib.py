@@ -78,6 +78,8 @@ def _declare(l):
     l.o3g_last_kernel_ms.argtypes = [P]
     l.o3g_launch_count.restype = c_i32
     l.o3g_launch_count.argtypes = [P]
+    l.o3g_release_scratch.restype = c_i32
+    l.o3g_release_scratch.argtypes = []
     l.o3g_alloc_count.restype = c_i32
     l.o3g_alloc_count.argtypes = [P]
     l.o3g_debug_wait_test.restype = c_i32
@@ -211,6 +213,12 @@ def lib():
 def check(status, where):
     if status != O3G_OK:
         raise O3GError(status, where)
+
+
+def release_scratch():
+    """Gives the scratch memory that split, merge, shedding and clear_inner_layer keep between calls
+    (up to 1 GiB per device) back, e.g. for PyTorch's allocator (o3g_release_scratch)."""
+    check(lib().o3g_release_scratch(), "o3g_release_scratch")
 
 
 def launch_count():

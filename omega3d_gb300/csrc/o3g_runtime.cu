@@ -121,8 +121,9 @@ static std::atomic<unsigned long long> g_allocs{0};
 // The pool behind dev_alloc_async, one per device.  The device's default pool returns its memory to
 // the system at every synchronisation: a split and a merge of 512,000 particles (about 100
 // arrays, 0.6 GB) spent 1.4 of 6.5 ms on mapping it again.  This one keeps up to kPoolKeep bytes (0.4 % of
-// the device) across synchronisations, hands the rest back, and hands all of it back when an
-// allocation of the library fails.  Stream-ordered, so safe with any streams and threads.
+// the device) across synchronisations and hands the rest back; it hands all of it back when an
+// allocation of the library fails and when the caller asks for it (o3g_release_scratch).
+// Stream-ordered, so safe with any streams and threads.
 constexpr uint64_t kPoolKeep = 1ull << 30;
 static std::mutex g_pool_mu;
 static std::map<int, cudaMemPool_t> g_pools;
@@ -151,6 +152,8 @@ static cudaMemPool_t async_pool() {
 static bool release_pool() {
   int dev = -1;
   if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  // (what was freed counts as used until the host has seen the stream get there)
+  if (cudaDeviceSynchronize() != cudaSuccess) return false;
   std::lock_guard<std::mutex> lk(g_pool_mu);
   auto it = g_pools.find(dev);
   return it != g_pools.end() && it->second && cudaMemPoolTrimTo(it->second, 0) == cudaSuccess;
@@ -238,6 +241,14 @@ int32_t o3g_flops_per_pair(int32_t core, int32_t grads, int32_t have_tr) {
 
 int32_t o3g_debug_wait_test(int32_t enable) {
   o3g::g_wait_test.store(enable == 2 ? 2 : enable != 0 ? 1 : 0);
+  return O3G_OK;
+}
+
+int32_t o3g_release_scratch(void) {
+  o3g::DeviceFacts f;
+  O3G_TRY(o3g::device_facts(&f));
+  (void)o3g::release_pool();
+  O3G_CUDA_TRY(cudaGetLastError());
   return O3G_OK;
 }
 
