@@ -149,14 +149,13 @@ __device__ const __align__(16) float kGaussPoly[{DEG + 1} * {len(table)}] = {{
 
 
 # ---- the accurate (double-single) evaluation: o3g_gauss_poly_ds.h ----------------------
-# Degree DEG_DS in t = q s + o, with s and o the float32 values the kernel uses (the fit is
-# made in that t, so the map itself adds no error).  The kernel runs Horner's rule in float
+# Degree DEG_DS in t = 2 q - (2 j + 1) on interval j.  The kernel runs Horner's rule in float
 # for the coefficients of degree >= 3 (together at most 0.14 % of |G| or |D| on every
 # interval, so their float rounding stays near 1e-10 relative) and in double-single
 # arithmetic for degrees 2, 1, 0, whose coefficients are stored as (hi, lo) float pairs.
 DEG_DS = 8
 NDS = 3          # low-order coefficients kept as (hi, lo) pairs
-STRIDE_DS = 2 + 2 * (DEG_DS + 1 - NDS) + 4 * NDS
+STRIDE_DS = 2 * (DEG_DS + 1 - NDS) + 4 * NDS
 
 
 def _split(v):
@@ -167,11 +166,10 @@ def _split(v):
 def fit_ds():
     table, worst = [], 0.0
     for lo, hi in zip(EDGES[:-1], EDGES[1:]):
-        s32, o32 = np.float32(2.0 / (hi - lo)), np.float32(-(hi + lo) / (hi - lo))
-        s, o = np.float64(s32), np.float64(o32)
+        s, o = 2.0 / (hi - lo), -(hi + lo) / (hi - lo)
         q = np.linspace(lo, hi, 40001)
         t = q * s + o
-        row = [s32, o32]
+        row = []
         polys = []
         for F in (gauss_G, gauss_D3):
             y = F(q)
@@ -204,7 +202,7 @@ def fit_ds():
 
 
 def write_ds(table, worst, path):
-    names = ["s", "o"] + ["%s%d" % (f, k) for k in range(DEG_DS, NDS - 1, -1) for f in ("G", "D")] + \
+    names = ["%s%d" % (f, k) for k in range(DEG_DS, NDS - 1, -1) for f in ("G", "D")] + \
             ["%s%d%s" % (f, k, h) for k in range(NDS - 1, -1, -1) for f in ("G", "D") for h in ("hi", "lo")]
     lines = []
     for k in range(STRIDE_DS):
@@ -213,8 +211,8 @@ def write_ds(table, worst, path):
     body = "\n".join(lines)
     txt = f"""// o3g_gauss_poly_ds.h -- GENERATED by gauss_poly_gen.py (do not edit): piecewise polynomials
 // of the Gaussian core for the accurate (double-single) precision mode: G(q) and
-// D(q) = -(2/3) G'(q), degree {DEG_DS} in t = q s + o (s, o the float
-// values below).  Coefficients of degree >= {NDS} are floats (Horner in float); degrees
+// D(q) = -(2/3) G'(q), degree {DEG_DS} in t = 2 q - (2 j + 1) on interval j.
+// Coefficients of degree >= {NDS} are floats (Horner in float); degrees
 // {NDS - 1}..0 are (hi, lo) float pairs (Horner in double-single).  Evaluated that way from an
 // exact q the result stays within {worst:.2e} relative of the double-precision functions
 // (D, which is rounded to float, needs the pairs of degrees 1 and 0 only).
@@ -225,7 +223,7 @@ namespace o3g {{
 constexpr int kGaussDsN = {len(table)};        // intervals; interval j covers [j, j + 1)
 constexpr int kGaussDsDeg = {DEG_DS};
 constexpr int kGaussDsPairs = {NDS};
-constexpr int kGaussDsStride = {STRIDE_DS};   // s, o, (G[k], D[k]) for k = {DEG_DS}..{NDS}, then (G[k] hi, lo, D[k] hi, lo) for k = {NDS - 1}..0
+constexpr int kGaussDsStride = {STRIDE_DS};   // (G[k], D[k]) for k = {DEG_DS}..{NDS}, then (G[k] hi, lo, D[k] hi, lo) for k = {NDS - 1}..0
 // entry e of interval j at kGaussPolyDs[e * kGaussDsN + j]
 __device__ const __align__(16) float kGaussPolyDs[{STRIDE_DS} * {len(table)}] = {{
 {body}

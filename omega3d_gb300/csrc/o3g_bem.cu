@@ -423,7 +423,7 @@ __global__ void __launch_bounds__(kPanelThreads) k_panel_lu(PanelArgs a) {
 // ---- the panel factorisation in one thread-block cluster ---------------------------------
 // What bounds a panel is latency: one pivot exchange per column.  Through global memory
 // (k_panel_lu, 152 blocks) it costs 3.1 us a column; among the 16 blocks of one cluster the
-// candidates travel through distributed shared memory behind the hardware's cluster barrier.
+// candidates travel through distributed shared memory, counted in on mbarriers.
 // The rows then have to fit 16 SMs: up to 640 rows of W = 64 columns in a block's registers, so
 // 10,240 rows fit; a kNb-column panel is factored W columns at a time (k_panel_next brings the
 // second half up to date).  More rows than that go to k_panel_lu.  A column's steps are a chain that

@@ -133,7 +133,7 @@ __host__ __device__ constexpr double gauss_coef(int n) {
   return (n % 2 == 1) ? c : -c;
 }
 template <class T> struct GaussP;
-template <> struct GaussP<float>  { static constexpr float  qfar = 48.0f; static constexpr int nterms = 9; };
+template <> struct GaussP<float>  { static constexpr float  qfar = 48.0f; };
 template <> struct GaussP<double> { static constexpr double qfar = 90.0;  static constexpr int nterms = 17; };
 
 // the hardware's reciprocal square root with nothing around it (rsqrtf() scales subnormal
@@ -240,10 +240,6 @@ __device__ __forceinline__ double dist2_ref(double dx, double dy, double dz) {
   return __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
 }
 
-__device__ __forceinline__ float dev_erf(float x) { return erff(x); }
-__device__ __forceinline__ double dev_erf(double x) { return erf(x); }
-__device__ __forceinline__ float dev_exp(float x) { return expf(x); }
-__device__ __forceinline__ double dev_exp(double x) { return exp(x); }
 __device__ __forceinline__ float dev_expm1(float x) { return expm1f(x); }
 __device__ __forceinline__ double dev_expm1(double x) { return expm1(x); }
 __device__ __forceinline__ float dev_sqrt(float x) { return sqrtf(x); }

@@ -129,16 +129,16 @@ __device__ __forceinline__ void gauss_poly_ds(dsf q, dsf& G, dsf& D) {
   t.l = __fmaf_rn(2.0f, q.l, t.l);
   constexpr int NF = kGaussDsDeg + 1 - kGaussDsPairs;      // float coefficients per function
   static_assert(kGaussDsPairs == 3, "degrees 2 to 0");
-  float g = __ldg(tb + 2 * N + j), d = GRAD ? __ldg(tb + 3 * N + j) : 0.f;
+  float g = __ldg(tb + j), d = GRAD ? __ldg(tb + N + j) : 0.f;
 #pragma unroll
   for (int k = 1; k < NF; ++k) {
-    g = __fmaf_rn(g, t.h, __ldg(tb + (2 + 2 * k) * N + j));
-    if (GRAD) d = __fmaf_rn(d, t.h, __ldg(tb + (3 + 2 * k) * N + j));
+    g = __fmaf_rn(g, t.h, __ldg(tb + 2 * k * N + j));
+    if (GRAD) d = __fmaf_rn(d, t.h, __ldg(tb + (2 * k + 1) * N + j));
   }
   dsf gg{g, 0.f}, dd{d, 0.f};
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    const int e = 2 + 2 * NF + 4 * k;
+    const int e = 2 * NF + 4 * k;
     gg = ds_horner(gg, t, __ldg(tb + e * N + j), __ldg(tb + (e + 1) * N + j));
     if (GRAD) {
       if (k == 0) dd.h = __fmaf_rn(d, t.h, __ldg(tb + (e + 2) * N + j));
