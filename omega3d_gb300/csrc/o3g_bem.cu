@@ -427,8 +427,8 @@ __global__ void __launch_bounds__(kPanelThreads) k_panel_lu(PanelArgs a) {
 // The rows then have to fit 16 SMs: up to 640 rows of W = 64 columns in a block's registers, so
 // 10,240 rows fit; a kNb-column panel is factored W columns at a time (k_panel_next brings the
 // second half up to date).  More rows than that go to k_panel_lu.  A column's steps are a chain that
-// every warp runs for itself, so the fewer warps share a scheduler the faster: 64 columns take 86 us
-// with 10 warps a block (10,240 rows), 73 with 8 (8,192), 65 with 4 (4,096), whatever the cluster's size.
+// every warp runs for itself, so the fewer warps share a scheduler the faster: 64 columns take 90 us
+// with 10 warps a block (10,240 rows), 77 with 8 (8,192), 69 with 4 (4,096), whatever the cluster's size.
 //
 // Rows do not move while the sub-panel is factored: each thread tracks the position its rows have
 // after the interchanges so far (LAPACK's order); the sub-panel's rows are stored there at
@@ -441,8 +441,8 @@ __global__ void __launch_bounds__(kPanelThreads) k_panel_lu(PanelArgs a) {
 // of the group, held as tiles of 4 rows x 4 columns per thread and chunk, take the rank-8 update: a
 // tile reads 4 multipliers and 4 elements of U for 16 products (two full rows per thread: 58 reads
 // for 112 products, and this update a fifth of the kernel).
-// Measured (one GB300), 64 columns with 10 warps: 112 -> 86 us (one warp's instructions in series
-// are what is left: 150 a column); factorisation at n = 10,240: 43.2 -> 21.6 ms with the kernels below.  Not kept: full
+// Measured (one GB300), 64 columns with 10 warps: 112 -> 90 us (one warp's instructions in series
+// are what is left); factorisation at n = 10,240: 43.2 -> 22.3 ms with the kernels below.  Not kept: full
 // rows in every exchange with a rank-1 update of the whole width per column (2.3 us a column),
 // the column's code unrolled (by 8: 108 against 97 us; fetching it takes longer than running
 // it), a block barrier and a second search by every warp before the exchange (112 against
@@ -694,8 +694,8 @@ __device__ __forceinline__ void panel_group(const ClusterPanelArgs& a, ClusterSh
           if (k >= B - jj) ue[k] = 0.f;
         // x / pv as the division rounds it: a reciprocal rounded to nearest, and per row two corrections by
         // the exact residual (P. Markstein, IBM J. Res. Dev. 34, 1990: the first leaves the quotient within
-        // an ulp, the second then rounds it correctly), where nothing underflows on the way.  The division
-        // itself for every row takes 23.5 ms of a factorisation at n = 10,240, this 22.1.
+        // an ulp, the second then rounds it correctly), where nothing underflows on the way.  A division per
+        // row costs 1.4 ms more of a factorisation at n = 10,240 (23.5 ms).
         const float rp = __frcp_rn(pv), ap = fabsf(pv);
         float l[RPT];
         bool good = ap > 1e-30f && ap < 1e30f;

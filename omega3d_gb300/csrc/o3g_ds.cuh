@@ -21,8 +21,8 @@
 //
 // What bounds it is the FMA pipe.  Intermediate values stay unnormalised where the next operation
 // takes them so (a low part of up to 2^-20 of the high one), one renormalisation per sum of
-// squares and per q: RM takes 174 operations a pair, 235 cycles per pair and warp scheduler at
-// 32,768 particles (276 with every result renormalised), Gaussian 240 (320).
+// squares and per q.  RM takes 176 operations a pair and 230 cycles per pair and warp scheduler (32,768
+// particles of a Gaussian cloud), Gaussian 231; renormalising every result took 1.2 and 1.3 times as long.
 //
 // Error-free transformations: two-sum (Knuth), fast two-sum (Dekker, |a| >= |b|), and the
 // product error fma(a, b, -a b) -- the standard float-float toolkit (Dekker 1971; Hida, Li

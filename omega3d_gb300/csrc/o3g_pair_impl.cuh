@@ -7,8 +7,8 @@
 //   (double4 for the FP64 mode).  Padding sources have zero strength and core parameter 1
 //   (as the reference's Vc padding, Influence.h:232-238) and sit at (1e9, 1e9, 1e9): every
 //   core and the singular far-field loop give finite r3 and bbb there (d^4 = 9e36 stays
-//   below the float range), so with zero strength they add exactly zero, also to a target
-//   at the origin.
+//   FLT_MAX), so with zero strength they add exactly zero, also to a target at the origin;
+//   against a target so far away that d^4 overflows V2's term is 0.
 //
 // Kernel k_pair: a block of kBlock threads owns kBlock*TPT targets; each warp owns a
 // contiguous run of 32*TPT of them (lane l holds targets l, l+32, ... so loads and stores
@@ -240,7 +240,7 @@ __device__ __forceinline__ void sweep_tile(const V4<T>* sp, const V4<T>* sw, con
 // What bounds these kernels is the FMA pipe: RM plain with gradients takes 34 packed
 // operations and two MUFU per pair of sources, 34 cycles per pair and warp scheduler at two
 // cycles each, and runs at 41 (65,536 particles, one GB300; was 47 with 37 operations), RM
-// compensated at 50 (60).
+// compensated at 51 (60).
 // The rest is the register file: a micro-benchmark of FFMA2 alone takes 2.1 cycles when one
 // operand is the previous instruction's, 2.95 with three new ones (FMUL2, FADD2 2.1; a
 // scalar FFMA 1.08), so the accumulations below are written in runs that share an operand.
@@ -402,8 +402,8 @@ __device__ __forceinline__ void pair2(const float2* tt, const float4& q0, const 
   core2<C, ACC, GRADS>(dx, dy, dz, cst, gtab, r3, b3);
   const float2 wx = f2lo(q2), wy = f2hi(q2);
   // which operands carry the signs decides the register assignment: at 65,536 particles (RM) the
-  // compensated kernel takes 49.7 cycles per pair with the strengths negated and 53.3 with the
-  // separations, the plain one 42.4 and 41.2 (51.5 and 41.3 with five staged rows)
+  // plain kernel takes 42.4 cycles per pair with the strengths negated and 41.2 with the separations, the
+  // compensated one 51.4 and 52.1 (51.5 and 50.7 on field points)
   constexpr bool NEGW = ACC || C == CORE_EXP;
   const float2 ndx = NEGW ? dx : neg2(dx), ndy = NEGW ? dy : neg2(dy), ndz = NEGW ? dz : neg2(dz);
   const float2 nwx = NEGW ? neg2(wx) : wx, nwy = NEGW ? neg2(wy) : wy, nwz = NEGW ? neg2(wz) : wz;
@@ -629,11 +629,12 @@ __global__ void __launch_bounds__(kBlock) k_pair(const PairArgs<T, O> a) {
 }
 
 // Blocks per SM asked of the compiler (0: its own choice).  The compensated Gaussian kernel
-// with gradients would take 124 registers (4 blocks); held to 5 blocks it spills 8 bytes outside the
-// pair loops and a 262,144-particle cloud takes 97.4 ms (4 blocks, with five staged rows: 102.8
-// against 98.0; 111 before gauss2's table, rsq2, the factored gradient and the four rows).  Two
-// targets per thread read half the rows but leave 3 blocks: RM 50.8 cycles per pair against
-// 49.7, Gaussian 62.7 against 62.5.
+// with gradients would take 124 registers (4 blocks); held to 5 blocks it spills 4 bytes outside the
+// pair loops and a 262,144-particle cloud takes 100.3 ms (4 blocks 102.4; 111 before gauss2's table, rsq2,
+// the factored gradient and the four rows).  RM takes 86 registers (5 blocks): held to 6 it spills 12 bytes with
+// target radii (5.75 against 5.59 ms at 65,536 particles; 5.48 against 5.60 on field points).  Two targets per
+// thread read half the rows but leave 3 blocks, and were no faster (RM 50.8 cycles per pair against 49.7,
+// Gaussian 62.7 against 62.5, without the zz sum).
 // The plain kernels with two targets per thread are held to the 128 registers of 4 blocks
 // (the batched ones would take 130 to 159).
 template <int C, int MODE, bool GRADS, int TPT> struct PairMinBlocks {

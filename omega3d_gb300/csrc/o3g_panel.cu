@@ -24,7 +24,7 @@
 //     lanes have a close panel at the same time, and their trees have 4 to 64 leaves.
 // The owner adds its nodes' sums in queue order: results do not depend on scheduling.
 // Measured (one GB300), 5,120 panels on 262,144 points with gradients, compensated: 4.32 ->
-// 2.23 ms; 100,000 particles on 20,480 panels: 3.05 -> 1.34 ms (2.43 and 1.41 with six rows a tile).
+// 2.33 ms; 100,000 particles on 20,480 panels: 3.05 -> 1.34 ms (1.41 with six rows a tile).
 //
 #include "o3g_pair_impl.cuh"
 
